@@ -251,7 +251,7 @@ def gpu_bench(args, world, rank, local):
         ms, by, la = g.bench_kernel(name, reps=20)
         kern[name] = {"ms": ms, "alg_bytes": by, "launches": la, "gbs": by / ms / 1e6}
     trace = {"fp64": g.ilu_trace(fp32=False), "fp32": g.ilu_trace(fp32=True)}
-    budget = iteration_budget(g, g64, st, b_dev, x_dev, local) if not args.quick else None
+    budget = iteration_budget(g, g64, st, s.rowptr, b_dev, x_dev, local) if not args.quick else None
     it_ms = value / max(1, (r0.half_iters + 1) / 2.0)
     solve_gbs = st["alg_bytes_iter"][0] / it_ms / 1e6 if it_ms > 0 else None
     traffic = None
@@ -313,26 +313,34 @@ FP64_FMA_LANES_PER_CLK_SM = 1.68   # measured on GB300 (independent DFMA chains)
 SM_CLOCK_HZ = 2.07e9
 
 
-def iteration_budget(g, g64, st, b_dev, x_dev, local):
+def iteration_budget(g, g64, st, rowptr, b_dev, x_dev, local):
     """Where one BiCGSTAB iteration's time goes: every kernel of the
     iteration timed alone (back to back, CUDA events), beside its HBM floor
     (algorithmic bytes at the measured copy peak) and, for FP64, its FP64
     floor (DFMA count at the measured FP64 rate); and the measured time per
     iteration of whole solves (the slope between maxit 4 and 12, tol 0)."""
+    import numpy as np
     import torch
     peak, _ = peaks()
     sms = torch.cuda.get_device_properties(local).multi_processor_count
     fma_rate = FP64_FMA_LANES_PER_CLK_SM * sms * SM_CLOCK_HZ
-    n, nb, nnzb = 3 * st["nb"], st["nb"], st["nnzb"]
-    nlu = st["nnzb_lower"] + st["nnzb_upper"]
-    # DFMA per launch (FP64): SpMV 9 per block (+ the fused dots), apply 9
-    # per L, U and D block, update_s 2n, update_r 5n, update_p 2n
-    fmas = {"ilu": 9 * (nlu + nb), "spmv_alpha": 9 * nnzb + n, "spmv_omega": 9 * nnzb + 2 * n,
-            "update_s": 2 * n, "update_r": 5 * n, "update_p": 2 * n}
+    # DFMA per launch (FP64) over the rows that the iteration runs on: color 0
+    # (n0 rows, a0 blocks of A) takes part in the apply's last step alone; the
+    # other n rows in the SpMV (9 per block and the dots) and the vector
+    # kernels (update_s and update_p also apply D^-1 to color 1)
+    _, color, _, cp = g64.ordering()
+    n0, n1 = int(cp[1]), int(cp[2] - cp[1])
+    deg = np.diff(rowptr)
+    a0 = int(deg[color == 0].sum())
+    nb, nnzb, n = st["nb"], st["nnzb"], 3 * (st["nb"] - n0)
+    inner = st["nnzb_lower"] + st["nnzb_upper"] - 2 * (a0 - n0)
+    fmas = {"apply": 9 * (a0 - n0 + inner + nb - n1), "spmv_alpha": 9 * (nnzb - a0) + n,
+            "spmv_omega": 9 * (nnzb - a0) + 2 * n, "update_s": 3 * n + 9 * n1,
+            "update_r": 5 * n, "update_p": 3 * n + 9 * n1}
     out = {}
     for prec, suf in (("fp64", "64"), ("fp32", "32")):
         rows = {}
-        for name, count in (("ilu", 2), ("spmv_alpha", 1), ("spmv_omega", 1), ("update_s", 1),
+        for name, count in (("apply", 2), ("spmv_alpha", 1), ("spmv_omega", 1), ("update_s", 1),
                             ("update_r", 1), ("update_p", 1)):
             ms, by, la = g.bench_kernel(name + suf, reps=20)
             r = {"per_iter": count, "us": ms * 1e3, "alg_bytes": by,

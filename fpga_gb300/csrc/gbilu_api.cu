@@ -5,6 +5,7 @@
 #include "gbilu_fpga_export.hpp"
 #include "gbilu_host.hpp"
 #include "gbilu_kernels.cuh"
+#include "gbilu_reduced.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -48,15 +49,16 @@ struct DevMat {
 template <typename T> struct Vecs {
   DevBuf<T> x, r, rt, p, ph, v, s, sh, t;
   DevBuf<T> y;               // first sweep of a preconditioner apply
+  DevBuf<T> base;            // reduced iteration (gbilu_reduced.cuh)
   cudaError_t alloc(size_t n) {
-    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y}) {
+    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y, &base}) {
       cudaError_t e = b->alloc(n);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
   }
   void release() {
-    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y}) b->release();
+    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y, &base}) b->release();
   }
 };
 
@@ -66,6 +68,7 @@ template <typename V, typename T> struct Ops {
   const int *offA, *colA; const V *valA;     // A or A^T
   const int *off1, *col1; const V *val1;     // first sweep: L or U^T
   const int *off2, *col2; const V *val2;     // second sweep: U or L^T
+  const int *off1r, *col1r; const V *val1r;  // first sweep without color 0's columns
   const V *dmat;                             // Dinv or Dinv^T (sliced)
   Vecs<T> *vec;
 };
@@ -95,6 +98,7 @@ struct Handle {
   DevBuf<int> perm, iperm, dperm, prowptr, pcol, psrc;
   DevBuf<int> ibrow, icol;                   // input pattern: block -> row, column (dL/dA)
   DevMat A, L, U, At, Ut, Lt;
+  DevMat Lr, Utr;            // L and U^T without color 0's columns
   DevBuf<double> dinv64, dinvT64;
   DevBuf<float> dinv32, dinvT32;
   Vecs<double> v64;
@@ -113,17 +117,25 @@ struct Handle {
   cudaGraphExec_t graph_ru[2] = {nullptr, nullptr};  // mixed by replacement [transpose]
   int per_iter[2] = {0, 0};                // launches per iteration [transpose]
   long long last_launches = 0;
-  // color steps [fp32][transpose]: the full list (one launch per step), and
+  // color steps: the full list (one launch per step), and
   // the same as the single-launch apply's parameter when it fits (n = 0
   // otherwise: more than kMaxPhases / 2 colors)
-  std::vector<Phase> steps[2][2];
-  PhaseList phases[2][2];
-  StagePlan stage[2][2] = {};              // shared-memory staging of small steps
-  int stage_bytes[2][2] = {};
-  DevBuf<StageEntry> stage_tab[2][2];
-  DevBuf<int2> stage_cnt[2][2];
-  DevBuf<unsigned int> ring_tab[2][2];     // streamed slices per CTA (see StagePlan)
-  DevBuf<int> ring_cnt[2][2];
+  struct Sweep {
+    std::vector<Phase> steps;
+    PhaseList phases;
+    StagePlan stage = {};                  // shared-memory staging of small steps
+    int stage_bytes = 0;
+    DevBuf<StageEntry> stage_tab;
+    DevBuf<int2> stage_cnt;
+    DevBuf<unsigned int> ring_tab;         // streamed slices per CTA (see StagePlan)
+    DevBuf<int> ring_cnt;
+    void release() {
+      stage_tab.release(); stage_cnt.release(); ring_tab.release(); ring_cnt.release();
+      stage = StagePlan{};
+      stage_bytes = 0;
+    }
+  };
+  Sweep sweep[2][2][2];                    // [reduced][fp32][transpose]
   cudaError_t launch_err = cudaSuccess;    // first failed cooperative launch
   int coop_grid64 = 1, coop_grid32 = 1;    // CTAs of the cooperative apply
   size_t device_bytes = 0;
@@ -191,7 +203,10 @@ int reduce_grid(const Handle *h, long long work) {
 // U^T sweep with D^-T over all colors, the rows without a higher-colored
 // neighbour final at once (unit diagonal of L^T); the L^T sweep covers the
 // leading rows of colors C-2..0.
-std::vector<Phase> make_steps(const Analysis &an, bool transpose) {
+// reduced: the steps that the reduced iteration leaves to the apply
+// (gbilu_reduced.cuh): color 1's first-sweep step is part of the kernel
+// before, own values come from base, and color 0 has the last step alone.
+std::vector<Phase> make_steps(const Analysis &an, bool transpose, bool reduced = false) {
   std::vector<Phase> st;
   const int C = an.ncolors;
   st.reserve(2 * (size_t)C);
@@ -206,7 +221,25 @@ std::vector<Phase> make_steps(const Analysis &an, bool transpose) {
     p.mat = mat;
     return p;
   };
-  if (!transpose) {
+  if (reduced) {
+    for (int c = 2; c < C; ++c) {
+      Phase &p = add(c, 0, rows(c));
+      p.has_d = transpose;
+      p.own_base = 2;
+      p.to_y = 1;
+      p.final0 = an.color_ptr[c] + an.split[c];
+      p.final_d = !transpose;
+    }
+    for (int c = C - 2; c >= 0; --c) {
+      const int nr = c == 0 ? rows(0) : an.split[c];
+      if (nr == 0) continue;
+      Phase &p = add(c, 1, nr);
+      p.has_d = !transpose;
+      p.own_base = c == 0;
+      p.own_y = c != 0;
+      p.nbr_hat = 1;
+    }
+  } else if (!transpose) {
     if (C == 1) {   // no couplings: z = D^-1 src
       add(0, 1, rows(0)).has_d = 1;
       return st;
@@ -264,8 +297,12 @@ PhaseList phase_list(const std::vector<Phase> &st) {
 
 template <typename V, typename T>
 int coop_grid(Handle *h) {
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilu_coop<V, T>, coop_threads<T>(), 0);
+  int per_sm = 0, per_sm_red = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilu_coop<V, T, false>,
+                                                coop_threads<T>(), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_red, k_ilu_coop<V, T, true>,
+                                                coop_threads<T>(), 0);
+  per_sm = std::min(per_sm, per_sm_red);
   long long most = 0;
   for (int c = 0; c < h->an.ncolors; ++c) {
     const long long rows = h->an.color_ptr[c + 1] - h->an.color_ptr[c];
@@ -298,11 +335,13 @@ long long slice_bytes(const SlicedMatrix &m, int slice, bool uses_d) {
          (uses_d ? 9 * 32 * (long long)sizeof(V) : 0);
 }
 
-template <typename V, typename T>
+template <typename V, typename T, bool RED>
 int build_stage_plan(Handle *h, int f, int t, int grid) {
-  PhaseList &pl = h->phases[f][t];
+  Handle::Sweep &sw = h->sweep[RED][f][t];
+  PhaseList &pl = sw.phases;
   const Analysis &an = h->an;
   auto mat_of = [&](const Phase &P) -> const SlicedMatrix & {
+    if (RED && !P.mat) return t == 0 ? an.Lr : an.Utr;
     return t == 0 ? (P.mat ? an.U : an.L) : (P.mat ? an.Lt : an.Ut);
   };
   std::vector<std::vector<StageEntry>> per(grid);
@@ -330,8 +369,8 @@ int build_stage_plan(Handle *h, int f, int t, int grid) {
     most = std::max(most, bytes[b]);
     most_n = std::max(most_n, per[b].size());
   }
-  h->stage[f][t] = StagePlan{nullptr, nullptr, 0, 0, 0, 0, nullptr, nullptr, 0};
-  h->stage_bytes[f][t] = 0;
+  sw.stage = StagePlan{};
+  sw.stage_bytes = 0;
   const bool staged = h->opt.stage_small_steps && most_n > 0 && most <= kStageBudget &&
                       most_n <= (size_t)kMaxStage;
   if (!staged) {
@@ -342,7 +381,7 @@ int build_stage_plan(Handle *h, int f, int t, int grid) {
   int optin = 0;
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->opt.device));
   cudaFuncAttributes fa;
-  CK(cudaFuncGetAttributes(&fa, k_ilu_coop<V, T>));
+  CK(cudaFuncGetAttributes(&fa, k_ilu_coop<V, T, RED>));
   const long long ring_off = (most + 127) / 128 * 128;
   long long stride = 0;
   bool any_large = false;
@@ -377,10 +416,10 @@ int build_stage_plan(Handle *h, int f, int t, int grid) {
     for (int q = 0; q < pl.n; ++q) pl.p[q].streamed = streamable(q);
   const long long dyn = ring ? ring_off + ns * stride : most;
   if (dyn > 0) {
-    CK(cudaFuncSetAttribute(k_ilu_coop<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CK(cudaFuncSetAttribute(k_ilu_coop<V, T, RED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)std::max<long long>(dyn, fa.maxDynamicSharedSizeBytes)));
     int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilu_coop<V, T>, coop_threads<T>(),
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilu_coop<V, T, RED>, coop_threads<T>(),
                                                      (size_t)dyn));
     if (per_sm < 1)
       return h->fail(GBILU_CUDA_ERROR, "single-launch apply does not fit an SM with %lld bytes "
@@ -408,13 +447,13 @@ int build_stage_plan(Handle *h, int f, int t, int grid) {
       std::copy(lists[b].begin(), lists[b].end(), tab.begin() + (size_t)b * mx);
       cnt[b] = (int)lists[b].size();
     }
-    CK(h->ring_tab[f][t].alloc(tab.size()));
-    CK(h->ring_cnt[f][t].alloc(cnt.size()));
-    CK(cudaMemcpy(h->ring_tab[f][t].p, tab.data(), tab.size() * sizeof(unsigned int),
+    CK(sw.ring_tab.alloc(tab.size()));
+    CK(sw.ring_cnt.alloc(cnt.size()));
+    CK(cudaMemcpy(sw.ring_tab.p, tab.data(), tab.size() * sizeof(unsigned int),
                   cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->ring_cnt[f][t].p, cnt.data(), cnt.size() * sizeof(int), cudaMemcpyHostToDevice));
-    sp.ring_tab = h->ring_tab[f][t].p;
-    sp.ring_cnt = h->ring_cnt[f][t].p;
+    CK(cudaMemcpy(sw.ring_cnt.p, cnt.data(), cnt.size() * sizeof(int), cudaMemcpyHostToDevice));
+    sp.ring_tab = sw.ring_tab.p;
+    sp.ring_cnt = sw.ring_cnt.p;
     sp.ring_max = (int)mx;
   }
   if (staged) {
@@ -424,27 +463,28 @@ int build_stage_plan(Handle *h, int f, int t, int grid) {
       for (size_t e = 0; e < per[b].size(); ++e) tab[(size_t)b * kMaxStage + e] = per[b][e];
       cnt[b] = make_int2((int)per[b].size(), (int)bytes[b]);
     }
-    CK(h->stage_tab[f][t].alloc(tab.size()));
-    CK(h->stage_cnt[f][t].alloc(cnt.size()));
-    CK(cudaMemcpy(h->stage_tab[f][t].p, tab.data(), tab.size() * sizeof(StageEntry),
+    CK(sw.stage_tab.alloc(tab.size()));
+    CK(sw.stage_cnt.alloc(cnt.size()));
+    CK(cudaMemcpy(sw.stage_tab.p, tab.data(), tab.size() * sizeof(StageEntry),
                   cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->stage_cnt[f][t].p, cnt.data(), cnt.size() * sizeof(int2),
+    CK(cudaMemcpy(sw.stage_cnt.p, cnt.data(), cnt.size() * sizeof(int2),
                   cudaMemcpyHostToDevice));
-    sp.tab = h->stage_tab[f][t].p;
-    sp.cnt = h->stage_cnt[f][t].p;
+    sp.tab = sw.stage_tab.p;
+    sp.cnt = sw.stage_cnt.p;
     sp.enabled = 1;
   }
-  h->stage[f][t] = sp;
-  h->stage_bytes[f][t] = (int)dyn;
+  sw.stage = sp;
+  sw.stage_bytes = (int)dyn;
   return GBILU_OK;
 }
 
 // The single-launch preconditioner apply (cooperative, all CTAs resident).
-template <typename V, typename T>
+template <typename V, typename T, bool RED = false>
 cudaError_t launch_coop(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *hat,
-                        int trace) {
+                        int trace, const double *coef = nullptr) {
   const int f = sizeof(T) == 4 ? 1 : 0, t = o.transpose ? 1 : 0;
-  PhaseList pl = h->phases[f][t];
+  const Handle::Sweep &sw = h->sweep[RED][f][t];
+  PhaseList pl = sw.phases;
   pl.trace = trace;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -452,43 +492,49 @@ cudaError_t launch_coop(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *
   attr[0].val.cooperative = 1;
   cfg.gridDim = dim3(f ? h->coop_grid32 : h->coop_grid64);
   cfg.blockDim = dim3(coop_threads<T>());
-  cfg.dynamicSmemBytes = (size_t)h->stage_bytes[f][t];
+  cfg.dynamicSmemBytes = (size_t)sw.stage_bytes;
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_ilu_coop<V, T>, h->ctl.p, pl, h->stage[f][t], o.off1, o.col1,
-                            o.val1, o.off2, o.col2, o.val2, o.dmat, src, o.vec->y.p, hat);
+  return cudaLaunchKernelEx(&cfg, k_ilu_coop<V, T, RED>, h->ctl.p, pl, sw.stage,
+                            RED ? o.off1r : o.off1, RED ? o.col1r : o.col1,
+                            RED ? o.val1r : o.val1, o.off2, o.col2, o.val2, o.dmat, src,
+                            o.vec->y.p, hat, (const T *)o.vec->base.p, coef);
 }
 
 // hat = M^-1 src (forward) or M^-T src (transpose); the vector set's y holds
-// the first sweep's result.
-template <typename V, typename T>
+// the first sweep's result. RED: what the reduced iteration leaves of it,
+// with coef = &Ctl::cp (src = p) or &Ctl::cs (src = s); with two colors that
+// is one step, launched by itself.
+template <typename V, typename T, bool RED = false>
 void apply_prec(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *hat,
-                int &launches) {
+                int &launches, const double *coef = nullptr) {
   const int C = h->an.ncolors;
-  if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2) {
-    const cudaError_t e = launch_coop(h, s, o, src, hat, 0);
+  if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 && !(RED && C == 2)) {
+    const cudaError_t e = launch_coop<V, T, RED>(h, s, o, src, hat, 0, coef);
     if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
     ++launches;
     return;
   }
-  for (const Phase &P : h->steps[sizeof(T) == 4 ? 1 : 0][o.transpose ? 1 : 0]) {
-    k_phase<V, T><<<(unsigned)((P.nrows + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        h->ctl.p, P, P.mat ? o.off2 : o.off1, P.mat ? o.col2 : o.col1, P.mat ? o.val2 : o.val1,
-        o.dmat, src, o.vec->y.p, hat);
+  for (const Phase &P : h->sweep[RED][sizeof(T) == 4 ? 1 : 0][o.transpose ? 1 : 0].steps) {
+    k_phase<V, T, RED><<<(unsigned)((P.nrows + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+        h->ctl.p, P, P.mat ? o.off2 : RED ? o.off1r : o.off1,
+        P.mat ? o.col2 : RED ? o.col1r : o.col1, P.mat ? o.val2 : RED ? o.val1r : o.val1, o.dmat,
+        src, o.vec->y.p, hat, o.vec->base.p, coef);
     ++launches;
   }
 }
 
 template <typename V, typename T, int MODE>
 void spmv(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *x, T *y, const T *w,
-          int &launches, const int *x_nonzero = nullptr) {
+          int &launches, const int *x_nonzero = nullptr, int S0 = 0) {
   const int S = h->an.S;
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmv<V, T, MODE>, kThreads, 0);
-  const int grid = std::max(1, std::min((S + kWarps - 1) / kWarps, std::max(1, per_sm) * h->sm_count));
+  const int grid =
+      std::max(1, std::min((S - S0 + kWarps - 1) / kWarps, std::max(1, per_sm) * h->sm_count));
   k_spmv<V, T, MODE><<<grid, kThreads, 0, s>>>(
-      h->ctl.p, S, h->srows.p, o.offA, o.colA, o.valA, x, y, w, h->partials.p, x_nonzero);
+      h->ctl.p, S0, S, h->srows.p, o.offA, o.colA, o.valA, x, y, w, h->partials.p, x_nonzero);
   ++launches;
 }
 
@@ -524,6 +570,77 @@ void enqueue_iteration(Handle *h, cudaStream_t s, const Ops<V, T> &o,
   launches += 3;
 }
 
+// Whether a run of this handle uses the reduced iteration: not with one color
+// (the head would be everything), nor with residual replacement, whose new
+// residual is not a multiple of the initial one on the head.
+bool reduced_run(const Handle *h, bool ru) { return h->an.ncolors > 1 && !ru; }
+
+template <typename V, typename T> Tail<V, T> make_tail(const Handle *h, const Ops<V, T> &o, T *hat) {
+  const Analysis &an = h->an;
+  Tail<V, T> P;
+  P.row0 = an.color_ptr[1];
+  P.rows = an.nb - P.row0;
+  P.rows1 = an.color_ptr[2] - P.row0;
+  P.split1 = an.split[1];
+  P.slice1 = an.slice_color_ptr[1];
+  P.d_first = o.transpose;
+  P.dmat = o.dmat;
+  P.base = o.vec->base.p;
+  P.ybuf = o.vec->y.p;
+  P.hat = hat;
+  return P;
+}
+
+// CTAs of a kernel with one thread per row, at most cap: each thread gets
+// the same number of rows (a last round that few CTAs take part in costs as
+// much as a full one).
+int row_grid(const Handle *h, int rows, int ctas_per_sm) {
+  const long long cap = (long long)h->sm_count * ctas_per_sm * kThreads;
+  const long long rounds = std::max<long long>(1, (rows + cap - 1) / cap);
+  return (int)std::max<long long>(1, (rows + rounds * kThreads - 1) / (rounds * kThreads));
+}
+
+// One iteration of the reduced form (gbilu_reduced.cuh): the first sweep of
+// p on color 1 was done by the kernel before the loop body.
+template <typename V, typename T>
+void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned long long cond,
+                     int &launches) {
+  Vecs<T> &w = *o.vec;
+  Ctl *c = h->ctl.p;
+  double *part = h->partials.p;
+  const Tail<V, T> tp = make_tail(h, o, w.ph.p), ts = make_tail(h, o, w.sh.p);
+  const int S0 = tp.slice1, n0 = 3 * tp.row0, nt = 3 * tp.rows;
+  apply_prec<V, T, true>(h, s, o, w.p.p, w.ph.p, launches, &c->cp);
+  spmv<V, T, SPMV_ALPHA>(h, s, o, w.ph.p, w.v.p, w.rt.p, launches, nullptr, S0);
+  k_tail_s<V, T><<<row_grid(h, tp.rows, GBILU_REDUCE_CTAS_PER_SM), kThreads, 0, s>>>(
+      c, ts, w.r.p, w.v.p, w.s.p, part);
+  apply_prec<V, T, true>(h, s, o, w.s.p, w.sh.p, launches, &c->cs);
+  spmv<V, T, SPMV_OMEGA>(h, s, o, w.sh.p, w.t.p, w.s.p, launches, nullptr, S0);
+  k_update_r<T><<<reduce_grid(h, nt), kThreads, 0, s>>>(c, nt, w.x.p + n0, w.ph.p + n0,
+                                                        w.sh.p + n0, w.s.p + n0, w.t.p + n0,
+                                                        w.rt.p + n0, w.r.p + n0, part);
+  k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, s>>>(c, tp, w.r.p, w.v.p, w.p.p,
+                                                                       w.rt.p, cond);
+  launches += 3;
+}
+
+// The reduced form's start, after the initial residual (base holds the
+// head's r0): base everywhere and the first sweep of p on color 1.
+template <typename V, typename T>
+void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
+  const Tail<V, T> tp = make_tail(h, o, o.vec->ph.p);
+  if (o.transpose) {
+    k_base_head<V, T><<<(tp.row0 + kThreads - 1) / kThreads, kThreads, 0, h->st>>>(
+        h->ctl.p, tp.row0, o.dmat, o.vec->base.p);
+    ++launches;
+  }
+  const int S = h->an.S;
+  k_base_tail<V, T><<<std::min((S - tp.slice1 + kWarps - 1) / kWarps, 8 * h->sm_count), kThreads, 0,
+                      h->st>>>(h->ctl.p, tp, S, h->srows.p, o.off1, o.col1, o.val1, o.vec->p.p,
+                               o.vec->base.p);
+  ++launches;
+}
+
 template <typename V, typename T>
 int build_graph(Handle *h, const Ops<V, T> &o, cudaGraphExec_t &exec, int &per_iter,
                 const Ops<double, double> *ru64 = nullptr) {
@@ -542,7 +659,10 @@ int build_graph(Handle *h, const Ops<V, T> &o, cudaGraphExec_t &exec, int &per_i
   CK(cudaStreamBeginCaptureToGraph(h->cap, body, nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
   int launches = 0;
-  enqueue_iteration(h, h->cap, o, (unsigned long long)cond, launches, ru64);
+  if (reduced_run(h, ru64 != nullptr))
+    enqueue_reduced(h, h->cap, o, (unsigned long long)cond, launches);
+  else
+    enqueue_iteration(h, h->cap, o, (unsigned long long)cond, launches, ru64);
   cudaGraph_t captured = nullptr;
   CK(cudaStreamEndCapture(h->cap, &captured));
   CK(cudaGraphInstantiate(&exec, g, 0));
@@ -557,9 +677,11 @@ template <> Ops<double, double> make_ops(Handle *h, bool t) {
   Ops<double, double> o;
   o.transpose = t;
   DevMat &a = t ? h->At : h->A, &m1 = t ? h->Ut : h->L, &m2 = t ? h->Lt : h->U;
+  DevMat &mr = t ? h->Utr : h->Lr;
   o.offA = a.off.p; o.colA = a.col.p; o.valA = a.v64.p;
   o.off1 = m1.off.p; o.col1 = m1.col.p; o.val1 = m1.v64.p;
   o.off2 = m2.off.p; o.col2 = m2.col.p; o.val2 = m2.v64.p;
+  o.off1r = mr.off.p; o.col1r = mr.col.p; o.val1r = mr.v64.p;
   o.dmat = t ? h->dinvT64.p : h->dinv64.p;
   o.vec = &h->v64;
   return o;
@@ -569,23 +691,29 @@ template <> Ops<float, float> make_ops(Handle *h, bool t) {
   Ops<float, float> o;
   o.transpose = t;
   DevMat &a = t ? h->At : h->A, &m1 = t ? h->Ut : h->L, &m2 = t ? h->Lt : h->U;
+  DevMat &mr = t ? h->Utr : h->Lr;
   o.offA = a.off.p; o.colA = a.col.p; o.valA = a.v32.p;
   o.off1 = m1.off.p; o.col1 = m1.col.p; o.val1 = m1.v32.p;
   o.off2 = m2.off.p; o.col2 = m2.col.p; o.val2 = m2.v32.p;
+  o.off1r = mr.off.p; o.col1r = mr.col.p; o.val1r = mr.v32.p;
   o.dmat = t ? h->dinvT32.p : h->dinv32.p;
   o.vec = &h->v32;
   return o;
 }
 
 // Runs the iteration loop of an already initialised Ctl (after the init
-// kernels), as a graph or host-driven, then the x fix-up.
+// kernels), as a graph or host-driven, then the x fix-up. b: the run's
+// right-hand side in the device numbering (only the head's rows are read,
+// by the reduced form).
 template <typename V, typename T>
-int run_loop(Handle *h, bool transpose, int maxit, long long &launches, bool ru = false) {
+int run_loop(Handle *h, bool transpose, int maxit, long long &launches, const T *b, bool ru = false) {
   Ops<V, T> o = make_ops<V, T>(h, transpose);
   Ops<double, double> o64 = make_ops<double, double>(h, transpose);
   const Ops<double, double> *ru64 = ru ? &o64 : nullptr;
   const int fp32 = sizeof(T) == 4 ? 1 : 0, ti = transpose ? 1 : 0;
-  const int n = 3 * h->an.nb;
+  const bool red = reduced_run(h, ru);
+  const int n0 = red ? 3 * h->an.color_ptr[1] : 0, n = 3 * h->an.nb - n0;
+  if (red) reduced_start(h, o, launches);
   if (h->opt.use_graph) {
     cudaGraphExec_t &gx = ru ? h->graph_ru[ti] : h->graph[fp32][ti];
     if (!gx) {
@@ -597,8 +725,9 @@ int run_loop(Handle *h, bool transpose, int maxit, long long &launches, bool ru 
     // host-driven: enqueue two iterations, then look at the done flag
     for (int it = 0; it <= maxit + 1; it += 2) {
       int l = 0;
-      enqueue_iteration(h, h->st, o, 0ull, l, ru64);
-      enqueue_iteration(h, h->st, o, 0ull, l, ru64);
+      for (int k = 0; k < 2; ++k)
+        if (red) enqueue_reduced(h, h->st, o, 0ull, l);
+        else enqueue_iteration(h, h->st, o, 0ull, l, ru64);
       h->per_iter[ti] = l / 2;
       launches += l;
       CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
@@ -606,8 +735,15 @@ int run_loop(Handle *h, bool transpose, int maxit, long long &launches, bool ru 
       if (h->h_ctl->done) break;
     }
   }
-  k_finish_x<T><<<grid_for(h, n), kThreads, 0, h->st>>>(h->ctl.p, n, o.vec->x.p, o.vec->ph.p);
+  k_finish_x<T><<<grid_for(h, n), kThreads, 0, h->st>>>(h->ctl.p, n, o.vec->x.p + n0,
+                                                        o.vec->ph.p + n0);
   launches += 1;
+  if (red) {
+    const int rows = n0 / 3;
+    k_finish_head<V, T><<<(rows + kThreads - 1) / kThreads, kThreads, 0, h->st>>>(
+        h->ctl.p, rows, transpose, o.off2, o.col2, o.val2, o.dmat, b, o.vec->rt.p, o.vec->x.p);
+    launches += 1;
+  }
   CK(last_error(h));
   return GBILU_OK;
 }
@@ -692,16 +828,10 @@ void release_device(Handle *h) {
       if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   for (auto &g : h->graph_ru)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-  for (DevMat *m : {&h->A, &h->L, &h->U, &h->At, &h->Ut, &h->Lt}) m->release();
-  for (int f = 0; f < 2; ++f)
-    for (int t = 0; t < 2; ++t) {
-      h->stage_tab[f][t].release();
-      h->stage_cnt[f][t].release();
-      h->ring_tab[f][t].release();
-      h->ring_cnt[f][t].release();
-      h->stage[f][t] = StagePlan{nullptr, nullptr, 0, 0, 0, 0, nullptr, nullptr, 0};
-      h->stage_bytes[f][t] = 0;
-    }
+  for (DevMat *m : {&h->A, &h->L, &h->U, &h->At, &h->Ut, &h->Lt, &h->Lr, &h->Utr}) m->release();
+  for (auto &red : h->sweep)
+    for (auto &prec : red)
+      for (auto &sw : prec) sw.release();
   h->pdiag.release(); h->bad.release(); h->pbuf.release(); h->vals_in.release();
   h->dinvp.release();
   h->srows.release(); h->perm.release(); h->iperm.release(); h->dperm.release();
@@ -770,7 +900,8 @@ int setup_device(Handle *h) {
   CK(cudaMemcpy(h->psrc.p, an.psrc.data(), an.nnzb * sizeof(int), cudaMemcpyHostToDevice));
   for (auto pr : {std::make_pair(&an.A, &h->A), std::make_pair(&an.L, &h->L),
                   std::make_pair(&an.U, &h->U), std::make_pair(&an.At, &h->At),
-                  std::make_pair(&an.Ut, &h->Ut), std::make_pair(&an.Lt, &h->Lt)}) {
+                  std::make_pair(&an.Ut, &h->Ut), std::make_pair(&an.Lt, &h->Lt),
+                  std::make_pair(&an.Lr, &h->Lr), std::make_pair(&an.Utr, &h->Utr)}) {
     int rc = upload_mat(h, *pr.first, *pr.second);
     if (rc) return rc;
   }
@@ -797,25 +928,31 @@ int setup_device(Handle *h) {
     CK(h->dinvp.alloc((size_t)an.nb * 9));
     h->device_bytes += (size_t)an.nnzb * 9 * 16 + (size_t)an.nb * 76;
   }
-  for (int f = 0; f < 2; ++f) {
-    for (int t = 0; t < 2; ++t) {
-      h->steps[f][t] = make_steps(an, t != 0);
-      h->phases[f][t] = phase_list(h->steps[f][t]);
-    }
-  }
+  for (int red = 0; red < 2; ++red)
+    for (int f = 0; f < 2; ++f)
+      for (int t = 0; t < 2; ++t) {
+        Handle::Sweep &sw = h->sweep[red][f][t];
+        if (red && an.ncolors == 1) sw.steps.clear();
+        else sw.steps = make_steps(an, t != 0, red != 0);
+        sw.phases = phase_list(sw.steps);
+      }
   h->coop_grid64 = coop_grid<double, double>(h);
   h->coop_grid32 = coop_grid<float, float>(h);
   if (an.ncolors <= kMaxPhases / 2) {
     for (int t = 0; t < 2; ++t) {
-      int rc = build_stage_plan<double, double>(h, 0, t, h->coop_grid64);
+      int rc = build_stage_plan<double, double, false>(h, 0, t, h->coop_grid64);
+      if (rc) return rc;
+      rc = build_stage_plan<double, double, true>(h, 0, t, h->coop_grid64);
       if (rc) return rc;
       if (h->with_32) {
-        rc = build_stage_plan<float, float>(h, 1, t, h->coop_grid32);
+        rc = build_stage_plan<float, float, false>(h, 1, t, h->coop_grid32);
+        if (rc) return rc;
+        rc = build_stage_plan<float, float, true>(h, 1, t, h->coop_grid32);
         if (rc) return rc;
       }
     }
   }
-  h->device_bytes += nd * 16 + (h->with_32 ? nd * 8 : 0) + n * 8 * 12 + (h->with_32 ? n * 4 * 9 : 0) +
+  h->device_bytes += nd * 16 + (h->with_32 ? nd * 8 : 0) + n * 8 * 14 + (h->with_32 ? n * 4 * 11 : 0) +
                      (size_t)an.nnzb * 16 + (size_t)an.nb * 16;
   return GBILU_OK;
 }
@@ -823,6 +960,7 @@ int setup_device(Handle *h) {
 // Sliced values of one matrix (FP64 and, in the mixed mode, FP32) from
 // per-block device values.
 void fill_mat_device(Handle *h, DevMat &m, const double *src) {
+  if (m.slots == 0) return;
   const int g = grid_for(h, m.slots * 32);
   k_fill_sliced<double><<<g, kThreads, 0, h->st>>>(m.slots, m.vsrc.p, m.transpose ? 1 : 0, src, m.v64.p);
   if (h->with_32)
@@ -859,6 +997,8 @@ int factor_device(Handle *h, const double *vals) {
   fill_mat_device(h, h->U, h->pbuf.p);
   fill_mat_device(h, h->Lt, h->pbuf.p);
   fill_mat_device(h, h->Ut, h->pbuf.p);
+  fill_mat_device(h, h->Lr, h->pbuf.p);
+  fill_mat_device(h, h->Utr, h->pbuf.p);
   const int gd = grid_for(h, (long long)an.S * 32);
   k_fill_diag<double><<<gd, kThreads, 0, h->st>>>(an.S, h->srows.p, h->dperm.p, 0, h->dinvp.p, h->dinv64.p);
   k_fill_diag<double><<<gd, kThreads, 0, h->st>>>(an.S, h->srows.p, h->dperm.p, 1, h->dinvp.p, h->dinvT64.p);
@@ -897,11 +1037,12 @@ int solve64(Handle *h, bool transpose, double tol, int maxit, Ctl &out, long lon
   spmv<double, double, SPMV_PLAIN>(h, h->st, o, w.x.p, w.r.p, nullptr, l, h->x0nz.p);
   launches += l;
   if (b_ready) CK(cudaStreamWaitEvent(h->st, b_ready, 0));
+  const int nh = reduced_run(h, false) ? 3 * h->an.color_ptr[1] : 0;
   k_init_resid<double><<<reduce_grid(h, n), kThreads, 0, h->st>>>(
-      h->ctl.p, n, b_in ? b_in : h->b64.p, b_in ? h->perm.p : nullptr, w.r.p, w.rt.p, w.p.p,
-      h->partials.p);
+      h->ctl.p, n, nh, b_in ? b_in : h->b64.p, b_in ? h->perm.p : nullptr, h->b64.p, w.r.p, w.rt.p,
+      w.p.p, w.base.p, h->partials.p);
   launches += 1;
-  int rc = run_loop<double, double>(h, transpose, maxit, launches);
+  int rc = run_loop<double, double>(h, transpose, maxit, launches, h->b64.p);
   if (rc) return rc;
   CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
   if (!sync) return GBILU_OK;
@@ -930,7 +1071,7 @@ int solve_mixed_ru(Handle *h, bool transpose, double tol, int maxit, gbilu_resul
   k_ru_init<<<reduce_grid(h, n), kThreads, 0, h->st>>>(h->ctl.p, n, h->opt.ru_delta, w.r.p, f.r.p,
                                                        f.rt.p, f.p.p, f.x.p, h->partials.p);
   launches += l + 2;
-  int rc = run_loop<float, float>(h, transpose, maxit, launches, true);
+  int rc = run_loop<float, float>(h, transpose, maxit, launches, nullptr, true);
   if (rc) return rc;
   // a stop after a first half owes xc += alpha p^ (k_finish_x in run_loop);
   // then the remaining FP32 correction goes into x
@@ -949,7 +1090,7 @@ int solve_mixed_ru(Handle *h, bool transpose, double tol, int maxit, gbilu_resul
     k_ctl_init<<<1, 32, 0, h->st>>>(outer, 0.0, 1, 0, 0ull);
     const int S = h->an.S;
     k_spmv<double, double, SPMV_RESID><<<std::min((S + kWarps - 1) / kWarps, 2 * h->sm_count),
-                                         kThreads, 0, h->st>>>(outer, S, h->srows.p, o64.offA,
+                                         kThreads, 0, h->st>>>(outer, 0, S, h->srows.p, o64.offA,
                                                                o64.colA, o64.valA, w.x.p, w.r.p,
                                                                h->b64.p, h->partials.p);
     launches += 2;
@@ -982,7 +1123,7 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
     k_ctl_init<<<1, 32, 0, h->st>>>(outer, 0.0, 1, 0, 0ull);
     const int S = h->an.S;
     k_spmv<double, double, SPMV_RESID><<<std::min((S + kWarps - 1) / kWarps, 2 * h->sm_count), kThreads, 0, h->st>>>(
-        outer, S, h->srows.p, o64.offA, o64.colA, o64.valA, w.x.p, w.r.p, h->b64.p, h->partials.p);
+        outer, 0, S, h->srows.p, o64.offA, o64.colA, o64.valA, w.x.p, w.r.p, h->b64.p, h->partials.p);
     launches += 2;
     CK(cudaMemcpyAsync(h->h_ctl, outer, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
@@ -1016,10 +1157,12 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
     // (staged in f.t, which the inner run overwrites only after reading it)
     k_scale_convert<<<g, kThreads, 0, h->st>>>(n, 1.0 / nrm, w.r.p, f.t.p);
     k_ctl_init<<<1, 32, 0, h->st>>>(h->ctl.p, h->opt.inner_tol, 0, left, tmo);
-    k_init_rhs<float><<<reduce_grid(h, n), kThreads, 0, h->st>>>(h->ctl.p, n, f.t.p, f.r.p, f.rt.p,
-                                                                 f.p.p, f.x.p, h->partials.p);
+    const int nh = reduced_run(h, false) ? 3 * h->an.color_ptr[1] : 0;
+    k_init_rhs<float><<<reduce_grid(h, n), kThreads, 0, h->st>>>(
+        h->ctl.p, n, nh, f.t.p, f.r.p, f.rt.p, f.p.p, f.x.p, f.base.p, h->partials.p);
     launches += 3;
-    rc = run_loop<float, float>(h, transpose, left, launches);
+    // the inner run starts from x = 0: its right-hand side is rt
+    rc = run_loop<float, float>(h, transpose, left, launches, f.rt.p);
     if (rc) return rc;
     CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
@@ -1054,12 +1197,77 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
 
 namespace gbilu {
 namespace {
-// One of the iteration's kernels for gbilu_bench_kernel (kind 4: SpMV with
-// the alpha dot, 5: SpMV with the omega dots, 6-8: update_s/r/p).
+// Algorithmic bytes of one iteration's kernels as they run (every operand
+// read or written once, x gathers counted once).
+struct IterBytes {
+  double apply, spmv, update_s, update_r, update_p;
+  double total() const { return 2 * apply + 2 * spmv + update_s + update_r + update_p; }
+};
+IterBytes iter_bytes(const Handle *h, double sv, double sx) {
+  const Analysis &an = h->an;
+  const double si = 4.0, blk = 9 * sv + si, nb = an.nb, row = 3 * sx;
+  IterBytes b;
+  if (!reduced_run(h, false)) {
+    b.apply = ((double)an.nnzb_l + an.nnzb_u) * blk + 2 * (nb + 1) * si + nb * 9 * sv + 4 * nb * row;
+    b.spmv = an.nnzb * blk + (nb + 1) * si + 3 * nb * row;
+    b.update_s = 3 * nb * row;
+    b.update_r = 8 * nb * row;
+    b.update_p = 4 * nb * row;
+    return b;
+  }
+  const double n0 = an.color_ptr[1], nt = nb - n0, n1 = an.color_ptr[2] - n0, split = an.split[1];
+  const double a0 = an.prowptr[an.color_ptr[1]], u0 = a0 - n0;   // the head's blocks of A and U
+  // apply: the head's U blocks, the L and U blocks inside the tail, D of
+  // every row but color 1's final ones; base and result of the head, the
+  // tail's result gathered
+  b.apply = (u0 + (an.nnzb_l - u0) + (an.nnzb_u - u0)) * blk + (nb - n1 + split) * 9 * sv +
+            (n0 + 1) * si + (2 * n0 + nt) * row;
+  b.spmv = (an.nnzb - a0) * blk + (nt + 1) * si + (nb + 2 * nt) * row;
+  const double d1 = (n1 - split) * 9 * sv;
+  b.update_s = 5 * nt * row + d1;    // r, v, base -> s, s^ of color 1
+  b.update_r = 8 * nt * row;
+  b.update_p = 6 * nt * row + d1;    // r, v, p, base -> p, p^ of color 1
+  return b;
+}
+
+// One of the iteration's kernels for gbilu_bench_kernel (kind 3: the
+// iteration's apply, 4: SpMV with the alpha dot, 5: SpMV with the omega dots,
+// 6-8: update_s/r/p), over the rows that it runs on.
 template <typename V, typename T>
 void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, int &l) {
   Vecs<T> &w = *o.vec;
-  if (kind == 4) {
+  if (reduced_run(h, false)) {
+    const Tail<V, T> tp = make_tail(h, o, w.ph.p), ts = make_tail(h, o, w.sh.p);
+    const int S0 = tp.slice1, n0 = 3 * tp.row0, nt = 3 * tp.rows;
+    Ctl *c = h->ctl.p;
+    if (kind == 3) {
+      apply_prec<V, T, true>(h, h->st, o, w.p.p, w.ph.p, l, &c->cp);
+      return;
+    }
+    if (kind == 4) {
+      spmv<V, T, SPMV_ALPHA>(h, h->st, o, w.ph.p, w.v.p, w.rt.p, l, nullptr, S0);
+      return;
+    }
+    if (kind == 5) {
+      spmv<V, T, SPMV_OMEGA>(h, h->st, o, w.ph.p, w.t.p, w.s.p, l, nullptr, S0);
+      return;
+    }
+    if (kind == 6)
+      k_tail_s<V, T><<<row_grid(h, tp.rows, GBILU_REDUCE_CTAS_PER_SM), kThreads, 0, h->st>>>(
+          c, ts, w.r.p, w.v.p, w.s.p, h->partials.p);
+    else if (kind == 7)
+      k_update_r<T><<<reduce_grid(h, nt), kThreads, 0, h->st>>>(
+          c, nt, w.x.p + n0, w.ph.p + n0, w.sh.p + n0, w.s.p + n0, w.t.p + n0, w.rt.p + n0,
+          w.r.p + n0, h->partials.p);
+    else
+      k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, h->st>>>(c, tp, w.r.p, w.v.p, w.p.p,
+                                                                       w.rt.p, 0ull);
+    ++l;
+    return;
+  }
+  if (kind == 3) {
+    apply_prec<V, T>(h, h->st, o, w.p.p, w.ph.p, l);
+  } else if (kind == 4) {
     spmv<V, T, SPMV_ALPHA>(h, h->st, o, w.p.p, w.v.p, w.rt.p, l);
   } else if (kind == 5) {
     spmv<V, T, SPMV_OMEGA>(h, h->st, o, w.p.p, w.t.p, w.s.p, l);
@@ -1223,6 +1431,8 @@ int gbilu_factor(void *handle, const double *vals) {
     if ((rc = upload_vals(h, an.At, h->pvals.data(), h->At))) return rc;
     if ((rc = upload_vals(h, an.Ut, h->lu.data(), h->Ut))) return rc;
     if ((rc = upload_vals(h, an.Lt, h->lu.data(), h->Lt))) return rc;
+    if ((rc = upload_vals(h, an.Lr, h->lu.data(), h->Lr))) return rc;
+    if ((rc = upload_vals(h, an.Utr, h->lu.data(), h->Utr))) return rc;
     if ((rc = upload_diag(h, false, h->dinv64, h->dinv32))) return rc;
     if ((rc = upload_diag(h, true, h->dinvT64, h->dinvT32))) return rc;
   }
@@ -1545,9 +1755,9 @@ int gbilu_get_stats(void *handle, gbilu_stats *s) {
   s->color_ms = h->color_ms;
   s->color_on_device = h->opt.color_on_device && h->opt.device >= 0 && h->opt.coloring == 0;
   for (int p = 0; p < 2; ++p) {
-    s->ring_stages[p] = h->stage[p][0].ring_ns;
-    s->ring_stage_bytes[p] = h->stage[p][0].ring_stride;
-    s->apply_smem_bytes[p] = h->stage_bytes[p][0];
+    s->ring_stages[p] = h->sweep[0][p][0].stage.ring_ns;
+    s->ring_stage_bytes[p] = h->sweep[0][p][0].stage.ring_stride;
+    s->apply_smem_bytes[p] = h->sweep[0][p][0].stage_bytes;
   }
   for (int p = 0; p < 2; ++p) {
     const double sv = p ? 4.0 : 8.0, sx = sv, si = 4.0;
@@ -1555,11 +1765,7 @@ int gbilu_get_stats(void *handle, gbilu_stats *s) {
     const double nlu = (double)an.nnzb_l + an.nnzb_u;
     s->alg_bytes_spmv[p] = an.nnzb * (9 * sv + si) + (nb + 1) * si + 2 * n * sx;
     s->alg_bytes_ilu[p] = nlu * (9 * sv + si) + 2 * (nb + 1) * si + nb * 9 * sv + 4 * n * sx;
-    // fused vector kernels of one iteration: update_s (r, v -> s),
-    // update_r (x, p^, s^, s, t, rt -> x, r), update_p (r, v, p -> p)
-    // and the dot operands of the two SpMV epilogues (rt, s)
-    const double vec = 17.0 * n * sx;
-    s->alg_bytes_iter[p] = 2 * s->alg_bytes_spmv[p] + 2 * s->alg_bytes_ilu[p] + vec;
+    s->alg_bytes_iter[p] = iter_bytes(h, sv, sx).total();
   }
   return GBILU_OK;
 }
@@ -1652,7 +1858,7 @@ int gbilu_ilu_trace(void *handle, int fp32, int transpose, double *us, int *rows
   if (h->an.ncolors > kMaxPhases / 2) return h->fail(GBILU_BAD_INPUT, "too many colors to trace");
   CK(cudaSetDevice(h->opt.device));
   const int t = transpose ? 1 : 0;
-  const PhaseList &pl = h->phases[fp32 ? 1 : 0][t];
+  const PhaseList &pl = h->sweep[0][fp32 ? 1 : 0][t].phases;
   const int n = 3 * h->an.nb;
   CK(cudaMemsetAsync(h->v64.p.p, 0, n * sizeof(double), h->st));
   if (h->with_32) CK(cudaMemsetAsync(h->v32.p.p, 0, n * sizeof(float), h->st));
@@ -1685,8 +1891,8 @@ int gbilu_bench_kernel(void *handle, int which, int reps, double *avg_ms, double
   if (!h) return GBILU_BAD_INPUT;
   int rc = check_solve_ready(h);
   if (rc) return rc;
-  if (which < 0 || which > 13 || reps <= 0) return h->fail(GBILU_BAD_INPUT, "bad kernel id or reps");
-  const bool fp32 = which == 2 || which == 3 || which >= 9;
+  if (which < 0 || which > 15 || reps <= 0) return h->fail(GBILU_BAD_INPUT, "bad kernel id or reps");
+  const bool fp32 = which == 2 || which == 3 || (which >= 9 && which != 14);
   if (fp32 && !h->with_32) return h->fail(GBILU_BAD_INPUT, "FP32 kernels need GBILU_MIXED");
   CK(cudaSetDevice(h->opt.device));
   gbilu_stats st;
@@ -1709,7 +1915,7 @@ int gbilu_bench_kernel(void *handle, int which, int reps, double *avg_ms, double
     Vecs<double> &w = h->v64;
     std::vector<double> xv(n);
     int k = 0;
-    for (DevBuf<double> *b : {&w.x, &w.r, &w.rt, &w.ph, &w.v, &w.s, &w.sh, &w.t, &w.y}) {
+    for (DevBuf<double> *b : {&w.x, &w.r, &w.rt, &w.ph, &w.v, &w.s, &w.sh, &w.t, &w.y, &w.base}) {
       ++k;
       for (int i = 0; i < n; ++i) {
         z ^= z << 13; z ^= z >> 7; z ^= z << 17;
@@ -1720,20 +1926,20 @@ int gbilu_bench_kernel(void *handle, int which, int reps, double *avg_ms, double
     }
     if (h->with_32) {
       Vecs<float> &f = h->v32;
-      DevBuf<double> *src[9] = {&w.x, &w.r, &w.rt, &w.ph, &w.v, &w.s, &w.sh, &w.t, &w.y};
-      DevBuf<float> *dst[9] = {&f.x, &f.r, &f.rt, &f.ph, &f.v, &f.s, &f.sh, &f.t, &f.y};
-      for (int j = 0; j < 9; ++j)
+      DevBuf<double> *src[10] = {&w.x, &w.r, &w.rt, &w.ph, &w.v, &w.s, &w.sh, &w.t, &w.y, &w.base};
+      DevBuf<float> *dst[10] = {&f.x, &f.r, &f.rt, &f.ph, &f.v, &f.s, &f.sh, &f.t, &f.y, &f.base};
+      for (int j = 0; j < 10; ++j)
         k_scale_convert<<<g, kThreads, 0, h->st>>>(n, 1.0, src[j]->p, dst[j]->p);
     }
   }
-  // the iteration's other kernels (4-8 FP64, 9-13 FP32): the SpMV with the
-  // alpha dot, the SpMV with the omega dots, update_s, update_r, update_p,
-  // with solver scalars that never stop the run
-  const int kind = which >= 9 ? which - 5 : which;
+  // the iteration's kernels as they run: 4-8 FP64, 9-13 FP32 (SpMV with the
+  // alpha dot, SpMV with the omega dots, update_s, update_r, update_p) and
+  // the apply, 14 FP64, 15 FP32, with solver scalars that never stop the run
+  const int kind = which >= 14 ? 3 : which >= 9 ? which - 5 : which;
   if (which >= 4) k_ctl_bench<<<1, 32, 0, h->st>>>(h->ctl.p);
   const int gr = reduce_grid(h, n);
   auto run = [&](int &l) {
-    if (which >= 9) {
+    if (which >= 9 && fp32) {
       iter_kernel<float, float>(h, kind, make_ops<float, float>(h, false), n, g, gr, l);
     } else if (which >= 4) {
       iter_kernel<double, double>(h, kind, make_ops<double, double>(h, false), n, g, gr, l);
@@ -1763,14 +1969,10 @@ int gbilu_bench_kernel(void *handle, int which, int reps, double *avg_ms, double
   CK(cudaEventElapsedTime(&ms, h->e0, h->e1));
   if (avg_ms) *avg_ms = ms / reps;
   if (alg_bytes) {
-    const double sx = fp32 ? 4.0 : 8.0, nn = n;
-    const int p = fp32 ? 1 : 0;
-    // each operand read or written once: the SpMV plus its dot operand
-    // (alpha: rt; omega: s), update_s r, v -> s; update_r x, p^, s^, s, t,
-    // rt -> x, r; update_p r, v, p -> p
-    const double by[5] = {st.alg_bytes_spmv[p] + nn * sx, st.alg_bytes_spmv[p] + nn * sx,
-                          3 * nn * sx, 8 * nn * sx, 4 * nn * sx};
-    *alg_bytes = which >= 4 ? by[kind - 4]
+    const double sx = fp32 ? 4.0 : 8.0;
+    const IterBytes ib = iter_bytes(h, sx, sx);
+    const double by[6] = {ib.apply, ib.spmv, ib.spmv, ib.update_s, ib.update_r, ib.update_p};
+    *alg_bytes = which >= 4 ? by[kind - 3]
                             : (which == 0 || which == 2) ? st.alg_bytes_spmv[which / 2]
                                                          : st.alg_bytes_ilu[which / 2];
   }

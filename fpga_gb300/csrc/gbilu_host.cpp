@@ -209,6 +209,21 @@ Csr transpose_csr(int nb, const Csr &m) {
   return t;
 }
 
+// The blocks of m whose column is c0 or later.
+Csr from_column(int nb, const Csr &m, int c0) {
+  Csr r;
+  r.rowptr.assign(static_cast<size_t>(nb) + 1, 0);
+  for (int i = 0; i < nb; ++i) {
+    for (int k = m.rowptr[i]; k < m.rowptr[i + 1]; ++k)
+      if (m.col[k] >= c0) {
+        r.col.push_back(m.col[k]);
+        r.src.push_back(m.src[k]);
+      }
+    r.rowptr[i + 1] = static_cast<int>(r.col.size());
+  }
+  return r;
+}
+
 }  // namespace
 
 std::string analyze(int nb, const int *rowptr, const int *colind, Analysis &an,
@@ -338,10 +353,13 @@ std::string analyze(int nb, const int *rowptr, const int *colind, Analysis &an,
   slice_matrix(an, a, false, an.A);
   slice_matrix(an, l, false, an.L);
   slice_matrix(an, u, false, an.U);
+  slice_matrix(an, from_column(nb, l, an.color_ptr[1]), false, an.Lr);
   if (with_transposes) {
     slice_matrix(an, transpose_csr(nb, a), true, an.At);
     // rows of U^T hold U_ij^T (i < j): lower part; rows of L^T: upper part
-    slice_matrix(an, transpose_csr(nb, u), true, an.Ut);
+    const Csr ut = transpose_csr(nb, u);
+    slice_matrix(an, ut, true, an.Ut);
+    slice_matrix(an, from_column(nb, ut, an.color_ptr[1]), true, an.Utr);
     slice_matrix(an, transpose_csr(nb, l), true, an.Lt);
   }
   return "";

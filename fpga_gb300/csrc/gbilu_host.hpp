@@ -60,6 +60,7 @@ struct Analysis {
   std::vector<int> slice_row0, slice_len; // [S]
   SlicedMatrix A, L, U;                   // forward operators
   SlicedMatrix At, Ut, Lt;                // transposed operators (adjoint)
+  SlicedMatrix Lr, Utr;                   // L and U^T without color 0's columns
 };
 
 // Greedy first-fit coloring in natural row order; returns the color count.

@@ -55,6 +55,13 @@ struct Ctl {
   double rho_prev;                // rho before the last update_r (for beta after a replacement)
   double true_norm;               // ||b - A x|| of the last replacement (FP64)
   int replacements;
+  // reduced iteration: the color-0 rows of r, p, s are cr, cp, cs times those
+  // of the initial residual, whose squared norm is head_rr (0: not reduced)
+  double cr, cp, cs, head_rr;
+  double crt, rt_norm;            // the same for rt, and ||rt||
+  int reduced;                    // the run is reduced
+  int restart;                    // rt = r from here on (see k_update_r)
+  int x_moved;                    // a second half has advanced x
   unsigned long long phase_ns[kMaxPhases + 1];   // traced ILU apply: phase starts
   unsigned int step_next[kMaxPhases];   // single-launch apply: next slice of a large step
 };
@@ -231,6 +238,11 @@ __device__ __forceinline__ void push_norm(Ctl *c, double nrm) {
   c->norm = nrm;
 }
 
+// c times the head's squared norm; 0 when nothing is reduced, whatever c is
+__device__ __forceinline__ double head_part(const Ctl *ctl, double c) {
+  return ctl->head_rr != 0.0 ? c * ctl->head_rr : 0.0;
+}
+
 __device__ __forceinline__ void stop(Ctl *c, int status, int stop_half) {
   c->status = status;
   c->stop_half = stop_half;
@@ -271,6 +283,13 @@ __global__ void k_ctl_init(Ctl *c, double tol, int absolute, int maxit,
     c->rho_prev = 0.0;
     c->true_norm = 0.0;
     c->replacements = 0;
+    c->cr = c->cp = 1.0;
+    c->cs = 0.0;
+    c->head_rr = 0.0;
+    c->crt = 1.0;
+    c->rt_norm = 0.0;
+    c->reduced = c->restart = 0;
+    c->x_moved = 0;
     for (int q = 0; q < kMaxPhases; ++q) c->step_next[q] = 0u;
   }
 }
@@ -287,6 +306,9 @@ __global__ void k_ctl_bench(Ctl *c) {
     c->k = 0;
     c->done = 0;
     c->ru_mode = 0;
+    c->cr = c->cp = c->cs = c->crt = 1.0;
+    c->head_rr = 0.0;
+    c->reduced = c->restart = 0;
   }
 }
 
@@ -294,9 +316,14 @@ __global__ void k_ctl_bench(Ctl *c) {
 // r = b - A x0, rho = ||r||^2, the "already solved" test and the absolute
 // stopping bound. MODE 0: r = b - A x (vals/x given); MODE 1: r = b (x0 = 0,
 // used by the inner solves of iterative refinement).
+// head_rr: the color-0 rows' share of rr (reduced iteration; else 0).
 template <typename T>
-__device__ __forceinline__ void finish_init(Ctl *c, double rr) {
+__device__ __forceinline__ void finish_init(Ctl *c, double rr, int reduced = 0,
+                                            double head_rr = 0.0) {
   const double n0 = sqrt(rr);
+  c->reduced = reduced;
+  c->head_rr = head_rr;
+  c->rt_norm = n0;
   c->norm0 = n0;
   c->norm = n0;
   c->norms[0] = n0;
@@ -392,7 +419,9 @@ __device__ __forceinline__ void row_blocks(const int *__restrict__ col, const V 
 
 enum SpmvMode { SPMV_PLAIN = 0, SPMV_RESID = 1, SPMV_ALPHA = 2, SPMV_OMEGA = 3, SPMV_TRUE = 4 };
 
-// y = A x over all slices. RESID: y = b - A x, ||y||^2 -> init. ALPHA:
+// y = A x over the slices S0 .. S-1 (the reduced iteration leaves out color
+// 0's, whose rows of A x are known: their part of the dots is cp or cs times
+// the initial residual's). RESID: y = b - A x, ||y||^2 -> init. ALPHA:
 // (y, w) -> alpha = rho/(y,w) (step 5). OMEGA: (y, w), (y, y) ->
 // omega = (y,w)/(y,y) (step 10). TRUE: y = b - A x and ||y|| into
 // Ctl::true_norm, only when a residual replacement is due.
@@ -412,7 +441,7 @@ enum SpmvMode { SPMV_PLAIN = 0, SPMV_RESID = 1, SPMV_ALPHA = 2, SPMV_OMEGA = 3, 
 // without reading A (the initial residual of a solve from x0 = 0).
 template <typename V, typename T, int MODE>
 __global__ void __launch_bounds__(kThreads, sizeof(V) == 4 ? GBILU_SPMV32_MINB : GBILU_SPMV64_MINB)
-k_spmv(Ctl *ctl, int S, const int2 *__restrict__ srows, const int *__restrict__ off,
+k_spmv(Ctl *ctl, int S0, int S, const int2 *__restrict__ srows, const int *__restrict__ off,
        const int *__restrict__ col, const V *__restrict__ val, const T *__restrict__ x,
        T *__restrict__ y, const T *__restrict__ w, double *partials,
        const int *x_nonzero = nullptr) {
@@ -443,7 +472,7 @@ k_spmv(Ctl *ctl, int S, const int2 *__restrict__ srows, const int *__restrict__ 
   // FP32 matrices only: the FP64 SpMV is bound by the FP64 unit
   constexpr bool PF = sizeof(V) == 4;
 #endif
-  int s = blockIdx.x * kWarps + (threadIdx.x >> 5);
+  int s = S0 + blockIdx.x * kWarps + (threadIdx.x >> 5);
   int2 sr_n = make_int2(0, 0);
   int o_n = 0, e_n = 0;
   if (AHEAD && s < S) { sr_n = srows[s]; o_n = off[s]; e_n = off[s + 1]; }
@@ -510,20 +539,24 @@ k_spmv(Ctl *ctl, int S, const int2 *__restrict__ srows, const int *__restrict__ 
   } else if (MODE == SPMV_ALPHA) {
     double v[1] = {d1}, tot[1];
     if (grid_sum<1>(v, partials, &ctl->counter[1], tot) && threadIdx.x == 0) {
-      const double a = ctl->rho / tot[0];
-      ctl->dots[0] = tot[0];
+      const double vrt = tot[0] + head_part(ctl, ctl->cp * ctl->crt);
+      const double a = ctl->rho / vrt;
+      ctl->dots[0] = vrt;
       ctl->alpha = a;
-      if (tot[0] == 0.0 || !finite(a)) stop(ctl, ST_BREAKDOWN, 0);
+      ctl->cs = fma(-a, ctl->cp, ctl->cr);
+      if (vrt == 0.0 || !finite(a)) stop(ctl, ST_BREAKDOWN, 0);
     }
   } else {
     double v[2] = {d1, d2}, tot[2];
     if (grid_sum<2>(v, partials, &ctl->counter[2], tot) && threadIdx.x == 0) {
-      const double om = tot[0] / tot[1];
-      ctl->dots[1] = tot[0];
-      ctl->dots[2] = tot[1];
+      const double hh = head_part(ctl, ctl->cs * ctl->cs);
+      const double ts = tot[0] + hh, tt = tot[1] + hh;
+      const double om = ts / tt;
+      ctl->dots[1] = ts;
+      ctl->dots[2] = tt;
       ctl->omega = om;
       // half 1 already advanced x by alpha p^: keep it on a stop here
-      if (tot[1] == 0.0 || !finite(om)) stop(ctl, ST_BREAKDOWN, 1);
+      if (tt == 0.0 || !finite(om)) stop(ctl, ST_BREAKDOWN, 1);
     }
   }
 }
@@ -551,6 +584,8 @@ struct Phase {
   int to_y;       // first sweep: the result goes to ybuf ...
   int final0;     // ... and rows from final0 on are final: hat = [D] result
   int final_d;    //     with D = D^-1 (forward) or the identity (adjoint)
+  int own_base;   // reduced iteration: own rows read coef * base (1), or
+                  // src + coef * base (2), see k_tail_s
   int staged;     // the step's matrix rows come from shared memory
   int local_after;  // this step and the next have one slice each and run on
                     // CTA 0: a CTA barrier between them instead of a grid one
@@ -584,29 +619,48 @@ __device__ __forceinline__ void apply_dp(const V *d, int l, T &a0, T &a1, T &a2)
 }
 
 // Stores one row's result as the phase says (d: the slot of the row's D
-// block, l: the row's lane).
+// block, l: the row's lane). Rows from final0 on have no neighbour of a
+// higher color, so nothing reads their y: only hat is written.
 template <typename V, typename T, bool GLOBAL>
 __device__ __forceinline__ void phase_store(const Phase &P, int row, const V *d, int l, T a0,
                                             T a1, T a2, T *ybuf, T *hat) {
   if (P.has_d) apply_dp<V, T, GLOBAL>(d, l, a0, a1, a2);
   if (P.to_y) {
-    ybuf[3 * row] = a0; ybuf[3 * row + 1] = a1; ybuf[3 * row + 2] = a2;
-    if (row < P.final0) return;
+    if (row < P.final0) {
+      ybuf[3 * row] = a0; ybuf[3 * row + 1] = a1; ybuf[3 * row + 2] = a2;
+      return;
+    }
     if (P.final_d) apply_dp<V, T, GLOBAL>(d, l, a0, a1, a2);
   }
   hat[3 * row] = a0; hat[3 * row + 1] = a1; hat[3 * row + 2] = a2;
+}
+
+// The own values of a reduced step: coef * base, or src + coef * base (a
+// holds what own pointed to).
+template <typename T>
+__device__ __forceinline__ void scale_own(const Phase &P, const T *__restrict__ base, int row,
+                                          T coef, T &a0, T &a1, T &a2) {
+  if (P.own_base == 1) {
+    a0 *= coef; a1 *= coef; a2 *= coef;
+  } else {
+    a0 = fma(coef, base[3 * row], a0);
+    a1 = fma(coef, base[3 * row + 1], a1);
+    a2 = fma(coef, base[3 * row + 2], a2);
+  }
 }
 
 #ifndef GBILU_D_PREFETCH
 #define GBILU_D_PREFETCH 1
 #endif
 // One row of a step, one thread: a = own_i - sum_j B_ij nbr_j, then stored.
-template <typename V, typename T, bool CG>
+// RED: steps of the reduced iteration, own rows from base (Phase::own_base).
+template <typename V, typename T, bool CG, bool RED>
 __device__ __forceinline__ void phase_row(const Phase &P, int row, int s, int lane,
                                           const int *__restrict__ off, const int *__restrict__ col,
                                           const V *__restrict__ val, const V *__restrict__ dmat,
-                                          const T *src, T *ybuf, T *hat) {
-  const T *own = P.own_y ? ybuf : src;
+                                          const T *src, T *ybuf, T *hat,
+                                          const T *__restrict__ base, T coef) {
+  const T *own = P.own_y ? ybuf : RED && P.own_base == 1 ? base : src;
   if (GBILU_D_PREFETCH && (P.has_d || (P.to_y && P.final_d && row - lane + 31 >= P.final0))) {
     // the slice's D block (9 * 32 values, one 128-byte line per lane) is
     // read at the end of the row: asked from L2 now, without registers
@@ -617,6 +671,7 @@ __device__ __forceinline__ void phase_row(const Phase &P, int row, int s, int la
   }
   const int o = off[s], wdt = off[s + 1] - o;
   T a0 = ldv<CG>(own + 3 * row), a1 = ldv<CG>(own + 3 * row + 1), a2 = ldv<CG>(own + 3 * row + 2);
+  if (RED && P.own_base) scale_own(P, base, row, coef, a0, a1, a2);
   row_blocks<V, T, true, CG, true>(col, val, o, wdt, lane, P.nbr_hat ? hat : ybuf, src, P.src_rows, a0,
                              a1, a2);
   phase_store<V, T, true>(P, row, dmat + (size_t)s * 9 * 32, lane, a0, a1, a2, ybuf, hat);
@@ -628,15 +683,17 @@ constexpr int kSmallRows = 16384;
 
 // One step per launch (the per-color mode; the same row arithmetic as the
 // single-launch apply, so both give identical bits).
-template <typename V, typename T>
+template <typename V, typename T, bool RED>
 __global__ void __launch_bounds__(kThreads, 2)
 k_phase(const Ctl *ctl, Phase P, const int *__restrict__ off, const int *__restrict__ col,
-        const V *__restrict__ val, const V *__restrict__ dmat, const T *src, T *ybuf, T *hat) {
+        const V *__restrict__ val, const V *__restrict__ dmat, const T *src, T *ybuf, T *hat,
+        const T *__restrict__ base, const double *coef) {
   if (ctl->done) return;
   const int t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= P.nrows) return;
-  phase_row<V, T, false>(P, P.row0 + t, P.slice0 + (t >> 5), t & 31, off, col, val, dmat, src,
-                         ybuf, hat);
+  const T c = RED ? (T)*coef : (T)0;
+  phase_row<V, T, false, RED>(P, P.row0 + t, P.slice0 + (t >> 5), t & 31, off, col, val, dmat, src,
+                              ybuf, hat, base, c);
 }
 
 // --------------------------------------------------------------------------
@@ -877,14 +934,14 @@ __device__ __forceinline__ bool poll_again(Ctl *ctl, unsigned int &spins) {
 // One staged row (thread per row, data in shared memory): the column
 // indices come first so that all neighbour gathers of the row are in flight
 // together. Same arithmetic as phase_row.
-template <typename V, typename T>
+template <typename V, typename T, bool RED>
 __device__ __forceinline__ void staged_row(const Phase &P, int row, int lane, int w, const V *sv,
                                            const int *sc, const V *sd, const T *src, T *ybuf,
-                                           T *hat, Ctl *ctl) {
+                                           T *hat, Ctl *ctl, const T *__restrict__ base, T coef) {
   // gathers in flight per batch (8 in FP32 spilled once the ring's state
   // was added to the kernel)
   constexpr int SB = sizeof(T) == 8 ? 4 : 6;
-  const T *own = P.own_y ? ybuf : src;
+  const T *own = P.own_y ? ybuf : RED && P.own_base == 1 ? base : src;
   const T *nbr = P.nbr_hat ? hat : ybuf;
   // only values of ybuf and hat can be sentinels: reads of the input src are
   // never checked (any bit pattern there is data)
@@ -895,6 +952,7 @@ __device__ __forceinline__ void staged_row(const Phase &P, int row, int lane, in
     a2 = ld_relaxed(own + 3 * row + 2);
   } while (P.own_y && (is_sentinel(a0) || is_sentinel(a1) || is_sentinel(a2)) &&
            poll_again(ctl, spins));
+  if (RED && P.own_base) scale_own(P, base, row, coef, a0, a1, a2);
   for (int k0 = 0; k0 < w; k0 += SB) {
     int c[SB];
     T y[SB][3];
@@ -931,9 +989,11 @@ __device__ __forceinline__ void staged_row(const Phase &P, int row, int lane, in
   }
   if (P.has_d) apply_dp<V, T, false>(sd, lane, a0, a1, a2);
   if (P.to_y) {
-    st_relaxed(ybuf + 3 * row, a0); st_relaxed(ybuf + 3 * row + 1, a1);
-    st_relaxed(ybuf + 3 * row + 2, a2);
-    if (row < P.final0) return;
+    if (row < P.final0) {
+      st_relaxed(ybuf + 3 * row, a0); st_relaxed(ybuf + 3 * row + 1, a1);
+      st_relaxed(ybuf + 3 * row + 2, a2);
+      return;
+    }
     if (P.final_d) apply_dp<V, T, false>(sd, lane, a0, a1, a2);
   }
   st_relaxed(hat + 3 * row, a0); st_relaxed(hat + 3 * row + 1, a1); st_relaxed(hat + 3 * row + 2, a2);
@@ -942,18 +1002,19 @@ __device__ __forceinline__ void staged_row(const Phase &P, int row, int lane, in
 // Component c of one staged row: own_c - sum_k B_k[c,:] y_k with the FMA
 // sequence of that component in staged_row, so a row whose three components
 // are computed by three warps gets the same bits.
-template <typename V, typename T>
+template <typename V, typename T, bool RED>
 __device__ __forceinline__ T staged_comp(const Phase &P, int c, int row, int lane, int w,
                                          const V *sv, const int *sc, const T *src, const T *ybuf,
-                                         const T *hat, Ctl *ctl) {
+                                         const T *hat, Ctl *ctl, const T *__restrict__ base, T coef) {
   constexpr int SB = sizeof(T) == 8 ? 4 : 8;
-  const T *own = P.own_y ? ybuf : src;
+  const T *own = P.own_y ? ybuf : RED && P.own_base == 1 ? base : src;
   const T *nbr = P.nbr_hat ? hat : ybuf;
   T a;
   unsigned int spins = 0;
   do {   // (src is never checked: see staged_row)
     a = ld_relaxed(own + 3 * row + c);
   } while (P.own_y && is_sentinel(a) && poll_again(ctl, spins));
+  if (RED && P.own_base) a = P.own_base == 1 ? a * coef : fma(coef, base[3 * row + c], a);
   for (int k0 = 0; k0 < w; k0 += SB) {
     int cc[SB];
     T y[SB][3];
@@ -1129,15 +1190,16 @@ __device__ void ring_produce(Ctl *ctl, const StagePlan &sp, unsigned char *ring,
 // One row of a streamed slice: the same arithmetic as phase_row (blocks in
 // slot order, three FMAs per block row entry, then phase_store), with the
 // slice's values, column indices and D block read from the ring stage.
-template <typename V, typename T>
+template <typename V, typename T, bool RED>
 __device__ __forceinline__ void ring_row(const Phase &P, int row, int lane, int w, const V *sv,
                                          const int *sc, const V *sd, const T *src, T *ybuf,
-                                         T *hat) {
+                                         T *hat, const T *__restrict__ base, T coef) {
   // gathers in flight per batch (within the kernel's 128 registers)
   constexpr int B = sizeof(T) == 8 ? 2 : 4;
-  const T *own = P.own_y ? ybuf : src;
+  const T *own = P.own_y ? ybuf : RED && P.own_base == 1 ? base : src;
   const T *nbr = P.nbr_hat ? hat : ybuf;
   T a0 = ldl(own + 3 * row), a1 = ldl(own + 3 * row + 1), a2 = ldl(own + 3 * row + 2);
+  if (RED && P.own_base) scale_own(P, base, row, coef, a0, a1, a2);
   for (int k0 = 0; k0 < w; k0 += B) {
     int c[B];
     T x[B][3];
@@ -1177,12 +1239,15 @@ __device__ __forceinline__ void ring_row(const Phase &P, int row, int lane, int 
 // ring (sp.ring_ns > 0) the last warp becomes the producer of the large
 // steps' slices and the other warps compute, synchronising among
 // themselves on a named barrier.
-template <typename V, typename T>
+// RED: the steps of the reduced iteration (base, coef: see k_tail_s). The
+// sentinels of its staged rows were written by the kernel before, so its
+// first steps start at once.
+template <typename V, typename T, bool RED>
 __global__ void __launch_bounds__(coop_threads<T>(), 1)
 k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
            const int *__restrict__ col1, const V *__restrict__ val1, const int *__restrict__ off2,
            const int *__restrict__ col2, const V *__restrict__ val2, const V *__restrict__ dmat,
-           const T *src, T *ybuf, T *hat) {
+           const T *src, T *ybuf, T *hat, const T *__restrict__ base, const double *coefp) {
   extern __shared__ __align__(128) unsigned char stage_smem[];
   __shared__ uint64_t stage_bar;
   __shared__ uint64_t ring_full[kRingMax], ring_empty[kRingMax];
@@ -1192,6 +1257,7 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
   __shared__ int stage_n;
   __shared__ T xch[sizeof(T) == 8 ? comp_groups<T>() : 1][3][32];   // FP64 component exchange
   if (ctl->done) return;
+  const T coef = RED ? (T)*coefp : (T)0;
   constexpr int NT = coop_threads<T>();
   const bool ring = sp.ring_ns > 0;
   const int ncw = ring ? NT / 32 - 1 : NT / 32;   // compute warps
@@ -1234,7 +1300,7 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
     // sentinels into the outputs of this CTA's staged rows; a grid barrier
     // separates them from every consumer
     const T sent = sentinel_value<T>();
-    for (int e = warp; e < stage_n; e += NT / 32) {
+    for (int e = warp; !RED && e < stage_n; e += NT / 32) {
       const StageEntry E = stage_tab[e];
       const Phase &P = ph.p[E.q];
       const int r = 32 * E.j + lane;
@@ -1275,10 +1341,19 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
     return false;
   };
   bool run = true;
+  // reduced: a copy that never arrived; this CTA then only takes part in the
+  // next grid barrier, which fails the run
+  bool copies_lost = false;
   if (first_staged == 0) {
-    // every step is small: the sentinels need a grid barrier before any step
-    run = grid_barrier(ctl, copies_late(), nct);
-    staged_ready = run;
+    // the general apply: every step is small, and the sentinels need a grid
+    // barrier before any step
+    if (RED) {
+      copies_lost = cta_sync_or(nct, copies_late());
+      staged_ready = !copies_lost;
+    } else {
+      run = grid_barrier(ctl, copies_late(), nct);
+      staged_ready = run;
+    }
   }
   unsigned int gseq = 0;   // ring slices of this CTA in the streamed steps so far
   for (int q = 0; run && q < ph.n; ++q) {
@@ -1287,8 +1362,9 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
     const int *off = P.mat ? off2 : off1;
     const int *col = P.mat ? col2 : col1;
     const V *val = P.mat ? val2 : val1;
-    bool late = false;   // a ring wait of this warp ran out
-    if (P.staged && sp.enabled) {
+    bool late = RED && copies_lost;   // or a ring wait of this warp ran out
+    if (RED && copies_lost) {
+    } else if (P.staged && sp.enabled) {
       if constexpr (sizeof(T) == 8) {
         // FP64: three warps per slice, one per row component. A small step
         // gives each SM one or two slices, and one warp's FP64 instructions
@@ -1303,8 +1379,8 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
         while (e0 < stage_n && stage_tab[e0].q < q) ++e0;
         int e1 = e0;
         while (e1 < stage_n && stage_tab[e1].q == q) ++e1;
-        for (int base = e0; base < e1; base += G) {
-          const int e = base + grp;
+        for (int eb = e0; eb < e1; eb += G) {
+          const int e = eb + grp;
           const bool act = grp < G && e < e1;
           bool valid = false;
           int row = 0;
@@ -1320,7 +1396,9 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
                 reinterpret_cast<const int *>(stage_smem + E.pos + E.w * 9 * 32 * sizeof(V));
             sd = reinterpret_cast<const V *>(stage_smem + E.pos + E.w * 9 * 32 * sizeof(V) +
                                              E.w * 32 * sizeof(int));
-            if (valid) a = staged_comp<V, T>(P, c, row, lane, E.w, sv, sc, src, ybuf, hat, ctl);
+            if (valid)
+              a = staged_comp<V, T, RED>(P, c, row, lane, E.w, sv, sc, src, ybuf, hat, ctl, base,
+                                         coef);
           }
           if (!act) continue;   // the whole group (same e) skips the round
           // the D products need all three components: the group's warps
@@ -1337,8 +1415,8 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
           }
           bool fin = true;
           if (P.to_y) {
-            if (valid) st_relaxed(ybuf + 3 * row + c, a);
             fin = row >= P.final0;
+            if (valid && !fin) st_relaxed(ybuf + 3 * row + c, a);
             if (P.final_d) {
               xch[grp][c][lane] = a;
               group_sync(grp);
@@ -1362,7 +1440,8 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
               reinterpret_cast<const int *>(stage_smem + E.pos + E.w * 9 * 32 * sizeof(V));
           const V *sd = reinterpret_cast<const V *>(stage_smem + E.pos + E.w * 9 * 32 * sizeof(V) +
                                                     E.w * 32 * sizeof(int));
-          staged_row<V, T>(P, P.row0 + r, lane, E.w, sv, sc, sd, src, ybuf, hat, ctl);
+          staged_row<V, T, RED>(P, P.row0 + r, lane, E.w, sv, sc, sd, src, ybuf, hat, ctl, base,
+                                coef);
         }
       }
     } else if (P.streamed && ring) {
@@ -1388,11 +1467,11 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
         const unsigned char *stage = ring_base + (size_t)st * sp.ring_stride;
         const int w = ring_w[st];
         if (r < P.nrows)
-          ring_row<V, T>(P, P.row0 + r, lane, w, reinterpret_cast<const V *>(stage),
+          ring_row<V, T, RED>(P, P.row0 + r, lane, w, reinterpret_cast<const V *>(stage),
                          reinterpret_cast<const int *>(stage + w * 9 * 32 * sizeof(V)),
                          reinterpret_cast<const V *>(stage + w * 9 * 32 * sizeof(V) +
                                                      w * 32 * sizeof(int)),
-                         src, ybuf, hat);
+                         src, ybuf, hat, base, coef);
         __syncwarp();
         if (lane == 0) mbar_arrive(&ring_empty[st]);
       }
@@ -1444,8 +1523,8 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
 #endif
         const int t = 32 * j + lane;
         if (t < P.nrows)
-          phase_row<V, T, !kLargeCached>(P, P.row0 + t, P.slice0 + j, lane, off, col, val, dmat,
-                                         src, ybuf, hat);
+          phase_row<V, T, !kLargeCached, RED>(P, P.row0 + t, P.slice0 + j, lane, off, col, val,
+                                              dmat, src, ybuf, hat, base, coef);
 #if GBILU_L2_PREFETCH > 0
         if (PF && lane == 0 && jp < nsl)
           prefetch_slice<V>(P.slice0 + jp, po, pe - po, col, val, dmat, pd);
@@ -1505,42 +1584,73 @@ __global__ void k_wait_probe(Ctl *ctl, int mode, const double *word) {
 // r = b - y (the RESID epilogue's arithmetic), rt = p = r, rho = ||r||^2 and
 // the stop tests of the start. Split from the SpMV so that b can still be in
 // transit while A x0 is computed. perm non-null: b is in the input numbering
-// (device row i reads input row perm[i], as k_gather).
+// (device row i reads input row perm[i], as k_gather). The first nh entries
+// are the reduced iteration's head (color 0): their base is r (see
+// k_tail_s), their p is never read, and bp keeps their b for the end of the
+// solve (bp may be b).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_init_resid(Ctl *ctl, int n, const T *__restrict__ b, const int *__restrict__ perm,
-             T *__restrict__ r, T *__restrict__ rt, T *__restrict__ p, double *partials) {
-  double d = 0.0;
-  DF f = {0.f, 0.f};
+k_init_resid(Ctl *ctl, int n, int nh, const T *b, const int *__restrict__ perm, T *bp,
+             T *__restrict__ r, T *__restrict__ rt, T *__restrict__ p, T *__restrict__ base,
+             double *partials) {
+  double d = 0.0, dh = 0.0;
+  DF f = {0.f, 0.f}, fh = {0.f, 0.f};
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
     const int row = i / 3;
-    const T v = (perm ? b[3 * perm[row] + (i - 3 * row)] : b[i]) - r[i];
-    r[i] = v; rt[i] = v; p[i] = v;
-    if (sizeof(T) == 8) d += (double)v * v; else df_add_prod(f, (float)v, (float)v);
+    const T bi = perm ? b[3 * perm[row] + (i - 3 * row)] : b[i];
+    const T v = bi - r[i];
+    rt[i] = v;
+    if (i < nh) {
+      base[i] = v;
+      if (perm) bp[i] = bi;
+      if (sizeof(T) == 8) dh += (double)v * v; else df_add_prod(fh, (float)v, (float)v);
+    } else {
+      r[i] = v; p[i] = v;
+      if (sizeof(T) == 8) d += (double)v * v; else df_add_prod(f, (float)v, (float)v);
+    }
   }
-  if (sizeof(T) == 4) d = df_value(f);
-  double vv[1] = {d}, tot[1];
-  if (grid_sum<1>(vv, partials, &ctl->counter[0], tot) && threadIdx.x == 0)
-    finish_init<T>(ctl, tot[0]);
+  if (sizeof(T) == 4) { d = df_value(f); dh = df_value(fh); }
+  double vv[2] = {d, dh}, tot[2];
+  if (grid_sum<2>(vv, partials, &ctl->counter[0], tot) && threadIdx.x == 0)
+    finish_init<T>(ctl, tot[0] + tot[1], nh > 0, tot[1]);
 }
 
 // Inner solves of iterative refinement start from d = 0: r = rt = p = rhs,
-// rho = ||rhs||^2 (step 1 without the SpMV of step 0).
+// rho = ||rhs||^2 (step 1 without the SpMV of step 0). nh, base: as in
+// k_init_resid.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_init_rhs(Ctl *ctl, int n, const T *__restrict__ rhs, T *__restrict__ r,
-           T *__restrict__ rt, T *__restrict__ p, T *__restrict__ x, double *partials) {
-  double d = 0.0;
-  DF f = {0.f, 0.f};
+k_init_rhs(Ctl *ctl, int n, int nh, const T *__restrict__ rhs, T *__restrict__ r,
+           T *__restrict__ rt, T *__restrict__ p, T *__restrict__ x, T *__restrict__ base,
+           double *partials) {
+  double d = 0.0, dh = 0.0;
+  DF f = {0.f, 0.f}, fh = {0.f, 0.f};
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
     const T v = rhs[i];
-    r[i] = v; rt[i] = v; p[i] = v; x[i] = 0;
-    if (sizeof(T) == 8) d += (double)v * v; else df_add_prod(f, (float)v, (float)v);
+    rt[i] = v; x[i] = 0;
+    if (i < nh) {
+      base[i] = v;
+      if (sizeof(T) == 8) dh += (double)v * v; else df_add_prod(fh, (float)v, (float)v);
+    } else {
+      r[i] = v; p[i] = v;
+      if (sizeof(T) == 8) d += (double)v * v; else df_add_prod(f, (float)v, (float)v);
+    }
   }
-  if (sizeof(T) == 4) d = df_value(f);
-  double v[1] = {d}, tot[1];
-  if (grid_sum<1>(v, partials, &ctl->counter[0], tot) && threadIdx.x == 0)
-    finish_init<T>(ctl, tot[0]);
+  if (sizeof(T) == 4) { d = df_value(f); dh = df_value(fh); }
+  double v[2] = {d, dh}, tot[2];
+  if (grid_sum<2>(v, partials, &ctl->counter[0], tot) && threadIdx.x == 0)
+    finish_init<T>(ctl, tot[0] + tot[1], nh > 0, tot[1]);
+}
+
+// The stop tests after the first half; ss: ||s||^2 over the rows whose s is
+// formed (all, or the reduced iteration's tail).
+__device__ __forceinline__ void finish_s(Ctl *ctl, double ss) {
+  const double ns = sqrt(ss + head_part(ctl, ctl->cs * ctl->cs));
+  push_norm(ctl, ns);
+  if (!finite(ns)) stop(ctl, ST_NONFINITE, 1);
+  else if (!ctl->ru_mode && !(ns > ctl->bound)) stop(ctl, ST_OK, 1);
+  else if (ctl->k == ctl->maxit) stop(ctl, ST_MAXIT, 1);
+  else ctl->half = 2 * ctl->k + 1;
 }
 
 // Steps 6-8 without the x update (deferred to the second half): s = r - alpha v,
@@ -1574,14 +1684,7 @@ k_update_s(Ctl *ctl, int n, const T *__restrict__ r, const T *__restrict__ v,
   }
   if (sizeof(T) == 4) d = df_value(f);
   double vv[1] = {d}, tot[1];
-  if (grid_sum<1>(vv, partials, &ctl->counter[3], tot) && threadIdx.x == 0) {
-    const double ns = sqrt(tot[0]);
-    push_norm(ctl, ns);
-    if (!finite(ns)) stop(ctl, ST_NONFINITE, 1);
-    else if (!ctl->ru_mode && !(ns > ctl->bound)) stop(ctl, ST_OK, 1);
-    else if (ctl->k == ctl->maxit) stop(ctl, ST_MAXIT, 1);
-    else ctl->half = 2 * ctl->k + 1;
-  }
+  if (grid_sum<1>(vv, partials, &ctl->counter[3], tot) && threadIdx.x == 0) finish_s(ctl, tot[0]);
 }
 
 // Steps 11-14: x += alpha p^ + omega s^ (both halves' updates in one pass),
@@ -1621,9 +1724,14 @@ k_update_r(Ctl *ctl, int n, T *__restrict__ x, const T *__restrict__ ph,
   if (sizeof(T) == 4) { d1 = df_value(f1); d2 = df_value(f2); }
   double vv[2] = {d1, d2}, tot[2];
   if (grid_sum<2>(vv, partials, &ctl->counter[4], tot) && threadIdx.x == 0) {
-    const double nr = sqrt(tot[0]);
+    // the color-0 rows of the reduced iteration: t = s there, so
+    // r = (1 - omega) s
+    const double cr = fma(-ctl->omega, ctl->cs, ctl->cs);
+    ctl->cr = cr;
+    ctl->x_moved = 1;
+    const double nr = sqrt(tot[0] + head_part(ctl, cr * cr));
     push_norm(ctl, nr);
-    ctl->dots[3] = tot[1];
+    ctl->dots[3] = tot[1] + head_part(ctl, cr * ctl->crt);
     if (!finite(nr)) { stop(ctl, ST_NONFINITE, 0); return; }
     if (ctl->ru_mode) {
       // the recursive residual of the FP32 iteration only schedules a
@@ -1634,11 +1742,25 @@ k_update_r(Ctl *ctl, int n, T *__restrict__ x, const T *__restrict__ ph,
       stop(ctl, ST_OK, 0);
       return;
     }
-    const double rho_new = tot[1];
+    double rho_new = ctl->dots[3];
+    if (ctl->reduced) {
+      // A right-hand side on color 0 alone makes (r, rt) zero after one
+      // iteration: the head's residual is eliminated exactly and rt has no
+      // tail. (The full iteration goes on from the rounding errors that it
+      // leaves there.) The iteration then starts again from r: rt = p = r.
+      ctl->restart = fabs(rho_new) < 1e-15 * nr * ctl->rt_norm;
+      if (ctl->restart) {
+        ctl->crt = cr;
+        ctl->rt_norm = nr;
+        ctl->rho = rho_new = nr * nr;
+        ctl->alpha = 0.0;   // beta = 0
+      }
+    }
     const double beta = (rho_new / ctl->rho) * (ctl->alpha / ctl->omega);
     ctl->rho_prev = ctl->rho;
     ctl->rho = rho_new;
     ctl->beta = beta;
+    ctl->cp = fma(beta, fma(-ctl->omega, ctl->cp, ctl->cp), cr);   // v = p there
     if (ctl->omega == 0.0 || !finite(beta)) { stop(ctl, ST_BREAKDOWN, 0); return; }
     if (ctl->timeout_ns && globaltimer() - ctl->t_start > ctl->timeout_ns) {
       stop(ctl, ST_TIMEOUT, 0);

@@ -351,7 +351,8 @@ class GbIlu:
     KERNELS = {"spmv64": 0, "ilu64": 1, "spmv32": 2, "ilu32": 3,
                "spmv_alpha64": 4, "spmv_omega64": 5, "update_s64": 6, "update_r64": 7,
                "update_p64": 8, "spmv_alpha32": 9, "spmv_omega32": 10, "update_s32": 11,
-               "update_r32": 12, "update_p32": 13}
+               "update_r32": 12, "update_p32": 13,
+               "apply64": 14, "apply32": 15}
 
     def ilu_trace(self, fp32=False, transpose=False):
         """[(rows, microseconds)] per color step of one single-launch ILU apply."""

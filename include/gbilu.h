@@ -149,7 +149,9 @@ typedef struct {
   double factor_ms;         /* host ILU0 + upload time of the last factor */
   double analyze_ms;
   /* algorithmic bytes (every operand read or written once, x gathers
-   * counted once) of one SpMV, one ILU apply and one full iteration:
+   * counted once) of one SpMV and one ILU apply over all rows, and of one
+   * iteration as it runs (with two or more colors: without the rows of color
+   * 0, whose part of every vector is a multiple of the initial residual's):
    * [0] FP64 storage and vectors, [1] FP32 storage and vectors */
   double alg_bytes_spmv[2];
   double alg_bytes_ilu[2];
@@ -280,10 +282,11 @@ int gbilu_get_stats(void *handle, gbilu_stats *stats);
 
 /* Times one kernel family on the handle's stream with CUDA events, reps
  * applications back to back on the factored system: which = 0 SpMV FP64,
- * 1 ILU apply FP64 (all colors), 2 SpMV FP32, 3 ILU apply FP32; the other
- * kernels of one iteration, 4-8 in FP64 and 9-13 in FP32: SpMV with the
- * alpha dot, SpMV with the omega dots, update_s, update_r, update_p (FP32
- * ids need GBILU_MIXED). Returns the average device ms per application, its
+ * 1 ILU apply FP64 (all colors), 2 SpMV FP32, 3 ILU apply FP32; the
+ * kernels of one iteration over the rows that it runs on, 4-8 in FP64 and
+ * 9-13 in FP32: SpMV with the alpha dot, SpMV with the omega dots, update_s,
+ * update_r, update_p, and 14 (FP64), 15 (FP32) its part of the ILU apply
+ * (FP32 ids need GBILU_MIXED). Returns the average device ms per application, its
  * algorithmic bytes and the kernel launches per application. The
  * counterpart of the reference's kernel timing around clEnqueueTask
  * (fpga_functions_bicgstab.cpp:1305-1325), per kernel instead of per run. */
