@@ -591,13 +591,9 @@ template <typename V, typename T> Tail<V, T> make_tail(const Handle *h, const Op
   return P;
 }
 
-// CTAs of a kernel with one thread per row, at most cap: each thread gets
-// the same number of rows (a last round that few CTAs take part in costs as
-// much as a full one).
+// CTAs of a kernel with one thread per row.
 int row_grid(const Handle *h, int rows, int ctas_per_sm) {
-  const long long cap = (long long)h->sm_count * ctas_per_sm * kThreads;
-  const long long rounds = std::max<long long>(1, (rows + cap - 1) / cap);
-  return (int)std::max<long long>(1, (rows + rounds * kThreads - 1) / (rounds * kThreads));
+  return std::max(1, std::min((rows + kThreads - 1) / kThreads, h->sm_count * ctas_per_sm));
 }
 
 // One iteration of the reduced form (gbilu_reduced.cuh): the first sweep of

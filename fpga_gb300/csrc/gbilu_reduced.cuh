@@ -124,6 +124,12 @@ k_base_tail(const Ctl *ctl, Tail<V, T> P, int S, const int2 *__restrict__ srows,
   }
 }
 
+// The vector kernels deal their warps' groups of 32 rows to the CTAs in turn,
+// so that the groups of a last, partial round spread over all SMs.
+__device__ __forceinline__ int first_row() {
+  return 32 * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) + (threadIdx.x & 31);
+}
+
 // Steps 6-8 on the tail (k_update_s) and the first sweep of the next apply:
 // s = r - alpha v, ||s|| and the stop tests; y or hat of color 1 from s.
 template <typename V, typename T>
@@ -134,7 +140,7 @@ k_tail_s(Ctl *ctl, Tail<V, T> P, const T *__restrict__ r, const T *__restrict__ 
   const T alpha = (T)ctl->alpha, cs = (T)ctl->cs;
   double d = 0.0;
   DF f = {0.f, 0.f};
-  for (int t = blockIdx.x * kThreads + threadIdx.x; t < P.rows; t += gridDim.x * kThreads) {
+  for (int t = first_row(); t < P.rows; t += gridDim.x * kThreads) {
     const int i = 3 * (P.row0 + t);
     const T *b = P.base + i;
     const T b0 = b[0], b1 = b[1], b2 = b[2];
@@ -170,7 +176,7 @@ k_tail_p(Ctl *ctl, Tail<V, T> P, const T *__restrict__ r, const T *__restrict__ 
   if (ctl->done) return;
   const T beta = (T)ctl->beta, omega = (T)ctl->omega, cp = (T)ctl->cp;
   const bool restart = ctl->restart;
-  for (int t = blockIdx.x * kThreads + threadIdx.x; t < P.rows; t += gridDim.x * kThreads) {
+  for (int t = first_row(); t < P.rows; t += gridDim.x * kThreads) {
     const int i = 3 * (P.row0 + t);
     const T *b = P.base + i;
     const T b0 = b[0], b1 = b[1], b2 = b[2];
