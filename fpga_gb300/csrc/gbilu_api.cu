@@ -6,6 +6,7 @@
 #include "gbilu_host.hpp"
 #include "gbilu_kernels.cuh"
 #include "gbilu_reduced.cuh"
+#include "gbilu_small.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -138,6 +139,11 @@ struct Handle {
   Sweep sweep[2][2][2];                    // [reduced][fp32][transpose]
   cudaError_t launch_err = cudaSuccess;    // first failed cooperative launch
   int coop_grid64 = 1, coop_grid32 = 1;    // CTAs of the cooperative apply
+  // solves in one launch (gbilu_small.cuh), [fp32]: CTAs (0: not used),
+  // dynamic shared memory; their barrier counters and x0 flag
+  int small_grid[2] = {0, 0}, small_smem[2] = {0, 0};
+  DevBuf<unsigned long long> small_bar;
+  Ctl *h_inner = nullptr;                  // pinned: an inner solve's outcome
   size_t device_bytes = 0;
 
   int fail(int code, const char *fmt, ...) {
@@ -637,6 +643,97 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
   ++launches;
 }
 
+// Block rows up to which a solve runs in one launch. FP64, FP32.
+#ifndef GBILU_SMALL_ROWS64
+#define GBILU_SMALL_ROWS64 60000
+#endif
+#ifndef GBILU_SMALL_ROWS32
+#define GBILU_SMALL_ROWS32 120000
+#endif
+
+// Plans the one-launch solve: its CTAs and the shared memory that the
+// largest share of slices wants (as much as there is when it is more).
+template <typename V, typename T> int plan_small(Handle *h, int rows) {
+  const Analysis &an = h->an;
+  const int f = sizeof(T) == 4;
+  h->small_grid[f] = 0;
+  if (!reduced_run(h, false) || an.nb > rows || h->sweep[1][f][0].phases.n == 0 ||
+      h->sweep[1][f][1].phases.n == 0)
+    return GBILU_OK;
+  const int grid = std::min(h->sm_count, an.S);
+  if ((an.S + grid - 1) / grid > kSmallOwn || grid > kSmallThreads) return GBILU_OK;
+  cudaFuncAttributes fa;
+  int optin = 0;
+  CK(cudaFuncGetAttributes(&fa, k_solve_small<V, T>));
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->opt.device));
+  const int room = optin - (int)fa.sharedSizeBytes;
+  std::vector<long long> bytes(grid, 0);
+  for (int s = 0; s < an.S; ++s)
+    bytes[s % grid] += s < an.slice_color_ptr[1] ? slice_bytes<V>(an.U, s, true)
+                                                 : slice_bytes<V>(an.A, s, s < an.slice_color_ptr[2]);
+  const int smem = (int)std::min<long long>(room, *std::max_element(bytes.begin(), bytes.end()));
+  CK(cudaFuncSetAttribute(k_solve_small<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_small<V, T>, kSmallThreads,
+                                                   (size_t)smem));
+  if (per_sm < 1) return GBILU_OK;
+  h->small_grid[f] = grid;
+  h->small_smem[f] = smem;
+  return GBILU_OK;
+}
+
+// The arguments that do not depend on the call.
+template <typename V, typename T> SmallArgs<V, T> small_args(Handle *h, const Ops<V, T> &o) {
+  const Analysis &an = h->an;
+  const int f = sizeof(T) == 4;
+  Vecs<T> &w = *o.vec;
+  SmallArgs<V, T> A = {};
+  A.ctl = h->ctl.p;
+  A.bar = h->small_bar.p + f;
+  A.x_nonzero = reinterpret_cast<int *>(h->small_bar.p + 2);
+  A.partials = h->partials.p;
+  A.srows = h->srows.p;
+  A.S = an.S;
+  A.S0 = an.slice_color_ptr[1];
+  A.S1 = an.slice_color_ptr[2];
+  A.n0 = an.color_ptr[1];
+  A.rows1 = an.color_ptr[2] - A.n0;
+  A.split1 = an.split[1];
+  A.transpose = o.transpose;
+  A.offA = o.offA; A.colA = o.colA; A.valA = o.valA;
+  A.off1 = o.off1; A.col1 = o.col1; A.val1 = o.val1;
+  A.off1r = o.off1r; A.col1r = o.col1r; A.val1r = o.val1r;
+  A.off2 = o.off2; A.col2 = o.col2; A.val2 = o.val2;
+  A.dmat = o.dmat;
+  A.x = w.x.p; A.r = w.r.p; A.rt = w.rt.p; A.p = w.p.p; A.ph = w.ph.p; A.v = w.v.p;
+  A.s = w.s.p; A.sh = w.sh.p; A.t = w.t.p; A.y = w.y.p; A.base = w.base.p;
+  A.smem_bytes = h->small_smem[f];
+  return A;
+}
+
+template <typename V, typename T>
+cudaError_t launch_small(Handle *h, const SmallArgs<V, T> &A) {
+  const int f = sizeof(T) == 4;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.gridDim = dim3(h->small_grid[f]);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = (size_t)h->small_smem[f];
+  cfg.stream = h->st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_solve_small<V, T>, A, h->sweep[1][f][A.transpose].phases);
+}
+
+// After a failed wait the barrier counters no longer hold a multiple of
+// their grid.
+int reset_small(Handle *h, const Ctl &c) {
+  if (c.bar_fail) CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
+  return GBILU_OK;
+}
+
 template <typename V, typename T>
 int build_graph(Handle *h, const Ops<V, T> &o, cudaGraphExec_t &exec, int &per_iter,
                 const Ops<double, double> *ru64 = nullptr) {
@@ -837,6 +934,8 @@ void release_device(Handle *h) {
   h->dinvT32.release(); h->v64.release(); h->v32.release(); h->b64.release();
   h->io64.release(); h->io64b.release(); h->partials.release(); h->dA.release();
   h->x0nz.release();
+  h->small_bar.release();
+  h->small_grid[0] = h->small_grid[1] = 0;
   h->ctl.release();
   h->device_bytes = 0;
 }
@@ -854,6 +953,7 @@ int setup_device(Handle *h) {
     CK(cudaEventCreate(&h->e0));
     CK(cudaEventCreate(&h->e1));
     CK(cudaMallocHost(&h->h_ctl, sizeof(Ctl)));
+    CK(cudaMallocHost(&h->h_inner, sizeof(Ctl)));
     CK(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->opt.device));
   }
   release_device(h);
@@ -915,6 +1015,8 @@ int setup_device(Handle *h) {
   CK(h->x0nz.alloc(1));
   CK(cudaMemset(h->x0nz.p, 0xff, sizeof(int)));   // "nonzero" until a gather clears it
   CK(h->ctl.alloc(2));
+  CK(h->small_bar.alloc(3));
+  CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
   if (h->opt.factor_on_device) {
     CK(h->pdiag.alloc(an.nb));
     CK(cudaMemcpy(h->pdiag.p, an.pdiag.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice));
@@ -947,6 +1049,12 @@ int setup_device(Handle *h) {
         if (rc) return rc;
       }
     }
+  }
+  if (h->with_32) {
+    if (h->opt.mixed_scheme == 0)
+      if (int rc = plan_small<float, float>(h, GBILU_SMALL_ROWS32)) return rc;
+  } else if (int rc = plan_small<double, double>(h, GBILU_SMALL_ROWS64)) {
+    return rc;
   }
   h->device_bytes += nd * 16 + (h->with_32 ? nd * 8 : 0) + n * 8 * 14 + (h->with_32 ? n * 4 * 11 : 0) +
                      (size_t)an.nnzb * 16 + (size_t)an.nb * 16;
@@ -1114,14 +1222,18 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
   Vecs<float> &f = h->v32;
   Ctl *outer = h->ctl.p + 1;
   const int g = grid_for(h, n);
-  auto residual = [&](double &nrm) -> int {
-    // r = b - A x in FP64 with the FP64 copy of A, ||r|| read back
+  auto enqueue_residual = [&]() -> int {
+    // r = b - A x in FP64 with the FP64 copy of A, ||r|| into h_ctl
     k_ctl_init<<<1, 32, 0, h->st>>>(outer, 0.0, 1, 0, 0ull);
     const int S = h->an.S;
     k_spmv<double, double, SPMV_RESID><<<std::min((S + kWarps - 1) / kWarps, 2 * h->sm_count), kThreads, 0, h->st>>>(
         outer, 0, S, h->srows.p, o64.offA, o64.colA, o64.valA, w.x.p, w.r.p, h->b64.p, h->partials.p);
     launches += 2;
     CK(cudaMemcpyAsync(h->h_ctl, outer, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
+    return GBILU_OK;
+  };
+  auto residual = [&](double &nrm) -> int {
+    if (int rc = enqueue_residual()) return rc;
     CK(cudaStreamSynchronize(h->st));
     nrm = h->h_ctl->norm0;
     return GBILU_OK;
@@ -1149,6 +1261,37 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
   const long long budget = 2LL * maxit + 1;
   while (nrm > bound && outer_steps < h->opt.max_outer && inner_half < budget) {
     const int left = (int)std::min<long long>((budget - inner_half - 1) / 2, h->opt.inner_maxit);
+    Ctl ic;
+    if (h->small_grid[1]) {
+      // the inner solve, its right-hand side and x += ||r|| d in one launch,
+      // the next residual behind it and one look at both (a run that broke
+      // down leaves x, and with it the residual, as they were)
+      SmallArgs<float, float> A = small_args(h, make_ops<float, float>(h, transpose));
+      A.host_ctl = h->h_inner;
+      A.r64 = w.r.p;
+      A.x64 = w.x.p;
+      A.scale = 1.0 / nrm;
+      A.unscale = nrm;
+      A.tol = h->opt.inner_tol;
+      A.maxit = left;
+      A.timeout_ns = tmo;
+      CK(launch_small(h, A));
+      ++launches;
+      rc = enqueue_residual();
+      if (rc) return rc;
+      CK(cudaStreamSynchronize(h->st));
+      CK(last_error(h));
+      ic = *h->h_inner;
+      rc = reset_small(h, ic);
+      if (rc) return rc;
+      inner_half += (ic.half >= 0 ? ic.half + 1 : 0);
+      ++outer_steps;
+      if (ic.status == ST_BREAKDOWN || ic.status == ST_NONFINITE) { out.status = ic.status; break; }
+      nrm = h->h_ctl->norm0;
+      if (!std::isfinite(nrm)) { out.status = ST_NONFINITE; break; }
+      if (ic.status == ST_TIMEOUT) { out.status = ST_TIMEOUT; break; }
+      continue;
+    }
     // right-hand side of the correction equation A d = r / ||r|| in FP32
     // (staged in f.t, which the inner run overwrites only after reading it)
     k_scale_convert<<<g, kThreads, 0, h->st>>>(n, 1.0 / nrm, w.r.p, f.t.p);
@@ -1162,7 +1305,7 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
     if (rc) return rc;
     CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
-    const Ctl ic = *h->h_ctl;
+    ic = *h->h_ctl;
     if (h->opt.use_graph) launches += (long long)ic.body_runs * h->per_iter[transpose ? 1 : 0];
     inner_half += (ic.half >= 0 ? ic.half + 1 : 0);
     ++outer_steps;
@@ -1338,6 +1481,7 @@ int gbilu_destroy(void *handle) {
     cudaEventDestroy(h->e0);
     cudaEventDestroy(h->e1);
     cudaFreeHost(h->h_ctl);
+    cudaFreeHost(h->h_inner);
   }
   delete h;
   return GBILU_OK;
@@ -1522,97 +1666,137 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
   const int nb = h->an.nb, n = 3 * nb;
   const int g = grid_for(h, n);
   long long launches = 0;
-  CK(cudaEventRecord(h->e0, h->st));
-  const double *db = b;
-  const double *dx = x;
-  double *mapped_x = nullptr;
-  if (!device_ptrs) {
-    // Page-locked host buffers are read and written by the gather/scatter
-    // kernels in place (mapped, over the CPU-GPU link); other host memory
-    // goes through staging copies.
-    cudaPointerAttributes ab, ax;
-    const bool zb = cudaPointerGetAttributes(&ab, b) == cudaSuccess &&
-                    ab.type == cudaMemoryTypeHost && ab.devicePointer;
-    const bool zx = cudaPointerGetAttributes(&ax, x) == cudaSuccess &&
-                    ax.type == cudaMemoryTypeHost && ax.devicePointer;
-    cudaGetLastError();   // a query on unregistered memory is not an error here
-    if (zb && zx) {
-      db = static_cast<const double *>(ab.devicePointer);
-      dx = mapped_x = static_cast<double *>(ax.devicePointer);
-    } else {
-      db = h->io64.p;   // staging copies below
-      dx = h->io64b.p;
-    }
-  }
-  // The FP64 solve needs b only after A x0 (k_init_resid): from host
-  // buffers, b moves on the auxiliary stream while the SpMV runs. The
-  // CPU-GPU link is one shared budget (about 200 GB/s for reads and writes
-  // together, measured), so x0 goes first and alone; b follows on the copy
-  // engine, which takes no SMs from the SpMV, and is permuted on the device.
-  const bool fp64 = h->opt.precision != GBILU_MIXED;
-  const bool overlap_b = fp64 && !device_ptrs;
-  if (!device_ptrs && !mapped_x)
-    CK(cudaMemcpyAsync(h->io64b.p, x, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemsetAsync(h->x0nz.p, 0, sizeof(int), h->st));
-  if (mapped_x)   // host side read in order, device side written permuted
-    k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->iperm.p, dx, h->v64.x.p, h->x0nz.p);
-  else
-    k_gather<double, double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, dx, h->v64.x.p, 1.0,
-                                                        h->x0nz.p);
-  cudaStream_t sb = h->st;
-  if (overlap_b) {
-    CK(cudaEventRecord(h->e_x, h->st));
-    CK(cudaStreamWaitEvent(h->aux, h->e_x, 0));
-    sb = h->aux;
-  }
-  if (!device_ptrs && (!mapped_x || overlap_b)) {
-    CK(cudaMemcpyAsync(h->io64.p, b, n * sizeof(double), cudaMemcpyHostToDevice, sb));
-    db = h->io64.p;
-  }
-  if (overlap_b)   // k_init_resid permutes b as it reads it
-    CK(cudaEventRecord(h->e_b, h->aux));
-  else if (mapped_x)
-    k_scatter<double><<<g, kThreads, 0, sb>>>(nb, h->iperm.p, db, h->b64.p);
-  else
-    k_gather<double, double><<<g, kThreads, 0, sb>>>(nb, h->perm.p, db, h->b64.p, 1.0);
-  launches += overlap_b ? 1 : 2;
   Ctl c;
   gbilu_result tmp;
   memset(&tmp, 0, sizeof tmp);
   gbilu_result *r = res ? res : &tmp;
   memset(r, 0, sizeof *r);
-  if (!fp64)
-    rc = solve_mixed(h, transpose, tol, maxit, r, c, launches);
-  else
-    rc = solve64(h, transpose, tol, maxit, c, launches, false, overlap_b ? h->e_b : nullptr,
-                 overlap_b ? db : nullptr);
-  if (rc) return rc;
-  if (gx && gdA) {
-    // lambda from the device numbering into the input numbering (x comes
-    // in it), then dL/dA in the input block order
-    const double *xin = gx;
-    if (!device_ptrs) {   // b's staging buffer is free once the solve read it
-      CK(cudaMemcpyAsync(h->io64.p, gx, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
-      xin = h->io64.p;
+  const bool fp64 = h->opt.precision != GBILU_MIXED;
+  const bool small = fp64 && h->small_grid[0] > 0;
+  CK(cudaEventRecord(h->e0, h->st));
+  // One launch reads b and x0 and writes x in the caller's numbering; host
+  // arrays go through staging copies.
+  if (small) {
+    const double *db = b;
+    double *dx = x;
+    if (!device_ptrs) {
+      CK(cudaMemcpyAsync(h->io64b.p, x, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
+      CK(cudaMemcpyAsync(h->io64.p, b, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
+      db = h->io64.p;
+      dx = h->io64b.p;
     }
-    k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, h->v64.x.p, h->v64.r.p);
-    k_grad_a<<<grid_for(h, (long long)h->an.nnzb * 9), kThreads, 0, h->st>>>(
-        h->an.nnzb, h->ibrow.p, h->icol.p, h->v64.r.p, xin, device_ptrs ? gdA : h->dA.p);
-    launches += 2;
+    SmallArgs<double, double> A = small_args(h, make_ops<double, double>(h, transpose));
+    A.host_ctl = h->h_ctl;
+    A.b = h->b64.p;
+    A.perm = h->perm.p;
+    A.b_in = db;
+    A.x_io = dx;
+    A.tol = tol;
+    A.absolute = h->opt.absolute_tol;
+    A.maxit = maxit;
+    A.timeout_ns = (unsigned long long)(h->opt.timeout_ms * 1e6);
+    CK(launch_small(h, A));
+    ++launches;
+    if (gx && gdA) {   // lambda is in the input numbering already
+      const double *xin = gx;
+      if (!device_ptrs) {   // b's staging buffer is free once the solve read it
+        CK(cudaMemcpyAsync(h->io64.p, gx, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
+        xin = h->io64.p;
+      }
+      k_grad_a<<<grid_for(h, (long long)h->an.nnzb * 9), kThreads, 0, h->st>>>(
+          h->an.nnzb, h->ibrow.p, h->icol.p, dx, xin, device_ptrs ? gdA : h->dA.p);
+      ++launches;
+    }
+    CK(cudaEventRecord(h->e1, h->st));
+    if (!device_ptrs)
+      CK(cudaMemcpyAsync(x, dx, n * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   }
-  // x back to the caller's numbering. When the initial residual already met
-  // the bound, v64.x still holds x0 (gathered), so this returns x0 unchanged
-  // bit for bit; the FP64 path therefore needs no status before it and the
-  // whole solve ends in one host synchronization.
-  if (mapped_x)   // device side read permuted, host side written in order
-    k_gather<double, double><<<g, kThreads, 0, h->st>>>(nb, h->iperm.p, h->v64.x.p, mapped_x, 1.0);
-  else
-    k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, h->v64.x.p,
-                                                 device_ptrs ? x : h->io64b.p);
-  launches += 1;
-  CK(cudaEventRecord(h->e1, h->st));
-  if (!device_ptrs && !mapped_x)
-    CK(cudaMemcpyAsync(x, h->io64b.p, n * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  if (!small) {
+    const double *db = b;
+    const double *dx = x;
+    double *mapped_x = nullptr;
+    if (!device_ptrs) {
+      // Page-locked host buffers are read and written by the gather/scatter
+      // kernels in place (mapped, over the CPU-GPU link); other host memory
+      // goes through staging copies.
+      cudaPointerAttributes ab, ax;
+      const bool zb = cudaPointerGetAttributes(&ab, b) == cudaSuccess &&
+                      ab.type == cudaMemoryTypeHost && ab.devicePointer;
+      const bool zx = cudaPointerGetAttributes(&ax, x) == cudaSuccess &&
+                      ax.type == cudaMemoryTypeHost && ax.devicePointer;
+      cudaGetLastError();   // a query on unregistered memory is not an error here
+      if (zb && zx) {
+        db = static_cast<const double *>(ab.devicePointer);
+        dx = mapped_x = static_cast<double *>(ax.devicePointer);
+      } else {
+        db = h->io64.p;   // staging copies below
+        dx = h->io64b.p;
+      }
+    }
+    // The FP64 solve needs b only after A x0 (k_init_resid): from host
+    // buffers, b moves on the auxiliary stream while the SpMV runs. The
+    // CPU-GPU link is one shared budget (about 200 GB/s for reads and writes
+    // together, measured), so x0 goes first and alone; b follows on the copy
+    // engine, which takes no SMs from the SpMV, and is permuted on the device.
+    const bool overlap_b = fp64 && !device_ptrs;
+    if (!device_ptrs && !mapped_x)
+      CK(cudaMemcpyAsync(h->io64b.p, x, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
+    CK(cudaMemsetAsync(h->x0nz.p, 0, sizeof(int), h->st));
+    if (mapped_x)   // host side read in order, device side written permuted
+      k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->iperm.p, dx, h->v64.x.p, h->x0nz.p);
+    else
+      k_gather<double, double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, dx, h->v64.x.p, 1.0,
+                                                          h->x0nz.p);
+    cudaStream_t sb = h->st;
+    if (overlap_b) {
+      CK(cudaEventRecord(h->e_x, h->st));
+      CK(cudaStreamWaitEvent(h->aux, h->e_x, 0));
+      sb = h->aux;
+    }
+    if (!device_ptrs && (!mapped_x || overlap_b)) {
+      CK(cudaMemcpyAsync(h->io64.p, b, n * sizeof(double), cudaMemcpyHostToDevice, sb));
+      db = h->io64.p;
+    }
+    if (overlap_b)   // k_init_resid permutes b as it reads it
+      CK(cudaEventRecord(h->e_b, h->aux));
+    else if (mapped_x)
+      k_scatter<double><<<g, kThreads, 0, sb>>>(nb, h->iperm.p, db, h->b64.p);
+    else
+      k_gather<double, double><<<g, kThreads, 0, sb>>>(nb, h->perm.p, db, h->b64.p, 1.0);
+    launches += overlap_b ? 1 : 2;
+    if (!fp64)
+      rc = solve_mixed(h, transpose, tol, maxit, r, c, launches);
+    else
+      rc = solve64(h, transpose, tol, maxit, c, launches, false, overlap_b ? h->e_b : nullptr,
+                   overlap_b ? db : nullptr);
+    if (rc) return rc;
+    if (gx && gdA) {
+      // lambda from the device numbering into the input numbering (x comes
+      // in it), then dL/dA in the input block order
+      const double *xin = gx;
+      if (!device_ptrs) {   // b's staging buffer is free once the solve read it
+        CK(cudaMemcpyAsync(h->io64.p, gx, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
+        xin = h->io64.p;
+      }
+      k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, h->v64.x.p, h->v64.r.p);
+      k_grad_a<<<grid_for(h, (long long)h->an.nnzb * 9), kThreads, 0, h->st>>>(
+          h->an.nnzb, h->ibrow.p, h->icol.p, h->v64.r.p, xin, device_ptrs ? gdA : h->dA.p);
+      launches += 2;
+    }
+    // x back to the caller's numbering. When the initial residual already met
+    // the bound, v64.x still holds x0 (gathered), so this returns x0 unchanged
+    // bit for bit; the FP64 path therefore needs no status before it and the
+    // whole solve ends in one host synchronization.
+    if (mapped_x)   // device side read permuted, host side written in order
+      k_gather<double, double><<<g, kThreads, 0, h->st>>>(nb, h->iperm.p, h->v64.x.p, mapped_x, 1.0);
+    else
+      k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, h->v64.x.p,
+                                                   device_ptrs ? x : h->io64b.p);
+    launches += 1;
+    CK(cudaEventRecord(h->e1, h->st));
+    if (!device_ptrs && !mapped_x)
+      CK(cudaMemcpyAsync(x, h->io64b.p, n * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  }
   if (gx && gdA && !device_ptrs)
     CK(cudaMemcpyAsync(gdA, h->dA.p, (size_t)h->an.nnzb * 9 * sizeof(double),
                        cudaMemcpyDeviceToHost, h->st));
@@ -1621,6 +1805,10 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
   if (fp64) {
     c = *h->h_ctl;
     if (h->opt.use_graph) launches += (long long)c.body_runs * h->per_iter[transpose ? 1 : 0];
+    if (small) {
+      rc = reset_small(h, c);
+      if (rc) return rc;
+    }
   }
   const int outer = r->outer_iters, inner = r->inner_half_iters;
   const double tr = r->true_relres;

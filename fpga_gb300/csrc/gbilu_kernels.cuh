@@ -253,45 +253,48 @@ __device__ __forceinline__ void stop(Ctl *c, int status, int stop_half) {
 // control
 // --------------------------------------------------------------------------
 
+__device__ __forceinline__ void init_ctl(Ctl *c, double tol, int absolute, int maxit,
+                                         unsigned long long timeout_ns) {
+  c->rho = c->alpha = c->omega = c->beta = 0.0;
+  c->bound = c->norm0 = c->norm = 0.0;
+  c->tol = tol;
+  for (int i = 0; i < 4; ++i) { c->norms[i] = 0.0; c->dots[i] = 0.0; }
+  c->absolute = absolute;
+  c->maxit = maxit;
+  c->last_norm_idx = 0;
+  c->half = -1;
+  c->k = 0;
+  c->done = 0;
+  c->status = ST_MAXIT;
+  c->stop_half = 0;
+  c->t_start = globaltimer();
+  c->timeout_ns = timeout_ns;
+  for (int i = 0; i < 8; ++i) c->counter[i] = 0u;
+  c->bar_count = 0u;
+  c->bar_gen = 0u;
+  c->bar_fail = 0;
+  c->body_runs = 0;
+  c->ru_mode = 0;
+  c->ru = 0;
+  c->sigma = 1.0;
+  c->ru_delta = 0.1;
+  c->rmax = 0.0;
+  c->rho_prev = 0.0;
+  c->true_norm = 0.0;
+  c->replacements = 0;
+  c->cr = c->cp = 1.0;
+  c->cs = 0.0;
+  c->head_rr = 0.0;
+  c->crt = 1.0;
+  c->rt_norm = 0.0;
+  c->reduced = c->restart = 0;
+  c->x_moved = 0;
+  for (int q = 0; q < kMaxPhases; ++q) c->step_next[q] = 0u;
+}
+
 __global__ void k_ctl_init(Ctl *c, double tol, int absolute, int maxit,
                            unsigned long long timeout_ns) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    c->rho = c->alpha = c->omega = c->beta = 0.0;
-    c->bound = c->norm0 = c->norm = 0.0;
-    c->tol = tol;
-    for (int i = 0; i < 4; ++i) { c->norms[i] = 0.0; c->dots[i] = 0.0; }
-    c->absolute = absolute;
-    c->maxit = maxit;
-    c->last_norm_idx = 0;
-    c->half = -1;
-    c->k = 0;
-    c->done = 0;
-    c->status = ST_MAXIT;
-    c->stop_half = 0;
-    c->t_start = globaltimer();
-    c->timeout_ns = timeout_ns;
-    for (int i = 0; i < 8; ++i) c->counter[i] = 0u;
-    c->bar_count = 0u;
-    c->bar_gen = 0u;
-    c->bar_fail = 0;
-    c->body_runs = 0;
-    c->ru_mode = 0;
-    c->ru = 0;
-    c->sigma = 1.0;
-    c->ru_delta = 0.1;
-    c->rmax = 0.0;
-    c->rho_prev = 0.0;
-    c->true_norm = 0.0;
-    c->replacements = 0;
-    c->cr = c->cp = 1.0;
-    c->cs = 0.0;
-    c->head_rr = 0.0;
-    c->crt = 1.0;
-    c->rt_norm = 0.0;
-    c->reduced = c->restart = 0;
-    c->x_moved = 0;
-    for (int q = 0; q < kMaxPhases; ++q) c->step_next[q] = 0u;
-  }
+  if (threadIdx.x == 0 && blockIdx.x == 0) init_ctl(c, tol, absolute, maxit, timeout_ns);
 }
 
 // Solver scalars for timing the iteration's kernels one at a time: unit
@@ -336,6 +339,88 @@ __device__ __forceinline__ void finish_init(Ctl *c, double rr, int reduced = 0,
   c->bound = bound;
   c->half = 0;
   c->k = 0;
+}
+
+// Scalars and stop tests after the reductions; the sums are over the rows
+// whose vectors are formed (all, or the reduced iteration's tail).
+// (v, rt) -> alpha
+__device__ __forceinline__ void finish_alpha(Ctl *ctl, double sum) {
+  const double vrt = sum + head_part(ctl, ctl->cp * ctl->crt);
+  const double a = ctl->rho / vrt;
+  ctl->dots[0] = vrt;
+  ctl->alpha = a;
+  ctl->cs = fma(-a, ctl->cp, ctl->cr);
+  if (vrt == 0.0 || !finite(a)) stop(ctl, ST_BREAKDOWN, 0);
+}
+
+// (t, s), (t, t) -> omega
+__device__ __forceinline__ void finish_omega(Ctl *ctl, double sum_ts, double sum_tt) {
+  const double hh = head_part(ctl, ctl->cs * ctl->cs);
+  const double ts = sum_ts + hh, tt = sum_tt + hh;
+  const double om = ts / tt;
+  ctl->dots[1] = ts;
+  ctl->dots[2] = tt;
+  ctl->omega = om;
+  // half 1 already advanced x by alpha p^: keep it on a stop here
+  if (tt == 0.0 || !finite(om)) stop(ctl, ST_BREAKDOWN, 1);
+}
+
+// ||s||^2 and the stop tests after the first half
+__device__ __forceinline__ void finish_s(Ctl *ctl, double ss) {
+  const double ns = sqrt(ss + head_part(ctl, ctl->cs * ctl->cs));
+  push_norm(ctl, ns);
+  if (!finite(ns)) stop(ctl, ST_NONFINITE, 1);
+  else if (!ctl->ru_mode && !(ns > ctl->bound)) stop(ctl, ST_OK, 1);
+  else if (ctl->k == ctl->maxit) stop(ctl, ST_MAXIT, 1);
+  else ctl->half = 2 * ctl->k + 1;
+}
+
+// ||r||^2, (r, rt) -> beta and the stop tests after the second half
+__device__ __forceinline__ void finish_r(Ctl *ctl, double rr, double rrt, bool timed_out) {
+  // the color-0 rows of the reduced iteration: t = s there, so
+  // r = (1 - omega) s
+  const double cr = fma(-ctl->omega, ctl->cs, ctl->cs);
+  ctl->cr = cr;
+  ctl->x_moved = 1;
+  const double nr = sqrt(rr + head_part(ctl, cr * cr));
+  push_norm(ctl, nr);
+  ctl->dots[3] = rrt + head_part(ctl, cr * ctl->crt);
+  if (!finite(nr)) { stop(ctl, ST_NONFINITE, 0); return; }
+  if (ctl->ru_mode) {
+    // the recursive residual of the FP32 iteration only schedules a
+    // replacement; the stop is decided on the true FP64 residual
+    if (!(nr > ctl->bound) || nr < ctl->ru_delta * ctl->rmax) ctl->ru = 1;
+    ctl->rmax = fmax(ctl->rmax, nr);
+  } else if (!(nr > ctl->bound)) {
+    stop(ctl, ST_OK, 0);
+    return;
+  }
+  double rho_new = ctl->dots[3];
+  if (ctl->reduced) {
+    // A right-hand side on color 0 alone makes (r, rt) zero after one
+    // iteration: the head's residual is eliminated exactly and rt has no
+    // tail. (The full iteration goes on from the rounding errors that it
+    // leaves there.) The iteration then starts again from r: rt = p = r.
+    ctl->restart = fabs(rho_new) < 1e-15 * nr * ctl->rt_norm;
+    if (ctl->restart) {
+      ctl->crt = cr;
+      ctl->rt_norm = nr;
+      ctl->rho = rho_new = nr * nr;
+      ctl->alpha = 0.0;   // beta = 0
+    }
+  }
+  const double beta = (rho_new / ctl->rho) * (ctl->alpha / ctl->omega);
+  ctl->rho_prev = ctl->rho;
+  ctl->rho = rho_new;
+  ctl->beta = beta;
+  ctl->cp = fma(beta, fma(-ctl->omega, ctl->cp, ctl->cp), cr);   // v = p there
+  if (ctl->omega == 0.0 || !finite(beta)) { stop(ctl, ST_BREAKDOWN, 0); return; }
+  if (timed_out) {
+    stop(ctl, ST_TIMEOUT, 0);
+    return;
+  }
+  ctl->k += 1;
+  ctl->half = 2 * ctl->k;
 }
 
 // --------------------------------------------------------------------------
@@ -538,26 +623,12 @@ k_spmv(Ctl *ctl, int S0, int S, const int2 *__restrict__ srows, const int *__res
       ctl->true_norm = sqrt(tot[0]);
   } else if (MODE == SPMV_ALPHA) {
     double v[1] = {d1}, tot[1];
-    if (grid_sum<1>(v, partials, &ctl->counter[1], tot) && threadIdx.x == 0) {
-      const double vrt = tot[0] + head_part(ctl, ctl->cp * ctl->crt);
-      const double a = ctl->rho / vrt;
-      ctl->dots[0] = vrt;
-      ctl->alpha = a;
-      ctl->cs = fma(-a, ctl->cp, ctl->cr);
-      if (vrt == 0.0 || !finite(a)) stop(ctl, ST_BREAKDOWN, 0);
-    }
+    if (grid_sum<1>(v, partials, &ctl->counter[1], tot) && threadIdx.x == 0)
+      finish_alpha(ctl, tot[0]);
   } else {
     double v[2] = {d1, d2}, tot[2];
-    if (grid_sum<2>(v, partials, &ctl->counter[2], tot) && threadIdx.x == 0) {
-      const double hh = head_part(ctl, ctl->cs * ctl->cs);
-      const double ts = tot[0] + hh, tt = tot[1] + hh;
-      const double om = ts / tt;
-      ctl->dots[1] = ts;
-      ctl->dots[2] = tt;
-      ctl->omega = om;
-      // half 1 already advanced x by alpha p^: keep it on a stop here
-      if (tt == 0.0 || !finite(om)) stop(ctl, ST_BREAKDOWN, 1);
-    }
+    if (grid_sum<2>(v, partials, &ctl->counter[2], tot) && threadIdx.x == 0)
+      finish_omega(ctl, tot[0], tot[1]);
   }
 }
 
@@ -1642,17 +1713,6 @@ k_init_rhs(Ctl *ctl, int n, int nh, const T *__restrict__ rhs, T *__restrict__ r
     finish_init<T>(ctl, tot[0] + tot[1], nh > 0, tot[1]);
 }
 
-// The stop tests after the first half; ss: ||s||^2 over the rows whose s is
-// formed (all, or the reduced iteration's tail).
-__device__ __forceinline__ void finish_s(Ctl *ctl, double ss) {
-  const double ns = sqrt(ss + head_part(ctl, ctl->cs * ctl->cs));
-  push_norm(ctl, ns);
-  if (!finite(ns)) stop(ctl, ST_NONFINITE, 1);
-  else if (!ctl->ru_mode && !(ns > ctl->bound)) stop(ctl, ST_OK, 1);
-  else if (ctl->k == ctl->maxit) stop(ctl, ST_MAXIT, 1);
-  else ctl->half = 2 * ctl->k + 1;
-}
-
 // Steps 6-8 without the x update (deferred to the second half): s = r - alpha v,
 // ||s|| and the stop tests (solver.vhd:867-936, is_final_iter solver.vhd:557).
 template <typename T>
@@ -1723,52 +1783,9 @@ k_update_r(Ctl *ctl, int n, T *__restrict__ x, const T *__restrict__ ph,
   }
   if (sizeof(T) == 4) { d1 = df_value(f1); d2 = df_value(f2); }
   double vv[2] = {d1, d2}, tot[2];
-  if (grid_sum<2>(vv, partials, &ctl->counter[4], tot) && threadIdx.x == 0) {
-    // the color-0 rows of the reduced iteration: t = s there, so
-    // r = (1 - omega) s
-    const double cr = fma(-ctl->omega, ctl->cs, ctl->cs);
-    ctl->cr = cr;
-    ctl->x_moved = 1;
-    const double nr = sqrt(tot[0] + head_part(ctl, cr * cr));
-    push_norm(ctl, nr);
-    ctl->dots[3] = tot[1] + head_part(ctl, cr * ctl->crt);
-    if (!finite(nr)) { stop(ctl, ST_NONFINITE, 0); return; }
-    if (ctl->ru_mode) {
-      // the recursive residual of the FP32 iteration only schedules a
-      // replacement; the stop is decided on the true FP64 residual
-      if (!(nr > ctl->bound) || nr < ctl->ru_delta * ctl->rmax) ctl->ru = 1;
-      ctl->rmax = fmax(ctl->rmax, nr);
-    } else if (!(nr > ctl->bound)) {
-      stop(ctl, ST_OK, 0);
-      return;
-    }
-    double rho_new = ctl->dots[3];
-    if (ctl->reduced) {
-      // A right-hand side on color 0 alone makes (r, rt) zero after one
-      // iteration: the head's residual is eliminated exactly and rt has no
-      // tail. (The full iteration goes on from the rounding errors that it
-      // leaves there.) The iteration then starts again from r: rt = p = r.
-      ctl->restart = fabs(rho_new) < 1e-15 * nr * ctl->rt_norm;
-      if (ctl->restart) {
-        ctl->crt = cr;
-        ctl->rt_norm = nr;
-        ctl->rho = rho_new = nr * nr;
-        ctl->alpha = 0.0;   // beta = 0
-      }
-    }
-    const double beta = (rho_new / ctl->rho) * (ctl->alpha / ctl->omega);
-    ctl->rho_prev = ctl->rho;
-    ctl->rho = rho_new;
-    ctl->beta = beta;
-    ctl->cp = fma(beta, fma(-ctl->omega, ctl->cp, ctl->cp), cr);   // v = p there
-    if (ctl->omega == 0.0 || !finite(beta)) { stop(ctl, ST_BREAKDOWN, 0); return; }
-    if (ctl->timeout_ns && globaltimer() - ctl->t_start > ctl->timeout_ns) {
-      stop(ctl, ST_TIMEOUT, 0);
-      return;
-    }
-    ctl->k += 1;
-    ctl->half = 2 * ctl->k;
-  }
+  if (grid_sum<2>(vv, partials, &ctl->counter[4], tot) && threadIdx.x == 0)
+    finish_r(ctl, tot[0], tot[1],
+             ctl->timeout_ns && globaltimer() - ctl->t_start > ctl->timeout_ns);
 }
 
 // --------------------------------------------------------------------------
