@@ -643,12 +643,17 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
   ++launches;
 }
 
-// Block rows up to which a solve runs in one launch. FP64, FP32.
+// Block rows up to which a solve runs in one launch, FP64 and FP32 (inner
+// solves): above, the CTA's 12 warps are too few to stream what its shared
+// memory does not hold. Measured per iteration, separate kernels / one launch,
+// us: FP64 4,000 rows 59 / 28, 35,000 69 / 36, 81,000 83 / 67, 108,000 88 / 72,
+// 180,000 112 / 130; with fault connections (three colors) 103,000 111 / 88,
+// 171,000 140 / 142; FP32 108,000 99 / 75, 180,000 116 / 118.
 #ifndef GBILU_SMALL_ROWS64
-#define GBILU_SMALL_ROWS64 60000
+#define GBILU_SMALL_ROWS64 140000
 #endif
 #ifndef GBILU_SMALL_ROWS32
-#define GBILU_SMALL_ROWS32 120000
+#define GBILU_SMALL_ROWS32 140000
 #endif
 
 // Plans the one-launch solve: its CTAs and the shared memory that the
@@ -730,7 +735,9 @@ cudaError_t launch_small(Handle *h, const SmallArgs<V, T> &A) {
 // After a failed wait the barrier counters no longer hold a multiple of
 // their grid.
 int reset_small(Handle *h, const Ctl &c) {
-  if (c.bar_fail) CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
+  if (!c.bar_fail) return GBILU_OK;
+  CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
+  CK(cudaMemset(h->ctl.p, 0, sizeof(Ctl)));
   return GBILU_OK;
 }
 
@@ -1015,6 +1022,7 @@ int setup_device(Handle *h) {
   CK(h->x0nz.alloc(1));
   CK(cudaMemset(h->x0nz.p, 0xff, sizeof(int)));   // "nonzero" until a gather clears it
   CK(h->ctl.alloc(2));
+  CK(cudaMemset(h->ctl.p, 0, 2 * sizeof(Ctl)));
   CK(h->small_bar.alloc(3));
   CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
   if (h->opt.factor_on_device) {

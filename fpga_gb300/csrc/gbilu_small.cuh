@@ -10,11 +10,17 @@
 // read from L2), three warps share a slice, one per component, so the FP64
 // chain is a third, all gathers of a row are in flight together, a vector
 // entry belongs to one thread for the whole solve, and a step boundary is a
-// grid barrier (about 1.4 us) instead of a kernel boundary. b and x are read
-// and written in the caller's numbering by the same launch. Solves of 4,000
-// cells (to 1e-2, numpy arrays) 356 -> NEW us, 33,000 cells 702 -> NEW us; above
-// kSmallRows (gbilu_api.cu) the separate kernels, with two to three times the
-// warps per SM, are as fast.
+// grid barrier (about 1.5 us) instead of a kernel boundary. ||s|| is summed
+// with the reduction after it, so a stop in a first half has run the second
+// SpMV in vain. b and x are read and written in the caller's numbering by the
+// same launch.
+//
+// Measured against the separate kernels: an iteration of 4,000 cells 59 -> 28
+// us, of 33,000 cells (three colors) 97 -> 53, of 108,000 cells 88 -> 72 (see
+// GBILU_SMALL_ROWS64 for where it ends). Ordering the steps between two
+// reductions by their data instead (results preset to a sentinel, consumers
+// polling) gave 28.7 us for 4,000 cells with two colors, but 47 instead of 44
+// with three and 75 instead of 53 for 33,000 cells: polled loads bypass L1.
 //
 // Per row and component the arithmetic is that of the separate kernels;
 // dot products are summed in this kernel's own fixed order. The scalars are
@@ -39,7 +45,7 @@ template <typename V, typename T> struct SmallArgs {
   Ctl *host_ctl;                  // the final state (mapped host memory)
   unsigned long long *bar;        // barrier counter: a multiple of the grid
   int *x_nonzero;                 // 0 between launches
-  double *partials;               // 5 reductions of up to 3 sums a CTA
+  double *partials;               // 9 sums a CTA
   const int2 *srows;
   int S, S0, S1;                  // slices; the first of the tail, of color 2
   int n0, rows1, split1;          // head rows; Tail's rows1 and split1
@@ -68,18 +74,19 @@ template <typename V, typename T> struct SmallCta {
   uint64_t copies;                // mbarrier of the bulk copies
   int pos[kSmallOwn], w[kSmallOwn], o[kSmallOwn];   // place (-1: L2), width, first slot
   int2 rows[kSmallOwn];
-  double red[3][kSmallThreads];
+  double red[3][kSmallThreads], tot[3];
   T xch[kSmallGroups][3][32];
   int ok;
 };
 
-// Component c of one row: a -+ sum over its blocks' row c times x (L2: other
-// SMs wrote it in this launch). Columns ascend; those from limit on end the
-// row, as padding does. All gathers of a row of up to eight blocks go out
-// together. (Not inlined: its eight sites would spill each other.)
+// Component c of one row: a -+ sum over its blocks' row c times x (other SMs
+// wrote it in this launch, before a grid barrier, whose acquire makes L1 loads
+// see it). Columns ascend; those from limit on end the row, as padding does.
+// All gathers of a row of up to eight blocks go out together. (Not inlined:
+// its sites would spill each other.)
 template <typename V, typename T, bool NEG>
-__device__ __noinline__ T comp_row(const V *sv, const int *sc, int w, int lane, int c,
-                                      const T *x, int limit, T a) {
+__device__ __noinline__ T comp_row(const V *sv, const int *sc, int w, int lane, int c, const T *x,
+                                   int limit, T a) {
   constexpr int B = 8;
   for (int k0 = 0; k0 < w; k0 += B) {
     int cc[B];
@@ -93,9 +100,8 @@ __device__ __noinline__ T comp_row(const V *sv, const int *sc, int w, int lane, 
     for (int j = 0; j < B; ++j)
       if (cc[j] >= 0) {
         const T *xs = x + 3 * cc[j];
-        y[j][0] = __ldcg(xs);
-        y[j][1] = __ldcg(xs + 1);
-        y[j][2] = __ldcg(xs + 2);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) y[j][e] = xs[e];
       }
 #pragma unroll
     for (int j = 0; j < B; ++j)
@@ -179,8 +185,7 @@ template <typename V, typename T> struct SmallSolve {
     const int any_late = __syncthreads_or(late);
     if (threadIdx.x == 0) {
       S.ok = !any_late;
-      if (any_late) mark_stage_timeout(A.ctl);
-      __threadfence();
+      if (any_late && !*(volatile int *)&A.ctl->bar_fail) mark_stage_timeout(A.ctl);
       unsigned long long ticket, now;
       asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
                    : "=l"(ticket) : "l"(A.bar), "l"(1ull) : "memory");
@@ -189,9 +194,10 @@ template <typename V, typename T> struct SmallSolve {
       while (true) {
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(A.bar) : "memory");
         if (now >= target) break;
-        if (++spins > kBarrierSpins) {
+        if (++spins > kBarrierSpins ||
+            ((spins & 1023) == 0 && *(volatile int *)&A.ctl->bar_fail)) {
           S.ok = 0;
-          atomicExch(&A.ctl->bar_fail, 1);
+          atomicCAS(&A.ctl->bar_fail, 0, 1);
           A.ctl->status = ST_TIMEOUT;
           __threadfence();
           atomicExch(&A.ctl->done, 1);
@@ -205,47 +211,50 @@ template <typename V, typename T> struct SmallSolve {
     return !failed;
   }
 
-  // Grid sums of NV doubles per thread in a fixed order, the same in every
-  // CTA; a grid barrier on the way. The totals are valid in thread 0. Slot:
-  // one per reduction of an iteration, so a CTA that is a reduction ahead
-  // does not overwrite what another still reads.
-  template <int NV> __device__ bool sum(double (&v)[NV], int slot) {
+  // Sums of NV doubles per thread over the CTA, in a fixed order, as its
+  // partials of slots slot .. slot + NV - 1. (A warp issues one FP64 add per
+  // 64 cycles: four warps add three values each, then one warp per sum.)
+  template <int NV> __device__ void partial(double (&v)[NV], int slot) {
     const int t = threadIdx.x;
 #pragma unroll
     for (int j = 0; j < NV; ++j) S.red[j][t] = v[j];
     __syncthreads();
     if (t < 128) {
 #pragma unroll
-      for (int j = 0; j < NV; ++j) v[j] = (S.red[j][t] + S.red[j][t + 128]) + S.red[j][t + 256];
+      for (int j = 0; j < NV; ++j)
+        S.red[j][t] = (S.red[j][t] + S.red[j][t + 128]) + S.red[j][t + 256];
     }
     __syncthreads();
-    if (t < 128)
+    if (t < 32 * NV) {
+      const double *q = S.red[t >> 5] + lane;
+      double x = (q[0] + q[32]) + (q[64] + q[96]);
 #pragma unroll
-      for (int j = 0; j < NV; ++j) S.red[j][t] = v[j];
-    __syncthreads();
-    double *part = A.partials + (size_t)slot * 3 * G;
-    if (t < 32) {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        double x = (S.red[j][t] + S.red[j][t + 32]) + (S.red[j][t + 64] + S.red[j][t + 96]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (t == 0) part[j * G + bid] = x;
-      }
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) A.partials[(size_t)(slot + (t >> 5)) * G + bid] = x;
     }
+  }
+
+  // A grid barrier, then the totals of slots slot .. slot + N - 1 in a fixed
+  // order, the same in every CTA, into tot. A slot is written once an
+  // iteration, so no CTA overwrites what another still reads.
+  template <int N> __device__ bool totals(int slot) {
     if (!barrier()) return false;
-    for (int q = t; q < NV * G; q += kSmallThreads) S.red[q / G][q % G] = __ldcg(part + q);
-    __syncthreads();
-    if (t < 32) {
+    const int t = threadIdx.x;
+    if (t < 32 * N) {
+      const double *q = A.partials + (size_t)(slot + (t >> 5)) * G;
+      double x = 0.0;
+      for (int b = 0; b < G; b += 128) {
+        double y[4];
 #pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        double x = 0.0;
-        for (int q = t; q < G; q += 32) x += S.red[j][q];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        v[j] = x;
+        for (int u = 0; u < 4; ++u)
+          y[u] = b + 32 * u + lane < G ? __ldcg(q + b + 32 * u + lane) : 0.0;
+        x += (y[0] + y[1]) + (y[2] + y[3]);
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) S.tot[t >> 5] = x;
     }
+    __syncthreads();
     return true;
   }
 
@@ -300,57 +309,65 @@ template <typename V, typename T> struct SmallSolve {
     while (!late && !mbar_try_wait(&S.copies, 0)) late = ++spins > kStageSpins;
   }
 
+  static constexpr int kNoLimit = 0x7fffffff;
+  template <bool NEG>
+  __device__ T row_sum(const V *sv, const int *sc, int w, const T *x, int limit, T a) const {
+    return comp_row<V, T, NEG>(sv, sc, w, lane, c, x, limit, a);
+  }
+
   // tail_first (gbilu_reduced.cuh) by component, for own slice i: w is the
-  // row's p or s. The small steps follow a grid barrier: no sentinels.
+  // row's p or s.
   __device__ __forceinline__ void first(int i, bool act, int row, T coef, T w, T *hat) {
     if (slice(i) >= A.S1) return;   // the same for the whole group
     const T a = act ? fma(coef, A.base[3 * row + c], w) : (T)0;
     const T z = comp_d<V, T>(S.xch[grp], grp, c, lane, dblk(i), a);
     if (!act) return;
     const bool split = row - A.n0 < A.split1;
-    T *out = split ? A.y : hat;
-    out[3 * row + c] = split && !A.transpose ? a : z;
+    (split ? A.y : hat)[3 * row + c] = split && !A.transpose ? a : z;
   }
 
-  // The reduced apply's steps after the first sweep of color 1, each behind
-  // a grid barrier.
-  __device__ bool apply(const PhaseList &ph, const T *src, T *hat, T coef, bool barrier_first) {
-    for (int q = 0; q < ph.n; ++q) {
-      if ((q > 0 || barrier_first) && !barrier()) return false;
-      if (q + 1 == ph.n) break;
+  // The reduced apply's steps after the first sweep of color 1, in step
+  // order, a grid barrier around each; w: the row's p or s. A small step's
+  // slice belongs to the group that it has in tail(), so a row's own values
+  // are this thread's.
+  __device__ bool apply(const PhaseList &ph, const T *w, T *hat, T coef) {
+    T *y = A.y;
+    for (int q = 0; q + 1 < ph.n; ++q) {
+      if (!barrier()) return false;
       const Phase &P = ph.p[q];
-      const int nsl = (P.nrows + 31) >> 5;
-      const int j0 = ((bid - P.slice0) % G + G) % G;
       const int *off = P.mat ? A.off2 : A.off1r, *col = P.mat ? A.col2 : A.col1r;
       const V *val = P.mat ? A.val2 : A.val1r;
-      if (grp >= kSmallGroups) continue;
-      for (int j = j0 + grp * G; j < nsl; j += kSmallGroups * G) {
-        const int s = P.slice0 + j, r = 32 * j + lane, row = P.row0 + r;
+      const int nsl = (P.nrows + 31) >> 5;
+      int i0 = (P.slice0 - bid + G - 1) / G;   // the first own slice of the step
+      i0 += (grp - (i0 - tail0) % kSmallGroups + kSmallGroups) % kSmallGroups;
+      for (int i = i0; slice(i) < P.slice0 + nsl; i += kSmallGroups) {
+        const int s = slice(i), r = 32 * (s - P.slice0) + lane, row = P.row0 + r;
         const bool act = r < P.nrows;
         const V *d = A.dmat + (size_t)s * 9 * 32;
         T a = 0;
         if (act) {
           const int e = 3 * row + c;
-          a = P.own_y ? __ldcg(A.y + e) : fma(coef, __ldcg(A.base + e), __ldcg(src + e));
-          const int o = off[s];
-          a = comp_row<V, T, true>(val + (size_t)o * 9 * 32, col + (size_t)o * 32, off[s + 1] - o,
-                                   lane, c, P.nbr_hat ? hat : A.y, 0x7fffffff, a);
+          const int o = off[s], wd = off[s + 1] - o;
+          a = P.own_y ? y[e] : fma(coef, A.base[e], w[e]);
+          a = row_sum<true>(val + (size_t)o * 9 * 32, col + (size_t)o * 32, wd,
+                                  P.nbr_hat ? hat : y, kNoLimit, a);
         }
         if (P.has_d) a = comp_d<V, T>(S.xch[grp], grp, c, lane, d, a);
         bool fin = true;
         if (P.to_y) {
           fin = row >= P.final0;
-          if (act && !fin) A.y[3 * row + c] = a;
+          if (act && !fin) y[3 * row + c] = a;
           if (P.final_d) a = comp_d<V, T>(S.xch[grp], grp, c, lane, d, a);
         }
         if (act && fin) hat[3 * row + c] = a;
       }
     }
+    if (!barrier()) return false;
     head([&](int i, bool act, int row) {
       T a = 0;
       if (act)
-        a = comp_row<V, T, true>(vals(i), cols(i), S.w[i], lane, c, hat, 0x7fffffff,
-                                 A.base[3 * row + c] * coef);
+        a = row_sum<true>(vals(i), cols(i), S.w[i], hat, 0x7fffffff,
+                                A.base[3 * row + c] * coef);
       if (!A.transpose) a = comp_d<V, T>(S.xch[grp], grp, c, lane, dblk(i), a);
       if (act) hat[3 * row + c] = a;
     });
@@ -384,8 +401,8 @@ template <typename V, typename T> struct SmallSolve {
         const int e = 3 * row + c, s = slice(i), o = A.offA[s];
         double q = 0.0;
         if (mul)
-          q = comp_row<V, T, false>(A.valA + (size_t)o * 9 * 32, A.colA + (size_t)o * 32,
-                                    A.offA[s + 1] - o, lane, c, A.x, 0x7fffffff, 0.0);
+          q = row_sum<false>(A.valA + (size_t)o * 9 * 32, A.colA + (size_t)o * 32,
+                                    A.offA[s + 1] - o, A.x, kNoLimit, 0.0);
         set(i, e, A.b[e] - q);
       });
     } else {
@@ -397,8 +414,9 @@ template <typename V, typename T> struct SmallSolve {
       });
     }
     double v[2] = {total(d, f), total(dh, fh)};
-    if (!sum(v, 0)) return false;
-    if (threadIdx.x == 0) finish_init<T>(&S.c, v[0] + v[1], 1, v[1]);
+    partial(v, 0);
+    if (!totals<2>(0)) return false;
+    if (threadIdx.x == 0) finish_init<T>(&S.c, S.tot[0] + S.tot[1], 1, S.tot[1]);
     __syncthreads();
     if (S.c.done) return true;
     wait_copies();
@@ -415,8 +433,8 @@ template <typename V, typename T> struct SmallSolve {
       T w = 0;
       if (act) {
         const int o = A.off1[s];
-        A.base[e] = comp_row<V, T, true>(A.val1 + (size_t)o * 9 * 32, A.col1 + (size_t)o * 32,
-                                         A.off1[s + 1] - o, lane, c, A.base, A.n0, (T)0);
+        A.base[e] = row_sum<true>(A.val1 + (size_t)o * 9 * 32, A.col1 + (size_t)o * 32,
+                                         A.off1[s + 1] - o, A.base, A.n0, (T)0);
         w = A.p[e];
       }
       first(i, act, row, (T)1, w, A.ph);
@@ -427,21 +445,21 @@ template <typename V, typename T> struct SmallSolve {
   __device__ bool iterate(const PhaseList &ph) {
     Ctl &k = S.c;
     while (true) {
-      if (!apply(ph, A.p, A.ph, (T)k.cp, true)) return false;
+      if (!apply(ph, A.p, A.ph, (T)k.cp)) return false;
       {
         double d = 0.0;
         DF f = {0.f, 0.f};
         tail([&](int i, bool act, int row) {
           if (!act) return;
           const int e = 3 * row + c;
-          const T a = comp_row<V, T, false>(vals(i), cols(i), S.w[i], lane, c, A.ph, 0x7fffffff,
-                                            (T)0);
+          const T a = row_sum<false>(vals(i), cols(i), S.w[i], A.ph, kNoLimit, (T)0);
           A.v[e] = a;
           add(d, f, a, A.rt[e]);
         });
         double v[1] = {total(d, f)};
-        if (!sum(v, 1)) return false;
-        if (threadIdx.x == 0) finish_alpha(&k, v[0]);
+        partial(v, 2);
+        if (!totals<1>(2)) return false;
+        if (threadIdx.x == 0) finish_alpha(&k, S.tot[0]);
         __syncthreads();
         if (k.done) return true;
       }
@@ -459,28 +477,24 @@ template <typename V, typename T> struct SmallSolve {
           }
           first(i, act, row, cs, s, A.sh);
         });
-        double v[1] = {total(d, f)};
-        if (!sum(v, 2)) return false;
-        if (threadIdx.x == 0) finish_s(&k, v[0]);
-        __syncthreads();
-        if (k.done) return true;
-      }
-      if (!apply(ph, A.s, A.sh, (T)k.cs, false)) return false;
-      {
+        if (!apply(ph, A.s, A.sh, cs)) return false;
         double d1 = 0.0, d2 = 0.0;
         DF f1 = {0.f, 0.f}, f2 = {0.f, 0.f};
         tail([&](int i, bool act, int row) {
           if (!act) return;
           const int e = 3 * row + c;
-          const T a = comp_row<V, T, false>(vals(i), cols(i), S.w[i], lane, c, A.sh, 0x7fffffff,
-                                            (T)0);
+          const T a = row_sum<false>(vals(i), cols(i), S.w[i], A.sh, kNoLimit, (T)0);
           A.t[e] = a;
           add(d1, f1, a, A.s[e]);
           add(d2, f2, a, a);
         });
-        double v[2] = {total(d1, f1), total(d2, f2)};
-        if (!sum(v, 3)) return false;
-        if (threadIdx.x == 0) finish_omega(&k, v[0], v[1]);
+        double v[3] = {total(d, f), total(d1, f1), total(d2, f2)};
+        partial(v, 3);
+        if (!totals<3>(3)) return false;
+        if (threadIdx.x == 0) {
+          finish_s(&k, S.tot[0]);
+          if (!k.done) finish_omega(&k, S.tot[1], S.tot[2]);
+        }
         __syncthreads();
         if (k.done) return true;
       }
@@ -491,7 +505,7 @@ template <typename V, typename T> struct SmallSolve {
         tail([&](int i, bool act, int row) {
           if (!act) return;
           const int e = 3 * row + c;
-          A.x[e] = fma(omega, __ldcg(A.sh + e), fma(alpha, __ldcg(A.ph + e), A.x[e]));
+          A.x[e] = fma(omega, A.sh[e], fma(alpha, A.ph[e], A.x[e]));
           const T r = fma(-omega, A.t[e], A.s[e]);
           A.r[e] = r;
           add(d1, f1, r, r);
@@ -502,8 +516,9 @@ template <typename V, typename T> struct SmallSolve {
         if (A.timeout_ns && bid == 0 && threadIdx.x == 0 &&
             globaltimer() - k.t_start > A.timeout_ns)
           v[2] = 1.0;
-        if (!sum(v, 4)) return false;
-        if (threadIdx.x == 0) finish_r(&k, v[0], v[1], v[2] != 0.0);
+        partial(v, 6);
+        if (!totals<3>(6)) return false;
+        if (threadIdx.x == 0) finish_r(&k, S.tot[0], S.tot[1], S.tot[2] != 0.0);
         __syncthreads();
         if (k.done) return true;
       }
@@ -532,7 +547,7 @@ template <typename V, typename T> struct SmallSolve {
         const T alpha = (T)k.alpha;
         tail([&](int i, bool act, int row) {
           const int e = 3 * row + c;
-          if (act) A.x[e] = fma(alpha, __ldcg(A.ph + e), A.x[e]);
+          if (act) A.x[e] = fma(alpha, A.ph[e], A.x[e]);
         });
       }
       if (!barrier()) return false;
@@ -542,8 +557,7 @@ template <typename V, typename T> struct SmallSolve {
         const int e = 3 * row + c;
         T a = act ? fma(-cc, A.rt[e], b[e]) : (T)0;
         if (A.transpose) a = comp_d<V, T>(S.xch[grp], grp, c, lane, dblk(i), a);
-        if (act)
-          a = comp_row<V, T, true>(vals(i), cols(i), S.w[i], lane, c, A.x, 0x7fffffff, a);
+        if (act) a = row_sum<true>(vals(i), cols(i), S.w[i], A.x, kNoLimit, a);
         if (!A.transpose) a = comp_d<V, T>(S.xch[grp], grp, c, lane, dblk(i), a);
         if (act) A.x[e] = a;
       });
