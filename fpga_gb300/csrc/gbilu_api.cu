@@ -76,6 +76,8 @@ template <typename V, typename T> struct Ops {
 
 }  // namespace
 
+constexpr int kMaxChunks = 32;            // of the input values of a factorization
+
 struct Handle {
   gbilu_options opt{};
   std::string err;
@@ -94,9 +96,8 @@ struct Handle {
   cudaEvent_t e_x = nullptr, e_b = nullptr;
   DevBuf<int2> srows;
   // perm/iperm: device row <-> input row (the vectors of a solve; lambda
-  // of the gradient); dperm: device row -> permuted row (the device
-  // factorization's layout); prowptr, pcol, psrc: the permuted pattern
-  DevBuf<int> perm, iperm, dperm, prowptr, pcol, psrc;
+  // of the gradient); prowptr, pcol, psrc: the permuted pattern
+  DevBuf<int> perm, iperm, prowptr, pcol, psrc;
   DevBuf<int> ibrow, icol;                   // input pattern: block -> row, column (dL/dA)
   DevMat A, L, U, At, Ut, Lt;
   DevMat Lr, Utr;            // L and U^T without color 0's columns
@@ -109,6 +110,19 @@ struct Handle {
   // device factorization: permuted values (factored in place), inverses
   DevBuf<int> pdiag, bad;
   DevBuf<double> pbuf, vals_in, dinvp;
+  // where each input block goes: permuted order, slot lane of A and of A^T
+  DevBuf<int> pblk, apos, tpos;
+  DevBuf<int> mate, fpos, ftpos, frpos, drow;   // see k_bilu0_rows, FactorOut
+  // the input values cross the link in chunks of whole block rows; a color's
+  // rows that chunk c completes: run [begin, ready[c]) of each run of colors
+  // 0 and 1 (split rows, other rows), see plan_chunks
+  struct Run {
+    int color, row0, rows;
+    std::vector<int> ready;
+  };
+  std::vector<long long> chunk;            // first block of each chunk, and nnzb
+  std::vector<Run> runs;
+  cudaEvent_t e_chunk[kMaxChunks] = {};
   bool host_factors_stale = false;
   std::unique_ptr<FpgaExport> fpga;        // the last gbilu_fpga_export (sizes query)
   DevBuf<Ctl> ctl;                         // [0] main run, [1] refinement residual
@@ -184,6 +198,11 @@ int grid_for(const Handle *h, long long work) {
   long long g = (work + kThreads - 1) / kThreads;
   const long long cap = (long long)h->sm_count * 8;
   return (int)std::max<long long>(1, std::min(g, cap));
+}
+
+// Kernels with one thread per entry of a block (kEntryThreads).
+int entry_grid(const Handle *h, long long blocks) {
+  return (int)std::max<long long>(1, std::min((blocks + 31) / 32, (long long)h->sm_count * 7));
 }
 
 // Kernels that end in a grid reduction: fewer, fuller CTAs, so the
@@ -934,7 +953,9 @@ void release_device(Handle *h) {
       for (auto &sw : prec) sw.release();
   h->pdiag.release(); h->bad.release(); h->pbuf.release(); h->vals_in.release();
   h->dinvp.release();
-  h->srows.release(); h->perm.release(); h->iperm.release(); h->dperm.release();
+  h->pblk.release(); h->apos.release(); h->tpos.release(); h->mate.release();
+  h->fpos.release(); h->ftpos.release(); h->frpos.release(); h->drow.release();
+  h->srows.release(); h->perm.release(); h->iperm.release();
   h->ibrow.release(); h->icol.release();
   h->prowptr.release(); h->pcol.release();
   h->psrc.release(); h->dinv64.release(); h->dinvT64.release(); h->dinv32.release();
@@ -947,6 +968,46 @@ void release_device(Handle *h) {
   h->device_bytes = 0;
 }
 
+// The chunks of a factorization's input and, for each run of rows of colors 0
+// and 1 (a color's split rows, its other rows: each in input order), the
+// leading rows whose blocks, and whose neighbours', have arrived with chunk
+// c. On a grid in natural order that is all but a few layers of the rows up
+// to the chunk's end; on any pattern the rows that wait longer are done with
+// a later chunk.
+void plan_chunks(Handle *h) {
+  const Analysis &an = h->an;
+  // 32 MB cross the link in 160 us; a chunk's own kernels take about 100
+  const long long per = 32ll << 20;
+  const int n = (int)std::max<long long>(
+      1, std::min<long long>(kMaxChunks, (long long)an.nnzb * 72 / per));
+  std::vector<int> row_end(n);             // first input row after each chunk
+  h->chunk.assign(1, 0);
+  for (int c = 0; c < n; ++c) {
+    const long long want = (long long)an.nnzb * (c + 1) / n;
+    const int row = c + 1 == n ? an.nb
+                               : (int)(std::lower_bound(an.rowptr.begin(), an.rowptr.end(), want) -
+                                       an.rowptr.begin());
+    row_end[c] = std::min(row, an.nb);
+    h->chunk.push_back(an.rowptr[row_end[c]]);
+  }
+  h->runs.clear();
+  for (int col = 0; col < std::min(2, an.ncolors); ++col)
+    for (int part = 0; part < 2; ++part) {
+      const int b = an.color_ptr[col] + (part ? an.split[col] : 0);
+      const int e = part ? an.color_ptr[col + 1] : an.color_ptr[col] + an.split[col];
+      Handle::Run run{col, b, e - b, std::vector<int>(n, 0)};
+      int c = 0;
+      for (int i = b; i < e; ++i) {
+        const int o = an.perm[i];
+        int last = o;
+        if (col > 0) last = std::max(o, an.colind[an.rowptr[o + 1] - 1]);
+        while (last >= row_end[c]) run.ready[c++] = i - b;   // the prefix so far
+      }
+      for (; c < n; ++c) run.ready[c] = run.rows;
+      h->runs.push_back(std::move(run));
+    }
+}
+
 // Allocates the device side for the current analysis (structure only).
 int setup_device(Handle *h) {
   if (h->opt.device < 0) return h->fail(GBILU_NO_DEVICE, "host-only handle has no device");
@@ -957,6 +1018,7 @@ int setup_device(Handle *h) {
     CK(cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&h->e_x, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&h->e_b, cudaEventDisableTiming));
+    for (auto &e : h->e_chunk) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaEventCreate(&h->e0));
     CK(cudaEventCreate(&h->e1));
     CK(cudaMallocHost(&h->h_ctl, sizeof(Ctl)));
@@ -984,8 +1046,6 @@ int setup_device(Handle *h) {
     CK(h->iperm.alloc(an.nb));
     CK(cudaMemcpy(h->iperm.p, idv.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice));
   }
-  CK(h->dperm.alloc(an.nb));
-  CK(cudaMemcpy(h->dperm.p, an.dperm.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice));
   {
     std::vector<int> br(an.nnzb);
     for (int i = 0; i < an.nb; ++i)
@@ -1032,6 +1092,47 @@ int setup_device(Handle *h) {
     CK(h->pbuf.alloc((size_t)an.nnzb * 9));
     CK(h->vals_in.alloc((size_t)an.nnzb * 9));
     CK(h->dinvp.alloc((size_t)an.nb * 9));
+    // the sliced arrays are written block by block: their padding stays zero
+    for (DevMat *m : {&h->A, &h->At, &h->L, &h->U, &h->Lt, &h->Ut, &h->Lr, &h->Utr}) {
+      CK(cudaMemsetAsync(m->v64.p, 0, m->v64.n * sizeof(double), h->st));
+      if (h->with_32) CK(cudaMemsetAsync(m->v32.p, 0, m->v32.n * sizeof(float), h->st));
+    }
+    CK(cudaMemsetAsync(h->dinv64.p, 0, nd * sizeof(double), h->st));
+    CK(cudaMemsetAsync(h->dinvT64.p, 0, nd * sizeof(double), h->st));
+    if (h->with_32) {
+      CK(cudaMemsetAsync(h->dinv32.p, 0, nd * sizeof(float), h->st));
+      CK(cudaMemsetAsync(h->dinvT32.p, 0, nd * sizeof(float), h->st));
+    }
+    // where each block goes: pblk, apos, tpos by input block, the others by
+    // permuted block (of a diagonal block: unused)
+    for (DevBuf<int> *b : {&h->pblk, &h->apos, &h->tpos, &h->mate, &h->fpos, &h->ftpos, &h->frpos})
+      CK(b->alloc(an.nnzb));
+    CK(cudaMemsetAsync(h->frpos.p, 0xff, an.nnzb * sizeof(int), h->st));
+    CK(h->drow.alloc(an.nb));
+    CK(cudaMemcpyAsync(h->drow.p, an.idperm.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice, h->st));
+    const int gi = grid_for(h, an.nnzb);
+    k_mates<<<grid_for(h, an.nb), kThreads, 0, h->st>>>(an.nb, h->prowptr.p, h->pcol.p, h->pdiag.p,
+                                                        h->mate.p);
+    k_invert<<<gi, kThreads, 0, h->st>>>(an.nnzb, h->psrc.p, h->pblk.p);
+    auto positions = [&](DevMat &m, const int *psrc, DevBuf<int> &pos) {
+      if (m.slots)
+        k_block_positions<<<gi, kThreads, 0, h->st>>>(m.slots * 32, m.vsrc.p, psrc, pos.p);
+      h->device_bytes -= (size_t)m.slots * 32 * sizeof(int);
+    };
+    positions(h->A, h->psrc.p, h->apos);
+    positions(h->At, h->psrc.p, h->tpos);
+    positions(h->L, nullptr, h->fpos);
+    positions(h->U, nullptr, h->fpos);
+    positions(h->Lt, nullptr, h->ftpos);
+    positions(h->Ut, nullptr, h->ftpos);
+    positions(h->Lr, nullptr, h->frpos);
+    positions(h->Utr, nullptr, h->frpos);
+    CK(cudaStreamSynchronize(h->st));
+    CK(cudaGetLastError());
+    for (DevMat *m : {&h->A, &h->At, &h->L, &h->U, &h->Lt, &h->Ut, &h->Lr, &h->Utr})
+      m->vsrc.release();
+    plan_chunks(h);
+    h->device_bytes += (size_t)an.nnzb * 28 + (size_t)an.nb * 4;
     h->device_bytes += (size_t)an.nnzb * 9 * 16 + (size_t)an.nb * 76;
   }
   for (int red = 0; red < 2; ++red)
@@ -1069,57 +1170,65 @@ int setup_device(Handle *h) {
   return GBILU_OK;
 }
 
-// Sliced values of one matrix (FP64 and, in the mixed mode, FP32) from
-// per-block device values.
-void fill_mat_device(Handle *h, DevMat &m, const double *src) {
-  if (m.slots == 0) return;
-  const int g = grid_for(h, m.slots * 32);
-  k_fill_sliced<double><<<g, kThreads, 0, h->st>>>(m.slots, m.vsrc.p, m.transpose ? 1 : 0, src, m.v64.p);
-  if (h->with_32)
-    k_fill_sliced<float><<<g, kThreads, 0, h->st>>>(m.slots, m.vsrc.p, m.transpose ? 1 : 0, src, m.v32.p);
+FactorOut factor_out(Handle *h) {
+  return FactorOut{h->fpos.p, h->ftpos.p, h->frpos.p, h->drow.p,
+                   h->L.v64.p, h->U.v64.p, h->Lt.v64.p, h->Ut.v64.p, h->Lr.v64.p, h->Utr.v64.p,
+                   h->dinv64.p, h->dinvT64.p,
+                   h->L.v32.p, h->U.v32.p, h->Lt.v32.p, h->Ut.v32.p, h->Lr.v32.p, h->Utr.v32.p,
+                   h->dinv32.p, h->dinvT32.p};
 }
 
-// Permute, factor and lay out on the device: values in input order (host
-// array) -> color-permuted blocks -> A and A^T slices -> IKJ block ILU(0)
-// color by color in place -> L, U, U^T, L^T and the inverse diagonal blocks.
+// Factors rows row_a .. and row_b .. of one color.
+void bilu0_rows(Handle *h, const FactorOut &F, int color, int row_a, int rows_a, int row_b = 0,
+                int rows_b = 0) {
+  const int rows = rows_a + rows_b;
+  if (rows <= 0) return;
+  k_bilu0_rows<<<(rows + kBiluRows - 1) / kBiluRows, kThreads, 0, h->st>>>(
+      row_a, rows_a, row_b, rows_b, h->an.color_ptr[color], h->an.slice_color_ptr[color],
+      h->prowptr.p, h->pcol.p, h->pdiag.p, h->mate.p, h->pbuf.p, h->dinvp.p, F, h->bad.p);
+}
+
+// Permute, factor and lay out on the device: the values (host array, input
+// order) cross the link in chunks on the auxiliary stream; behind each, its
+// blocks go to the permuted order, A and A^T, and the rows of colors 0 and 1
+// that it completes are factored, into L, U, U^T, L^T and the inverse
+// diagonal blocks; then the other colors. 500k cells: NEW.
 int factor_device(Handle *h, const double *vals) {
   const Analysis &an = h->an;
-  const size_t n9 = (size_t)an.nnzb * 9;
-  CK(cudaMemcpyAsync(h->vals_in.p, vals, n9 * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  k_permute_blocks<<<grid_for(h, (long long)n9), kThreads, 0, h->st>>>(an.nnzb, h->psrc.p,
-                                                                       h->vals_in.p, h->pbuf.p);
-  fill_mat_device(h, h->A, h->pbuf.p);
-  fill_mat_device(h, h->At, h->pbuf.p);
-  const int big = 0x7fffffff;
-  CK(cudaMemcpyAsync(h->bad.p, &big, sizeof(int), cudaMemcpyHostToDevice, h->st));
-  for (int c = 0; c < an.ncolors; ++c) {
-    const int row0 = an.color_ptr[c], rows = an.color_ptr[c + 1] - row0;
-    k_bilu0_color<<<(rows + kThreads - 1) / kThreads, kThreads, 0, h->st>>>(
-        row0, rows, h->prowptr.p, h->pcol.p, h->pdiag.p, h->pbuf.p, h->dinvp.p, h->bad.p);
+  CK(cudaMemsetAsync(h->bad.p, 0x7f, sizeof(int), h->st));
+  const int none = 0x7f7f7f7f;
+  // the values of an earlier factorization may still be read on st
+  CK(cudaEventRecord(h->e_x, h->st));
+  CK(cudaStreamWaitEvent(h->aux, h->e_x, 0));
+  const FactorOut F = factor_out(h);
+  const int n = (int)h->chunk.size() - 1;
+  for (int c = 0; c < n; ++c) {
+    const long long k0 = h->chunk[c], nk = h->chunk[c + 1] - k0;
+    if (nk > 0) {
+      CK(cudaMemcpyAsync(h->vals_in.p + 9 * k0, vals + 9 * k0, 9 * nk * sizeof(double),
+                         cudaMemcpyHostToDevice, h->aux));
+      CK(cudaEventRecord(h->e_chunk[c], h->aux));
+      CK(cudaStreamWaitEvent(h->st, h->e_chunk[c], 0));
+      k_scatter_blocks<<<entry_grid(h, nk), kEntryThreads, 0, h->st>>>(
+          (int)k0, (int)nk, h->vals_in.p, h->pblk.p, h->apos.p, h->tpos.p, h->pbuf.p, h->A.v64.p, h->At.v64.p,
+          h->with_32 ? h->A.v32.p : nullptr, h->with_32 ? h->At.v32.p : nullptr);
+    }
+    for (size_t q = 0; q + 1 < h->runs.size(); q += 2) {   // a color's two runs
+      const Handle::Run &a = h->runs[q], &b = h->runs[q + 1];
+      const int fa = c ? a.ready[c - 1] : 0, fb = c ? b.ready[c - 1] : 0;
+      bilu0_rows(h, F, a.color, a.row0 + fa, a.ready[c] - fa, b.row0 + fb, b.ready[c] - fb);
+    }
   }
-  int bad = big;
-  CK(cudaMemcpyAsync(&bad, h->bad.p, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+  for (int c = 2; c < an.ncolors; ++c)
+    bilu0_rows(h, F, c, an.color_ptr[c], an.color_ptr[c + 1] - an.color_ptr[c]);
+  int *bad = reinterpret_cast<int *>(h->h_inner);   // pinned
+  CK(cudaMemcpyAsync(bad, h->bad.p, sizeof(int), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
   CK(last_error(h));
-  if (bad != big)
+  if (*bad != none)
     return h->fail(GBILU_SINGULAR,
-                   "gbilu_factor: singular diagonal block in permuted row %d (input row %d)", bad,
-                   an.perm[bad]);
-  fill_mat_device(h, h->L, h->pbuf.p);
-  fill_mat_device(h, h->U, h->pbuf.p);
-  fill_mat_device(h, h->Lt, h->pbuf.p);
-  fill_mat_device(h, h->Ut, h->pbuf.p);
-  fill_mat_device(h, h->Lr, h->pbuf.p);
-  fill_mat_device(h, h->Utr, h->pbuf.p);
-  const int gd = grid_for(h, (long long)an.S * 32);
-  k_fill_diag<double><<<gd, kThreads, 0, h->st>>>(an.S, h->srows.p, h->dperm.p, 0, h->dinvp.p, h->dinv64.p);
-  k_fill_diag<double><<<gd, kThreads, 0, h->st>>>(an.S, h->srows.p, h->dperm.p, 1, h->dinvp.p, h->dinvT64.p);
-  if (h->with_32) {
-    k_fill_diag<float><<<gd, kThreads, 0, h->st>>>(an.S, h->srows.p, h->dperm.p, 0, h->dinvp.p, h->dinv32.p);
-    k_fill_diag<float><<<gd, kThreads, 0, h->st>>>(an.S, h->srows.p, h->dperm.p, 1, h->dinvp.p, h->dinvT32.p);
-  }
-  CK(cudaStreamSynchronize(h->st));
-  CK(last_error(h));
+                   "gbilu_factor: singular diagonal block in permuted row %d (input row %d)", *bad,
+                   an.perm[*bad]);
   h->host_factors_stale = true;
   return GBILU_OK;
 }
@@ -1486,6 +1595,7 @@ int gbilu_destroy(void *handle) {
     cudaStreamDestroy(h->aux);
     cudaEventDestroy(h->e_x);
     cudaEventDestroy(h->e_b);
+    for (auto &e : h->e_chunk) cudaEventDestroy(e);
     cudaEventDestroy(h->e0);
     cudaEventDestroy(h->e1);
     cudaFreeHost(h->h_ctl);
@@ -1711,7 +1821,7 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
         CK(cudaMemcpyAsync(h->io64.p, gx, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
         xin = h->io64.p;
       }
-      k_grad_a<<<grid_for(h, (long long)h->an.nnzb * 9), kThreads, 0, h->st>>>(
+      k_grad_a<<<entry_grid(h, h->an.nnzb), kEntryThreads, 0, h->st>>>(
           h->an.nnzb, h->ibrow.p, h->icol.p, dx, xin, device_ptrs ? gdA : h->dA.p);
       ++launches;
     }
@@ -1787,7 +1897,7 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
         xin = h->io64.p;
       }
       k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, h->v64.x.p, h->v64.r.p);
-      k_grad_a<<<grid_for(h, (long long)h->an.nnzb * 9), kThreads, 0, h->st>>>(
+      k_grad_a<<<entry_grid(h, h->an.nnzb), kEntryThreads, 0, h->st>>>(
           h->an.nnzb, h->ibrow.p, h->icol.p, h->v64.r.p, xin, device_ptrs ? gdA : h->dA.p);
       launches += 2;
     }

@@ -1979,17 +1979,15 @@ k_dot_check(Ctl *ctl, int n, const float *__restrict__ x, const float *__restric
 // order; lambda and x are read in the input numbering. (A thread per
 // permuted row spread each store over 32 cache lines, a warp per row waited
 // on a chain of dependent loads, a thread per entry of the permuted pattern
-// wrote scattered blocks: 1.44, 0.51 and 0.47 ms for the 2M-cell system.)
-__global__ void __launch_bounds__(kThreads)
-k_grad_a(long long nnzb, const int *__restrict__ brow, const int *__restrict__ col,
+// wrote scattered blocks: 1.44, 0.51 and 0.47 ms for the 2M-cell system; this
+// with a 64-bit division per entry 0.32, without NEW.)
+constexpr int kEntryThreads = 9 * 32;   // one thread per entry of 32 blocks
+__global__ void __launch_bounds__(kEntryThreads)
+k_grad_a(int nnzb, const int *__restrict__ brow, const int *__restrict__ col,
          const double *__restrict__ lam, const double *__restrict__ x, double *__restrict__ dA) {
-  const long long n = 9 * nnzb;
-  for (long long t = blockIdx.x * (long long)kThreads + threadIdx.x; t < n;
-       t += (long long)gridDim.x * kThreads) {
-    const long long b = t / 9;
-    const int e = (int)(t - 9 * b);
-    dA[t] = -lam[3 * brow[b] + e / 3] * x[3 * col[b] + e % 3];
-  }
+  const int e = threadIdx.x % 9, r = e / 3, c = e % 3;
+  for (long long b = blockIdx.x * 32 + threadIdx.x / 9; b < nnzb; b += (long long)gridDim.x * 32)
+    dA[9 * b + e] = -lam[3 * brow[b] + r] * x[3 * col[b] + c];
 }
 
 // --------------------------------------------------------------------------
@@ -2003,124 +2001,227 @@ __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 
-__device__ __forceinline__ void mul3_exact(const double *a, const double *b, double *o) {
+// row a0 a1 a2 of a 3x3 block times block b
+__device__ __forceinline__ void mul_row_exact(double a0, double a1, double a2, const double *b,
+                                              double (&o)[3]) {
 #pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      o[r * 3 + c] = dadd(dadd(dmul(a[r * 3], b[c]), dmul(a[r * 3 + 1], b[3 + c])),
-                          dmul(a[r * 3 + 2], b[6 + c]));
+  for (int c = 0; c < 3; ++c)
+    o[c] = dadd(dadd(dmul(a0, b[c]), dmul(a1, b[3 + c])), dmul(a2, b[6 + c]));
 }
 
-// 3x3 inverse by cofactors; false when the block is singular or not finite
-__device__ __forceinline__ bool inv3_exact(const double *a, double *o) {
+// One chunk of input blocks [k0, k0 + nk), just copied to vals: their values
+// in the color-permuted order (pv, block pblk[k]) and in the sliced A and A^T
+// (slot lane apos[k], tpos[k]). Runs beside the next chunk's copy over the
+// CPU-GPU link, which takes longer, so the scattered 8-byte stores (rows of
+// one color alternate in the input, so neighbouring lanes of a slice meet in
+// L2) cost nothing; the padding of the slices was zeroed when they were made.
+__global__ void __launch_bounds__(kEntryThreads)
+k_scatter_blocks(int k0, int nk, const double *__restrict__ vals, const int *__restrict__ pblk,
+                 const int *__restrict__ apos, const int *__restrict__ tpos,
+                 double *__restrict__ pv, double *__restrict__ a64, double *__restrict__ t64,
+                 float *__restrict__ a32, float *__restrict__ t32) {
+  const int e = threadIdx.x % 9, et = (e % 3) * 3 + e / 3;
+  for (int k = k0 + blockIdx.x * 32 + threadIdx.x / 9; k < k0 + nk; k += gridDim.x * 32) {
+    const double x = __ldcs(vals + 9 * (size_t)k + e);
+    const int pa = apos[k], pt = tpos[k];
+    pv[(size_t)pblk[k] * 9 + e] = x;
+    a64[sl_idx<double>((size_t)(pa >> 5), e, pa & 31)] = x;
+    t64[sl_idx<double>((size_t)(pt >> 5), et, pt & 31)] = x;
+    if (a32) {
+      a32[sl_idx<float>((size_t)(pa >> 5), e, pa & 31)] = (float)x;
+      t32[sl_idx<float>((size_t)(pt >> 5), et, pt & 31)] = (float)x;
+    }
+  }
+}
+
+// pos[b] = q over the slot lanes q of a sliced matrix that hold a block:
+// where each block goes, b its input block (psrc: permuted -> input block) or,
+// without psrc, its permuted one.
+__global__ void k_block_positions(long long n, const int *__restrict__ vsrc,
+                                  const int *__restrict__ psrc, int *__restrict__ pos) {
+  for (long long q = blockIdx.x * (long long)kThreads + threadIdx.x; q < n;
+       q += (long long)gridDim.x * kThreads)
+    if (vsrc[q] >= 0) pos[psrc ? psrc[vsrc[q]] : vsrc[q]] = (int)q;
+}
+__global__ void k_invert(int n, const int *__restrict__ src, int *__restrict__ inv) {
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) inv[src[i]] = i;
+}
+
+// IKJ block ILU(0) of rows of one color (rows of one color are never
+// coupled, and the rows of earlier colors that they read are final): for each
+// k < i in row i, L_ik = A_ik U_kk^-1, then A_ij -= L_ik U_kj for the j > k
+// present in both rows (a merge of the two sorted column lists);
+// D_i^-1 = inv(A_ii) by cofactors. A singular (or not finite) pivot records
+// the smallest failing row in *bad. Finished blocks also go straight to the
+// sliced L, U, their transposes and D^-1, D^-T (FactorOut): the FP64 unit
+// bounds the kernel, and a pass of its own for each array took 0.2 ms more.
+//
+// Three threads a row, one per row of its blocks: row r of L_ik and of every
+// update needs row r of A_ik alone, so they meet only in the inverse. On a
+// grid the one j > k that rows i and k share is i itself: mate[kk] says where
+// block (k, i) is, so the loads of all L blocks of a row are independent and
+// the next block's go out before this one's products (kMoreShared: the rows
+// share other columns too, found by the merge). The FP64 unit bounds it (99
+// operations, rounded one by one, per L block: 0.28 ms for color 1 of the
+// 500k-cell system); one thread a row, merging, took 0.67 ms, waiting for its
+// own chain of index loads, products and updates, and 0.15-0.17 ms for colors
+// of a few hundred rows.
+//
+// Finished blocks also go straight to the sliced L, U, their transposes, the
+// reduced iteration's copies and D^-1, D^-T (FactorOut): the stores ride
+// along with the arithmetic, where a pass of its own for each array took 0.2
+// ms after it.
+struct FactorOut {
+  const int *fpos, *tpos, *rpos;   // slot lane of a permuted block in L or U, in
+                                   // their transposes, in Lr or Utr (-1: none)
+  const int *drow;                 // permuted row -> device row
+  double *L, *U, *Lt, *Ut, *Lr, *Utr, *D, *Dt;
+  float *L32, *U32, *Lt32, *Ut32, *Lr32, *Utr32, *D32, *Dt32;   // null without FP32
+};
+
+// Row r (x0, x1, x2) of block b, which is an L block (lower) or a U block
+__device__ __forceinline__ void store_factor(const FactorOut &F, int b, bool lower, int r,
+                                             double x0, double x1, double x2) {
+  const int p = F.fpos[b], t = F.tpos[b], q = F.rpos[b];
+  const double x[3] = {x0, x1, x2};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    (lower ? F.L : F.U)[sl_idx<double>((size_t)(p >> 5), 3 * r + c, p & 31)] = x[c];
+    (lower ? F.Lt : F.Ut)[sl_idx<double>((size_t)(t >> 5), 3 * c + r, t & 31)] = x[c];
+    if (q >= 0) {   // Lr is by rows, Utr by columns
+      const int e = lower ? 3 * r + c : 3 * c + r;
+      (lower ? F.Lr : F.Utr)[sl_idx<double>((size_t)(q >> 5), e, q & 31)] = x[c];
+    }
+  }
+  if (F.L32) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      (lower ? F.L32 : F.U32)[sl_idx<float>((size_t)(p >> 5), 3 * r + c, p & 31)] = (float)x[c];
+      (lower ? F.Lt32 : F.Ut32)[sl_idx<float>((size_t)(t >> 5), 3 * c + r, t & 31)] = (float)x[c];
+      if (q >= 0) {
+        const int e = lower ? 3 * r + c : 3 * c + r;
+        (lower ? F.Lr32 : F.Utr32)[sl_idx<float>((size_t)(q >> 5), e, q & 31)] = (float)x[c];
+      }
+    }
+  }
+}
+
+constexpr int kBiluRows = kThreads / 32 * 10;   // rows a CTA: ten a warp
+constexpr int kMoreShared = 1 << 30;
+
+// mate[kk] for the L blocks kk = (i, k): the position of block (k, i), with
+// kMoreShared when rows i and k share a column j > k other than i.
+__global__ void k_mates(int nb, const int *__restrict__ rp, const int *__restrict__ ci,
+                        const int *__restrict__ diag, int *__restrict__ mate) {
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < nb; i += gridDim.x * kThreads) {
+    const int end = rp[i + 1];
+    for (int kk = rp[i]; kk < diag[i]; ++kk) {
+      const int k = ci[kk];
+      int p = kk + 1, m = 0;
+      for (int jj = diag[k] + 1; jj < rp[k + 1]; ++jj) {
+        const int j = ci[jj];
+        while (p < end && ci[p] < j) ++p;
+        if (j == i) m |= jj;
+        else if (p < end && ci[p] == j) m |= kMoreShared;
+      }
+      mate[kk] = m;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+k_bilu0_rows(int row_a, int rows_a, int row_b, int rows_b, int color_row0, int color_slice0,
+             const int *__restrict__ rp, const int *__restrict__ ci, const int *__restrict__ diag,
+             const int *__restrict__ mate, double *v, double *dinv, const FactorOut F, int *bad) {
+  const int lane = threadIdx.x & 31, r = lane % 3;
+  const int t = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * 10 + lane / 3;
+  // rows row_a .. and row_b .., of the color that starts at color_row0
+  const bool act = lane < 30 && t < rows_a + rows_b;
+  const int i = !act ? row_a : t < rows_a ? row_a + t : row_b + t - rows_a;
+  double g0 = 0, g1 = 0, g2 = 0;   // row r of the diagonal block
+  if (act) {
+    const int k0 = rp[i], di = diag[i];
+    const double *g = v + (size_t)di * 9 + 3 * r;
+    g0 = g[0]; g1 = g[1]; g2 = g[2];
+    double dk[9], u[9];
+    int m = 0;
+    auto load = [&](int kk) {
+      const double *d = dinv + (size_t)ci[kk] * 9;
+      m = mate[kk];
+      const double *b = v + (size_t)(m & ~kMoreShared) * 9;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) { dk[e] = d[e]; u[e] = b[e]; }
+    };
+    if (k0 < di) load(k0);
+    for (int kk = k0; kk < di; ++kk) {
+      double *a = v + (size_t)kk * 9 + 3 * r;
+      double l[3], s[3];
+      const int mk = m;
+      mul_row_exact(a[0], a[1], a[2], dk, l);
+      mul_row_exact(l[0], l[1], l[2], u, s);
+      if (kk + 1 < di) load(kk + 1);
+      a[0] = l[0]; a[1] = l[1]; a[2] = l[2];
+      store_factor(F, kk, true, r, l[0], l[1], l[2]);
+      g0 = dsub(g0, s[0]); g1 = dsub(g1, s[1]); g2 = dsub(g2, s[2]);
+      if (mk & kMoreShared) {
+        const int k = ci[kk], end = rp[i + 1], ke = rp[k + 1];
+        int p = kk + 1;
+        for (int jj = diag[k] + 1; jj < ke; ++jj) {
+          const int j = ci[jj];
+          while (p < end && ci[p] < j) ++p;
+          if (p == end) break;
+          if (ci[p] != j || j == i) continue;
+          mul_row_exact(l[0], l[1], l[2], v + (size_t)jj * 9, s);
+          double *d = v + (size_t)p * 9 + 3 * r;
+          d[0] = dsub(d[0], s[0]); d[1] = dsub(d[1], s[1]); d[2] = dsub(d[2], s[2]);
+        }
+      }
+    }
+    double *go = v + (size_t)di * 9 + 3 * r;
+    go[0] = g0; go[1] = g1; go[2] = g2;
+    const int end = rp[i + 1];
+    for (int jj = di + 1; jj < end; ++jj) {   // the row's U blocks are final
+      const double *b = v + (size_t)jj * 9 + 3 * r;
+      store_factor(F, jj, false, r, b[0], b[1], b[2]);
+    }
+  }
+  __syncwarp();
+  // the block's other rows from the row's other two threads
+  double a[9];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int from = lane < 30 ? lane - r + q : lane;
+    a[3 * q] = __shfl_sync(0xffffffffu, g0, from);
+    a[3 * q + 1] = __shfl_sync(0xffffffffu, g1, from);
+    a[3 * q + 2] = __shfl_sync(0xffffffffu, g2, from);
+  }
+  if (!act) return;
   const double c00 = dsub(dmul(a[4], a[8]), dmul(a[5], a[7]));
   const double c01 = dsub(dmul(a[5], a[6]), dmul(a[3], a[8]));
   const double c02 = dsub(dmul(a[3], a[7]), dmul(a[4], a[6]));
   const double det = dadd(dadd(dmul(a[0], c00), dmul(a[1], c01)), dmul(a[2], c02));
-  if (det == 0.0 || !isfinite(det)) return false;
-  const double id = __ddiv_rn(1.0, det);
-  o[0] = dmul(c00, id);
-  o[1] = dmul(dsub(dmul(a[2], a[7]), dmul(a[1], a[8])), id);
-  o[2] = dmul(dsub(dmul(a[1], a[5]), dmul(a[2], a[4])), id);
-  o[3] = dmul(c01, id);
-  o[4] = dmul(dsub(dmul(a[0], a[8]), dmul(a[2], a[6])), id);
-  o[5] = dmul(dsub(dmul(a[2], a[3]), dmul(a[0], a[5])), id);
-  o[6] = dmul(c02, id);
-  o[7] = dmul(dsub(dmul(a[1], a[6]), dmul(a[0], a[7])), id);
-  o[8] = dmul(dsub(dmul(a[0], a[4]), dmul(a[1], a[3])), id);
-  return true;
-}
-
-// pv[k] = vals[src[k]] (input order -> color-permuted order), 9 per block
-__global__ void k_permute_blocks(int nnzb, const int *__restrict__ src,
-                                 const double *__restrict__ vals, double *__restrict__ pv) {
-  for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < 9LL * nnzb;
-       i += (long long)gridDim.x * kThreads) {
-    const long long k = i / 9, e = i - 9 * k;
-    pv[i] = vals[(long long)src[k] * 9 + e];
+  double o0 = 0.0, o1 = 0.0, o2 = 0.0;   // row r of the inverse
+  if (det == 0.0 || !isfinite(det)) {
+    if (r == 0) atomicMin(bad, i);
+  } else {
+    const double id = __ddiv_rn(1.0, det);
+    auto pick = [&](int x, int y, int z) { return r == 0 ? a[x] : r == 1 ? a[y] : a[z]; };
+    o0 = dmul(r == 0 ? c00 : r == 1 ? c01 : c02, id);
+    o1 = dmul(dsub(dmul(pick(2, 0, 1), pick(7, 8, 6)), dmul(pick(1, 2, 0), pick(8, 6, 7))), id);
+    o2 = dmul(dsub(dmul(pick(1, 2, 0), pick(5, 3, 4)), dmul(pick(2, 0, 1), pick(4, 5, 3))), id);
   }
-}
-
-// IKJ block ILU(0) of the rows of one color (rows of one color are never
-// coupled, and all earlier colors are final): for each k < i in row i,
-// L_ik = A_ik U_kk^-1, then A_ij -= L_ik U_kj for the j > k present in both
-// rows (a merge of the two sorted column lists); D_i^-1 = inv(A_ii).
-// A singular pivot records the smallest failing row in *bad.
-__global__ void k_bilu0_color(int row0, int nrows, const int *__restrict__ rp,
-                              const int *__restrict__ ci, const int *__restrict__ diag,
-                              double *v, double *dinv, int *bad) {
-  const int t = blockIdx.x * kThreads + threadIdx.x;
-  if (t >= nrows) return;
-  const int i = row0 + t;
-  const int end = rp[i + 1];
-  for (int kk = rp[i]; kk < diag[i]; ++kk) {
-    const int k = ci[kk];
-    double a[9], dk[9], l[9];
+  double *o = dinv + (size_t)i * 9 + 3 * r;
+  o[0] = o0; o[1] = o1; o[2] = o2;
+  const int d = F.drow[i] - color_row0, dl = d & 31;
+  const size_t ds = (size_t)(color_slice0 + (d >> 5));
+  const double oo[3] = {o0, o1, o2};
 #pragma unroll
-    for (int e = 0; e < 9; ++e) { a[e] = v[(size_t)kk * 9 + e]; dk[e] = dinv[(size_t)k * 9 + e]; }
-    mul3_exact(a, dk, l);
-#pragma unroll
-    for (int e = 0; e < 9; ++e) v[(size_t)kk * 9 + e] = l[e];
-    int p = kk + 1;
-    for (int jj = diag[k] + 1; jj < rp[k + 1]; ++jj) {
-      const int j = ci[jj];
-      while (p < end && ci[p] < j) ++p;
-      if (p == end) break;
-      if (ci[p] != j) continue;
-      double u[9], t9[9];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) u[e] = v[(size_t)jj * 9 + e];
-      mul3_exact(l, u, t9);
-#pragma unroll
-      for (int e = 0; e < 9; ++e) v[(size_t)p * 9 + e] = dsub(v[(size_t)p * 9 + e], t9[e]);
-    }
-  }
-  double dgl[9], inv[9];
-#pragma unroll
-  for (int e = 0; e < 9; ++e) dgl[e] = v[(size_t)diag[i] * 9 + e];
-  if (!inv3_exact(dgl, inv)) {
-    atomicMin(bad, i);
-#pragma unroll
-    for (int e = 0; e < 9; ++e) inv[e] = 0.0;
-  }
-#pragma unroll
-  for (int e = 0; e < 9; ++e) dinv[(size_t)i * 9 + e] = inv[e];
-}
-
-// Sliced value array of one matrix from per-block values (9 doubles each),
-// vsrc = source block per slot lane (-1: padding -> 0), optional transpose.
-template <typename V>
-__global__ void k_fill_sliced(long long slots, const int *__restrict__ vsrc, int transpose,
-                              const double *__restrict__ src, V *__restrict__ out) {
-  for (long long q = blockIdx.x * (long long)kThreads + threadIdx.x; q < slots * 32;
-       q += (long long)gridDim.x * kThreads) {
-    const long long slot = q >> 5;
-    const int lane = (int)(q & 31);
-    const int sblk = vsrc[q];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      const int ee = transpose ? (e % 3) * 3 + e / 3 : e;
-      const double x = sblk >= 0 ? src[(size_t)sblk * 9 + ee] : 0.0;
-      out[sl_idx<V>((size_t)slot, e, lane)] = (V)x;
-    }
-  }
-}
-
-// Sliced per-row 3x3 blocks (sl_idx, one slot per slice) from nb*9 doubles in
-// permuted row order (drow: device row -> permuted row).
-template <typename V>
-__global__ void k_fill_diag(int S, const int2 *__restrict__ srows, const int *__restrict__ drow,
-                            int transpose, const double *__restrict__ d, V *__restrict__ out) {
-  for (long long q = blockIdx.x * (long long)kThreads + threadIdx.x; q < (long long)S * 32;
-       q += (long long)gridDim.x * kThreads) {
-    const int s = (int)(q >> 5), lane = (int)(q & 31);
-    const int2 sr = srows[s];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      const int ee = transpose ? (e % 3) * 3 + e / 3 : e;
-      const double x = lane < sr.y ? d[(size_t)drow[sr.x + lane] * 9 + ee] : 0.0;
-      out[sl_idx<V>((size_t)s, e, lane)] = (V)x;
+  for (int c = 0; c < 3; ++c) {
+    F.D[sl_idx<double>(ds, 3 * r + c, dl)] = oo[c];
+    F.Dt[sl_idx<double>(ds, 3 * c + r, dl)] = oo[c];
+    if (F.D32) {
+      F.D32[sl_idx<float>(ds, 3 * r + c, dl)] = (float)oo[c];
+      F.Dt32[sl_idx<float>(ds, 3 * c + r, dl)] = (float)oo[c];
     }
   }
 }
