@@ -107,11 +107,12 @@ struct Handle {
   Vecs<float> v32;
   DevBuf<double> b64, io64, io64b, partials, dA;
   DevBuf<int> x0nz;                        // set when x0 has a nonzero entry
-  // device factorization: permuted values (factored in place), inverses
+  // device factorization: values in input order (factored in place), inverses
   DevBuf<int> pdiag, bad;
   DevBuf<double> pbuf, vals_in, dinvp;
-  // where each input block goes: permuted order, slot lane of A and of A^T
-  DevBuf<int> pblk, apos, tpos;
+  // slot lane of each input block in A and in A^T; the input rows by chunk
+  // (see plan_chunks), in a chunk by color and input order; input row pointers
+  DevBuf<int> apos, tpos, crows, irowptr;
   DevBuf<int> mate, fpos, ftpos, frpos, drow;   // see k_bilu0_rows, FactorOut
   // the input values cross the link in chunks of whole block rows; a color's
   // rows that chunk c completes: run [begin, ready[c]) of each run of colors
@@ -120,7 +121,7 @@ struct Handle {
     int color, row0, rows;
     std::vector<int> ready;
   };
-  std::vector<long long> chunk;            // first block of each chunk, and nnzb
+  std::vector<int> chunk_row, chunk_blk;   // first row, block of each chunk; nb, nnzb
   std::vector<Run> runs;
   cudaEvent_t e_chunk[kMaxChunks] = {};
   bool host_factors_stale = false;
@@ -953,7 +954,7 @@ void release_device(Handle *h) {
       for (auto &sw : prec) sw.release();
   h->pdiag.release(); h->bad.release(); h->pbuf.release(); h->vals_in.release();
   h->dinvp.release();
-  h->pblk.release(); h->apos.release(); h->tpos.release(); h->mate.release();
+  h->crows.release(); h->irowptr.release(); h->apos.release(); h->tpos.release(); h->mate.release();
   h->fpos.release(); h->ftpos.release(); h->frpos.release(); h->drow.release();
   h->srows.release(); h->perm.release(); h->iperm.release();
   h->ibrow.release(); h->icol.release();
@@ -973,22 +974,29 @@ void release_device(Handle *h) {
 // leading rows whose blocks, and whose neighbours', have arrived with chunk
 // c. On a grid in natural order that is all but a few layers of the rows up
 // to the chunk's end; on any pattern the rows that wait longer are done with
-// a later chunk.
-void plan_chunks(Handle *h) {
+// a later chunk. Returns the input rows by chunk, in a chunk by color.
+std::vector<int> plan_chunks(Handle *h) {
   const Analysis &an = h->an;
-  // 32 MB cross the link in 160 us; a chunk's own kernels take about 100
-  const long long per = 32ll << 20;
+  // Chunks of 32 MB (160 us on the link; their own kernels take about 100, and
+  // launching them delays the next copy's staging by 15), or 8 MB where that
+  // gives fewer than six. Factorization of the 500k-cell system with 8, 16,
+  // 24, 32, 64 MB and in one piece: 2.06, 1.60, 1.65, 1.57, 1.73, 2.20 ms; of
+  // 59,000 cells with 8 MB and in one piece: 0.29, 0.35 ms.
+  const long long bytes = (long long)an.nnzb * 72, mb = 1 << 20;
   const int n = (int)std::max<long long>(
-      1, std::min<long long>(kMaxChunks, (long long)an.nnzb * 72 / per));
+      {1, std::min<long long>(bytes / (8 * mb), 6),
+       std::min<long long>(bytes / (32 * mb), kMaxChunks)});
   std::vector<int> row_end(n);             // first input row after each chunk
-  h->chunk.assign(1, 0);
+  h->chunk_row.assign(1, 0);
+  h->chunk_blk.assign(1, 0);
   for (int c = 0; c < n; ++c) {
     const long long want = (long long)an.nnzb * (c + 1) / n;
     const int row = c + 1 == n ? an.nb
                                : (int)(std::lower_bound(an.rowptr.begin(), an.rowptr.end(), want) -
                                        an.rowptr.begin());
     row_end[c] = std::min(row, an.nb);
-    h->chunk.push_back(an.rowptr[row_end[c]]);
+    h->chunk_row.push_back(row_end[c]);
+    h->chunk_blk.push_back(an.rowptr[row_end[c]]);
   }
   h->runs.clear();
   for (int col = 0; col < std::min(2, an.ncolors); ++col)
@@ -1006,6 +1014,12 @@ void plan_chunks(Handle *h) {
       for (; c < n; ++c) run.ready[c] = run.rows;
       h->runs.push_back(std::move(run));
     }
+  // a stable pass over the rows in permuted order, color by color
+  std::vector<int> chunk_of(an.nb), next(h->chunk_row.begin(), h->chunk_row.end() - 1), rows(an.nb);
+  for (int c = 0; c < n; ++c)
+    std::fill(chunk_of.begin() + h->chunk_row[c], chunk_of.begin() + h->chunk_row[c + 1], c);
+  for (int i = 0; i < an.nb; ++i) rows[next[chunk_of[an.perm[i]]]++] = an.perm[i];
+  return rows;
 }
 
 // Allocates the device side for the current analysis (structure only).
@@ -1103,17 +1117,16 @@ int setup_device(Handle *h) {
       CK(cudaMemsetAsync(h->dinv32.p, 0, nd * sizeof(float), h->st));
       CK(cudaMemsetAsync(h->dinvT32.p, 0, nd * sizeof(float), h->st));
     }
-    // where each block goes: pblk, apos, tpos by input block, the others by
-    // permuted block (of a diagonal block: unused)
-    for (DevBuf<int> *b : {&h->pblk, &h->apos, &h->tpos, &h->mate, &h->fpos, &h->ftpos, &h->frpos})
+    // where each block goes: apos, tpos by input block, the others by permuted
+    // block (of a diagonal block: unused)
+    for (DevBuf<int> *b : {&h->apos, &h->tpos, &h->mate, &h->fpos, &h->ftpos, &h->frpos})
       CK(b->alloc(an.nnzb));
     CK(cudaMemsetAsync(h->frpos.p, 0xff, an.nnzb * sizeof(int), h->st));
     CK(h->drow.alloc(an.nb));
     CK(cudaMemcpyAsync(h->drow.p, an.idperm.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice, h->st));
     const int gi = grid_for(h, an.nnzb);
     k_mates<<<grid_for(h, an.nb), kThreads, 0, h->st>>>(an.nb, h->prowptr.p, h->pcol.p, h->pdiag.p,
-                                                        h->mate.p);
-    k_invert<<<gi, kThreads, 0, h->st>>>(an.nnzb, h->psrc.p, h->pblk.p);
+                                                        h->psrc.p, h->mate.p);
     auto positions = [&](DevMat &m, const int *psrc, DevBuf<int> &pos) {
       if (m.slots)
         k_block_positions<<<gi, kThreads, 0, h->st>>>(m.slots * 32, m.vsrc.p, psrc, pos.p);
@@ -1131,8 +1144,12 @@ int setup_device(Handle *h) {
     CK(cudaGetLastError());
     for (DevMat *m : {&h->A, &h->At, &h->L, &h->U, &h->Lt, &h->Ut, &h->Lr, &h->Utr})
       m->vsrc.release();
-    plan_chunks(h);
-    h->device_bytes += (size_t)an.nnzb * 28 + (size_t)an.nb * 4;
+    const std::vector<int> crows = plan_chunks(h);
+    CK(h->crows.alloc(an.nb));
+    CK(cudaMemcpy(h->crows.p, crows.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice));
+    CK(h->irowptr.alloc(an.nb + 1));
+    CK(cudaMemcpy(h->irowptr.p, an.rowptr.data(), (an.nb + 1) * sizeof(int), cudaMemcpyHostToDevice));
+    h->device_bytes += (size_t)an.nnzb * 24 + (size_t)an.nb * 12;
     h->device_bytes += (size_t)an.nnzb * 9 * 16 + (size_t)an.nb * 76;
   }
   for (int red = 0; red < 2; ++red)
@@ -1185,14 +1202,16 @@ void bilu0_rows(Handle *h, const FactorOut &F, int color, int row_a, int rows_a,
   if (rows <= 0) return;
   k_bilu0_rows<<<(rows + kBiluRows - 1) / kBiluRows, kThreads, 0, h->st>>>(
       row_a, rows_a, row_b, rows_b, h->an.color_ptr[color], h->an.slice_color_ptr[color],
-      h->prowptr.p, h->pcol.p, h->pdiag.p, h->mate.p, h->pbuf.p, h->dinvp.p, F, h->bad.p);
+      h->prowptr.p, h->pcol.p, h->pdiag.p, h->psrc.p, h->mate.p, h->pbuf.p,
+      h->dinvp.p, F, h->bad.p);
 }
 
 // Permute, factor and lay out on the device: the values (host array, input
 // order) cross the link in chunks on the auxiliary stream; behind each, its
-// blocks go to the permuted order, A and A^T, and the rows of colors 0 and 1
-// that it completes are factored, into L, U, U^T, L^T and the inverse
-// diagonal blocks; then the other colors. 500k cells: NEW.
+// rows go into A and A^T, and the rows of colors 0 and 1 that it completes are
+// factored, into L, U, U^T, L^T and the inverse
+// diagonal blocks; then the other colors. 500k cells: 2.81 -> 1.57 ms, of
+// which the link alone takes 1.1.
 int factor_device(Handle *h, const double *vals) {
   const Analysis &an = h->an;
   CK(cudaMemsetAsync(h->bad.p, 0x7f, sizeof(int), h->st));
@@ -1201,17 +1220,19 @@ int factor_device(Handle *h, const double *vals) {
   CK(cudaEventRecord(h->e_x, h->st));
   CK(cudaStreamWaitEvent(h->aux, h->e_x, 0));
   const FactorOut F = factor_out(h);
-  const int n = (int)h->chunk.size() - 1;
+  const int n = (int)h->chunk_row.size() - 1;
   for (int c = 0; c < n; ++c) {
-    const long long k0 = h->chunk[c], nk = h->chunk[c + 1] - k0;
-    if (nk > 0) {
-      CK(cudaMemcpyAsync(h->vals_in.p + 9 * k0, vals + 9 * k0, 9 * nk * sizeof(double),
-                         cudaMemcpyHostToDevice, h->aux));
+    const int r0 = h->chunk_row[c], nr = h->chunk_row[c + 1] - r0;
+    const size_t v0 = 9 * (size_t)h->chunk_blk[c];
+    const size_t bytes = (9 * (size_t)h->chunk_blk[c + 1] - v0) * sizeof(double);
+    if (nr > 0) {
+      CK(cudaMemcpyAsync(h->vals_in.p + v0, vals + v0, bytes, cudaMemcpyHostToDevice, h->aux));
       CK(cudaEventRecord(h->e_chunk[c], h->aux));
       CK(cudaStreamWaitEvent(h->st, h->e_chunk[c], 0));
-      k_scatter_blocks<<<entry_grid(h, nk), kEntryThreads, 0, h->st>>>(
-          (int)k0, (int)nk, h->vals_in.p, h->pblk.p, h->apos.p, h->tpos.p, h->pbuf.p, h->A.v64.p, h->At.v64.p,
-          h->with_32 ? h->A.v32.p : nullptr, h->with_32 ? h->At.v32.p : nullptr);
+      CK(cudaMemcpyAsync(h->pbuf.p + v0, h->vals_in.p + v0, bytes, cudaMemcpyDeviceToDevice, h->st));
+      k_scatter_rows<<<std::min((nr + 31) / 32, 8 * h->sm_count), kThreads, 0, h->st>>>(
+          nr, h->crows.p + r0, h->irowptr.p, h->vals_in.p, h->apos.p, h->tpos.p, h->A.v64.p,
+          h->At.v64.p, h->with_32 ? h->A.v32.p : nullptr, h->with_32 ? h->At.v32.p : nullptr);
     }
     for (size_t q = 0; q + 1 < h->runs.size(); q += 2) {   // a color's two runs
       const Handle::Run &a = h->runs[q], &b = h->runs[q + 1];
@@ -1707,7 +1728,9 @@ int gbilu_get_factors(void *handle, double *lu, double *dinv) {
     CK(cudaSetDevice(h->opt.device));
     h->lu.resize((size_t)h->an.nnzb * 9);
     h->dinv.resize((size_t)h->an.nb * 9);
-    CK(cudaMemcpy(h->lu.data(), h->pbuf.p, h->lu.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    std::vector<double> in(h->lu.size());   // input order -> permuted order
+    CK(cudaMemcpy(in.data(), h->pbuf.p, in.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    permute_values(h->an, in.data(), h->lu.data());
     CK(cudaMemcpy(h->dinv.data(), h->dinvp.p, h->dinv.size() * sizeof(double),
                   cudaMemcpyDeviceToHost));
     h->host_factors_stale = false;

@@ -2009,27 +2009,40 @@ __device__ __forceinline__ void mul_row_exact(double a0, double a1, double a2, c
     o[c] = dadd(dadd(dmul(a0, b[c]), dmul(a1, b[3 + c])), dmul(a2, b[6 + c]));
 }
 
-// One chunk of input blocks [k0, k0 + nk), just copied to vals: their values
-// in the color-permuted order (pv, block pblk[k]) and in the sliced A and A^T
-// (slot lane apos[k], tpos[k]). Runs beside the next chunk's copy over the
-// CPU-GPU link, which takes longer, so the scattered 8-byte stores (rows of
-// one color alternate in the input, so neighbouring lanes of a slice meet in
-// L2) cost nothing; the padding of the slices was zeroed when they were made.
-__global__ void __launch_bounds__(kEntryThreads)
-k_scatter_blocks(int k0, int nk, const double *__restrict__ vals, const int *__restrict__ pblk,
-                 const int *__restrict__ apos, const int *__restrict__ tpos,
-                 double *__restrict__ pv, double *__restrict__ a64, double *__restrict__ t64,
-                 float *__restrict__ a32, float *__restrict__ t32) {
-  const int e = threadIdx.x % 9, et = (e % 3) * 3 + e / 3;
-  for (int k = k0 + blockIdx.x * 32 + threadIdx.x / 9; k < k0 + nk; k += gridDim.x * 32) {
-    const double x = __ldcs(vals + 9 * (size_t)k + e);
-    const int pa = apos[k], pt = tpos[k];
-    pv[(size_t)pblk[k] * 9 + e] = x;
-    a64[sl_idx<double>((size_t)(pa >> 5), e, pa & 31)] = x;
-    t64[sl_idx<double>((size_t)(pt >> 5), et, pt & 31)] = x;
-    if (a32) {
-      a32[sl_idx<float>((size_t)(pa >> 5), e, pa & 31)] = (float)x;
-      t32[sl_idx<float>((size_t)(pt >> 5), et, pt & 31)] = (float)x;
+// The block rows rows[0 .. n) (input rows of a chunk that just arrived, those
+// of one color together and in input order) into the sliced A and A^T, block
+// k at slot lanes apos[k], tpos[k]. Lane = row, warp = block of the row: the
+// rows of a warp are neighbours in a slice too, so each of the nine stores of
+// a block is one range of lanes (a thread per entry in input order scattered
+// 8 bytes a store: 98 against 33 us for 38 MB). Runs beside the next chunk's
+// copy over the CPU-GPU link; the padding of the slices was zeroed when they
+// were made.
+__global__ void __launch_bounds__(kThreads)
+k_scatter_rows(int n, const int *__restrict__ rows, const int *__restrict__ rowptr,
+               const double *__restrict__ vals, const int *__restrict__ apos,
+               const int *__restrict__ tpos, double *__restrict__ a64, double *__restrict__ t64,
+               float *__restrict__ a32, float *__restrict__ t32) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int g = blockIdx.x; 32 * g < n; g += gridDim.x) {
+    if (32 * g + lane >= n) continue;
+    const int row = rows[32 * g + lane], end = rowptr[row + 1];
+    for (int k = rowptr[row] + w; k < end; k += kWarps) {
+      const int pa = apos[k], pt = tpos[k];
+      double x[9];
+#pragma unroll
+      for (int e = 0; e < 9; ++e) x[e] = vals[(size_t)k * 9 + e];
+#pragma unroll
+      for (int e = 0; e < 9; ++e) {
+        a64[sl_idx<double>((size_t)(pa >> 5), e, pa & 31)] = x[e];
+        t64[sl_idx<double>((size_t)(pt >> 5), (e % 3) * 3 + e / 3, pt & 31)] = x[e];
+      }
+      if (a32) {
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+          a32[sl_idx<float>((size_t)(pa >> 5), e, pa & 31)] = (float)x[e];
+          t32[sl_idx<float>((size_t)(pt >> 5), (e % 3) * 3 + e / 3, pt & 31)] = (float)x[e];
+        }
+      }
     }
   }
 }
@@ -2043,11 +2056,8 @@ __global__ void k_block_positions(long long n, const int *__restrict__ vsrc,
        q += (long long)gridDim.x * kThreads)
     if (vsrc[q] >= 0) pos[psrc ? psrc[vsrc[q]] : vsrc[q]] = (int)q;
 }
-__global__ void k_invert(int n, const int *__restrict__ src, int *__restrict__ inv) {
-  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) inv[src[i]] = i;
-}
-
-// IKJ block ILU(0) of rows of one color (rows of one color are never
+// IKJ block ILU(0), in place in v (blocks in the input order; rp, ci, diag:
+// the permuted pattern, psrc: permuted -> input block), of rows of one color (rows of one color are never
 // coupled, and the rows of earlier colors that they read are final): for each
 // k < i in row i, L_ik = A_ik U_kk^-1, then A_ij -= L_ik U_kj for the j > k
 // present in both rows (a merge of the two sorted column lists);
@@ -2109,10 +2119,11 @@ __device__ __forceinline__ void store_factor(const FactorOut &F, int b, bool low
 constexpr int kBiluRows = kThreads / 32 * 10;   // rows a CTA: ten a warp
 constexpr int kMoreShared = 1 << 30;
 
-// mate[kk] for the L blocks kk = (i, k): the position of block (k, i), with
+// mate[kk] for the L blocks kk = (i, k): block (k, i) in the input order, with
 // kMoreShared when rows i and k share a column j > k other than i.
 __global__ void k_mates(int nb, const int *__restrict__ rp, const int *__restrict__ ci,
-                        const int *__restrict__ diag, int *__restrict__ mate) {
+                        const int *__restrict__ diag, const int *__restrict__ psrc,
+                        int *__restrict__ mate) {
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < nb; i += gridDim.x * kThreads) {
     const int end = rp[i + 1];
     for (int kk = rp[i]; kk < diag[i]; ++kk) {
@@ -2121,7 +2132,7 @@ __global__ void k_mates(int nb, const int *__restrict__ rp, const int *__restric
       for (int jj = diag[k] + 1; jj < rp[k + 1]; ++jj) {
         const int j = ci[jj];
         while (p < end && ci[p] < j) ++p;
-        if (j == i) m |= jj;
+        if (j == i) m |= psrc[jj];
         else if (p < end && ci[p] == j) m |= kMoreShared;
       }
       mate[kk] = m;
@@ -2132,7 +2143,8 @@ __global__ void k_mates(int nb, const int *__restrict__ rp, const int *__restric
 __global__ void __launch_bounds__(kThreads, 2)
 k_bilu0_rows(int row_a, int rows_a, int row_b, int rows_b, int color_row0, int color_slice0,
              const int *__restrict__ rp, const int *__restrict__ ci, const int *__restrict__ diag,
-             const int *__restrict__ mate, double *v, double *dinv, const FactorOut F, int *bad) {
+             const int *__restrict__ psrc, const int *__restrict__ mate, double *v, double *dinv,
+             const FactorOut F, int *bad) {
   const int lane = threadIdx.x & 31, r = lane % 3;
   const int t = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * 10 + lane / 3;
   // rows row_a .. and row_b .., of the color that starts at color_row0
@@ -2141,20 +2153,21 @@ k_bilu0_rows(int row_a, int rows_a, int row_b, int rows_b, int color_row0, int c
   double g0 = 0, g1 = 0, g2 = 0;   // row r of the diagonal block
   if (act) {
     const int k0 = rp[i], di = diag[i];
-    const double *g = v + (size_t)di * 9 + 3 * r;
+    double *g = v + (size_t)psrc[di] * 9 + 3 * r;
     g0 = g[0]; g1 = g[1]; g2 = g[2];
     double dk[9], u[9];
-    int m = 0;
+    int m = 0, at = 0;
     auto load = [&](int kk) {
       const double *d = dinv + (size_t)ci[kk] * 9;
       m = mate[kk];
+      at = psrc[kk];
       const double *b = v + (size_t)(m & ~kMoreShared) * 9;
 #pragma unroll
       for (int e = 0; e < 9; ++e) { dk[e] = d[e]; u[e] = b[e]; }
     };
     if (k0 < di) load(k0);
     for (int kk = k0; kk < di; ++kk) {
-      double *a = v + (size_t)kk * 9 + 3 * r;
+      double *a = v + (size_t)at * 9 + 3 * r;
       double l[3], s[3];
       const int mk = m;
       mul_row_exact(a[0], a[1], a[2], dk, l);
@@ -2171,17 +2184,16 @@ k_bilu0_rows(int row_a, int rows_a, int row_b, int rows_b, int color_row0, int c
           while (p < end && ci[p] < j) ++p;
           if (p == end) break;
           if (ci[p] != j || j == i) continue;
-          mul_row_exact(l[0], l[1], l[2], v + (size_t)jj * 9, s);
-          double *d = v + (size_t)p * 9 + 3 * r;
+          mul_row_exact(l[0], l[1], l[2], v + (size_t)psrc[jj] * 9, s);
+          double *d = v + (size_t)psrc[p] * 9 + 3 * r;
           d[0] = dsub(d[0], s[0]); d[1] = dsub(d[1], s[1]); d[2] = dsub(d[2], s[2]);
         }
       }
     }
-    double *go = v + (size_t)di * 9 + 3 * r;
-    go[0] = g0; go[1] = g1; go[2] = g2;
+    g[0] = g0; g[1] = g1; g[2] = g2;
     const int end = rp[i + 1];
     for (int jj = di + 1; jj < end; ++jj) {   // the row's U blocks are final
-      const double *b = v + (size_t)jj * 9 + 3 * r;
+      const double *b = v + (size_t)psrc[jj] * 9 + 3 * r;
       store_factor(F, jj, false, r, b[0], b[1], b[2]);
     }
   }
