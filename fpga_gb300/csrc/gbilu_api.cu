@@ -217,6 +217,16 @@ int reduce_grid(const Handle *h, long long work) {
   return (int)std::max<long long>(1, std::min(g, cap));
 }
 
+// k_update_r: 16 bytes a thread and load; CTAs a SM (2: 18.5 us FP64, 12.4 FP32
+// for the 500k-cell system's tail, 3: 18.5, 13.6, 4: 21.3, 13.4).
+#ifndef GBILU_UPDATE_R_CTAS
+#define GBILU_UPDATE_R_CTAS 2
+#endif
+template <typename T> int update_r_grid(const Handle *h, long long n) {
+  const long long g = (n / Pack<T>::N + 2 * kThreads - 1) / (2 * kThreads);
+  return (int)std::max<long long>(1, std::min(g, (long long)h->sm_count * GBILU_UPDATE_R_CTAS));
+}
+
 // ---------------------------------------------------------------------------
 // launch sequences
 // ---------------------------------------------------------------------------
@@ -583,7 +593,7 @@ void enqueue_iteration(Handle *h, cudaStream_t s, const Ops<V, T> &o,
   k_update_s<T><<<gr, kThreads, 0, s>>>(c, n, w.r.p, w.v.p, w.s.p, part);
   apply_prec(h, s, o, w.s.p, w.sh.p, launches);
   spmv<V, T, SPMV_OMEGA>(h, s, o, w.sh.p, w.t.p, w.s.p, launches);
-  k_update_r<T><<<gr, kThreads, 0, s>>>(c, n, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p,
+  k_update_r<T><<<gr, kThreads, 0, s>>>(c, 0, n, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p,
                                         w.r.p, part);
   if (ru64 && sizeof(T) == 4) {
     Vecs<double> &d = h->v64;
@@ -638,9 +648,8 @@ void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned lon
       c, ts, w.r.p, w.v.p, w.s.p, part);
   apply_prec<V, T, true>(h, s, o, w.s.p, w.sh.p, launches, &c->cs);
   spmv<V, T, SPMV_OMEGA>(h, s, o, w.sh.p, w.t.p, w.s.p, launches, nullptr, S0);
-  k_update_r<T><<<reduce_grid(h, nt), kThreads, 0, s>>>(c, nt, w.x.p + n0, w.ph.p + n0,
-                                                        w.sh.p + n0, w.s.p + n0, w.t.p + n0,
-                                                        w.rt.p + n0, w.r.p + n0, part);
+  k_update_r<T><<<update_r_grid<T>(h, nt), kThreads, 0, s>>>(
+      c, n0, n0 + nt, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p, w.r.p, part);
   k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, s>>>(c, tp, w.r.p, w.v.p, w.p.p,
                                                                        w.rt.p, cond);
   launches += 3;
@@ -1533,9 +1542,8 @@ void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, 
       k_tail_s<V, T><<<row_grid(h, tp.rows, GBILU_REDUCE_CTAS_PER_SM), kThreads, 0, h->st>>>(
           c, ts, w.r.p, w.v.p, w.s.p, h->partials.p);
     else if (kind == 7)
-      k_update_r<T><<<reduce_grid(h, nt), kThreads, 0, h->st>>>(
-          c, nt, w.x.p + n0, w.ph.p + n0, w.sh.p + n0, w.s.p + n0, w.t.p + n0, w.rt.p + n0,
-          w.r.p + n0, h->partials.p);
+      k_update_r<T><<<update_r_grid<T>(h, nt), kThreads, 0, h->st>>>(
+          c, n0, n0 + nt, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p, w.r.p, h->partials.p);
     else
       k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, h->st>>>(c, tp, w.r.p, w.v.p, w.p.p,
                                                                        w.rt.p, 0ull);
@@ -1552,7 +1560,7 @@ void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, 
     k_update_s<T><<<gr, kThreads, 0, h->st>>>(h->ctl.p, n, w.r.p, w.v.p, w.s.p, h->partials.p);
     ++l;
   } else if (kind == 7) {
-    k_update_r<T><<<gr, kThreads, 0, h->st>>>(h->ctl.p, n, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p,
+    k_update_r<T><<<gr, kThreads, 0, h->st>>>(h->ctl.p, 0, n, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p,
                                               w.rt.p, w.r.p, h->partials.p);
     ++l;
   } else {

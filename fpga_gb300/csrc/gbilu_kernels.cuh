@@ -165,29 +165,52 @@ __device__ __forceinline__ void df_add_prod(DF &acc, float a, float b) {
 __device__ __forceinline__ double df_value(const DF &a) { return (double)a.hi + (double)a.lo; }
 
 // Deterministic block reduction of NV doubles over a kThreads-thread CTA;
-// result valid in thread 0. GB300's FP64 pipe is 1/64 of FP32, so a shuffle
-// tree in every warp (45 FP64 warp instructions per CTA) costs microseconds:
-// the values go through shared memory instead and warp 0 alone sums them, 8
-// per lane in order and then a 5-level shuffle tree (12 instructions).
+// result valid in thread 0. GB300's FP64 pipe is 1/64 of FP32 and a warp
+// issues one FP64 instruction per 64 cycles, so a shuffle tree in every warp
+// (45 FP64 warp instructions per CTA) costs microseconds: the values go
+// through shared memory, two warps per value add four of them a lane, and one
+// warp per value adds two a lane and finishes with a 5-level shuffle tree.
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV]) {
+  static_assert(NV * 64 <= kThreads, "two warps per value");
   __shared__ double red[NV][kThreads];
+  const int t = threadIdx.x;
 #pragma unroll
-  for (int j = 0; j < NV; ++j) red[j][threadIdx.x] = v[j];
+  for (int j = 0; j < NV; ++j) red[j][t] = v[j];
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      double x = red[j][l];
-#pragma unroll
-      for (int k = 1; k < kWarps; ++k) x += red[j][l + 32 * k];
+  double x = 0.0;
+  if (t < 64 * NV) {
+    const double *q = red[t >> 6] + (t & 63);
+    x = (q[0] + q[64]) + (q[128] + q[192]);
+  }
+  if (NV > 1) {
+    // one warp per value: the values' two halves meet in its first warp
+    __syncthreads();
+    if (t < 64 * NV) red[t >> 6][t & 63] = x;
+    __syncthreads();
+    if (t < 32 * NV) {
+      const double *q = red[t >> 5] + (t & 31);
+      x = q[0] + q[32];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      v[j] = x;
+      if ((t & 31) == 0) red[t >> 5][64] = x;
     }
+    __syncthreads();
+    if (t == 0)
+#pragma unroll
+      for (int j = 0; j < NV; ++j) v[j] = red[j][64];
+    __syncthreads();
+  } else {
+    if (t >= 32 && t < 64) red[0][t] = x;   // read by no other thread before
+    __syncthreads();
+    if (t < 32) {
+      x += red[0][t + 32];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      v[0] = x;
+    }
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 // Writes this CTA's partials and returns true in every thread of the CTA
@@ -375,16 +398,25 @@ __device__ __forceinline__ void finish_s(Ctl *ctl, double ss) {
   else ctl->half = 2 * ctl->k + 1;
 }
 
-// ||r||^2, (r, rt) -> beta and the stop tests after the second half
+// ||r||^2, (r, rt) -> beta and the stop tests after the second half. Called by
+// a whole warp: two of its lanes form the two quotients of beta with one
+// division (an FP64 division or square root is a chain of instructions of 65
+// cycles each; one thread alone took 1.7 us here).
 __device__ __forceinline__ void finish_r(Ctl *ctl, double rr, double rrt, bool timed_out) {
   // the color-0 rows of the reduced iteration: t = s there, so
   // r = (1 - omega) s
-  const double cr = fma(-ctl->omega, ctl->cs, ctl->cs);
+  const int lane = threadIdx.x & 31;
+  const double omega = ctl->omega, cs = ctl->cs, cp = ctl->cp;
+  const double cr = fma(-omega, cs, cs);
+  double rho_new = rrt + head_part(ctl, cr * ctl->crt);
+  const double q = (lane == 1 ? ctl->alpha : rho_new) / (lane == 1 ? omega : ctl->rho);
+  const double nr = sqrt(rr + head_part(ctl, cr * cr));
+  double beta = __shfl_sync(0xffffffffu, q, 0) * __shfl_sync(0xffffffffu, q, 1);
+  if (lane != 0) return;
   ctl->cr = cr;
   ctl->x_moved = 1;
-  const double nr = sqrt(rr + head_part(ctl, cr * cr));
   push_norm(ctl, nr);
-  ctl->dots[3] = rrt + head_part(ctl, cr * ctl->crt);
+  ctl->dots[3] = rho_new;
   if (!finite(nr)) { stop(ctl, ST_NONFINITE, 0); return; }
   if (ctl->ru_mode) {
     // the recursive residual of the FP32 iteration only schedules a
@@ -395,7 +427,6 @@ __device__ __forceinline__ void finish_r(Ctl *ctl, double rr, double rrt, bool t
     stop(ctl, ST_OK, 0);
     return;
   }
-  double rho_new = ctl->dots[3];
   if (ctl->reduced) {
     // A right-hand side on color 0 alone makes (r, rt) zero after one
     // iteration: the head's residual is eliminated exactly and rt has no
@@ -405,16 +436,15 @@ __device__ __forceinline__ void finish_r(Ctl *ctl, double rr, double rrt, bool t
     if (ctl->restart) {
       ctl->crt = cr;
       ctl->rt_norm = nr;
-      ctl->rho = rho_new = nr * nr;
-      ctl->alpha = 0.0;   // beta = 0
+      rho_new = nr * nr;
+      beta = 0.0;
     }
   }
-  const double beta = (rho_new / ctl->rho) * (ctl->alpha / ctl->omega);
   ctl->rho_prev = ctl->rho;
   ctl->rho = rho_new;
   ctl->beta = beta;
-  ctl->cp = fma(beta, fma(-ctl->omega, ctl->cp, ctl->cp), cr);   // v = p there
-  if (ctl->omega == 0.0 || !finite(beta)) { stop(ctl, ST_BREAKDOWN, 0); return; }
+  ctl->cp = fma(beta, fma(-omega, cp, cp), cr);   // v = p there
+  if (omega == 0.0 || !finite(beta)) { stop(ctl, ST_BREAKDOWN, 0); return; }
   if (timed_out) {
     stop(ctl, ST_TIMEOUT, 0);
     return;
@@ -530,8 +560,6 @@ k_spmv(Ctl *ctl, int S0, int S, const int2 *__restrict__ srows, const int *__res
        const int *__restrict__ col, const V *__restrict__ val, const T *__restrict__ x,
        T *__restrict__ y, const T *__restrict__ w, double *partials,
        const int *x_nonzero = nullptr) {
-  if (MODE == SPMV_TRUE && (!ctl->ru || ctl->done)) return;
-  if (MODE != SPMV_PLAIN && MODE != SPMV_RESID && ctl->done) return;
   if (MODE == SPMV_PLAIN && x_nonzero && !*x_nonzero) {
     const int n = 3 * (srows[S - 1].x + srows[S - 1].y);
     for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
@@ -560,7 +588,11 @@ k_spmv(Ctl *ctl, int S0, int S, const int2 *__restrict__ srows, const int *__res
   int s = S0 + blockIdx.x * kWarps + (threadIdx.x >> 5);
   int2 sr_n = make_int2(0, 0);
   int o_n = 0, e_n = 0;
-  if (AHEAD && s < S) { sr_n = srows[s]; o_n = off[s]; e_n = off[s + 1]; }
+  if (s < S) { sr_n = srows[s]; o_n = off[s]; e_n = off[s + 1]; }
+  // the stop flag after the first slice's ranges are on their way: one round
+  // trip to L2 less before the first blocks are asked for
+  if (MODE == SPMV_TRUE && (!ctl->ru || ctl->done)) return;
+  if (MODE != SPMV_PLAIN && MODE != SPMV_RESID && ctl->done) return;
 #if GBILU_SPMV_PREFETCH > 0
   // the first rounds of this warp's slices asked from L2 here (lane k:
   // round k), then the slice GBILU_SPMV_PREFETCH rounds ahead of each
@@ -575,15 +607,10 @@ k_spmv(Ctl *ctl, int S0, int S, const int2 *__restrict__ srows, const int *__res
     const int po = PF && lane == 0 && sp < S ? off[sp] : 0;
     const int pe = PF && lane == 0 && sp < S ? off[sp + 1] : 0;
 #endif
-    int2 sr;
-    int o, wdt;
-    if (AHEAD) {
-      sr = sr_n; o = o_n; wdt = e_n - o_n;
-      if (s + nwarps < S) {
-        sr_n = srows[s + nwarps]; o_n = off[s + nwarps]; e_n = off[s + nwarps + 1];
-      }
-    } else {
-      sr = srows[s]; o = off[s]; wdt = off[s + 1] - o;
+    const int2 sr = sr_n;
+    const int o = o_n, wdt = e_n - o_n;
+    if (AHEAD && s + nwarps < S) {
+      sr_n = srows[s + nwarps]; o_n = off[s + nwarps]; e_n = off[s + nwarps + 1];
     }
     if (lane < sr.y) {
       const int row = sr.x + lane;
@@ -610,6 +637,9 @@ k_spmv(Ctl *ctl, int S0, int S, const int2 *__restrict__ srows, const int *__res
 #if GBILU_SPMV_PREFETCH > 0
     if (PF && lane == 0 && sp < S) prefetch_slice<V>(sp, po, pe - po, col, val, val, false);
 #endif
+    if (!AHEAD && s + nwarps < S) {
+      sr_n = srows[s + nwarps]; o_n = off[s + nwarps]; e_n = off[s + nwarps + 1];
+    }
   }
   if (MODE == SPMV_PLAIN) return;
   if (sizeof(T) == 4) { d1 = df_value(f1); d2 = df_value(f2); }
@@ -1747,43 +1777,89 @@ k_update_s(Ctl *ctl, int n, const T *__restrict__ r, const T *__restrict__ v,
   if (grid_sum<1>(vv, partials, &ctl->counter[3], tot) && threadIdx.x == 0) finish_s(ctl, tot[0]);
 }
 
-// Steps 11-14: x += alpha p^ + omega s^ (both halves' updates in one pass),
-// r = s - omega t, ||r||, rho' = (r, rt), beta = (rho'/rho)(alpha/omega).
+// 16 bytes of a vector
+template <typename T> struct Pack {
+  static constexpr int N = 16 / sizeof(T);
+  T v[N];
+};
+template <typename T> __device__ __forceinline__ Pack<T> load_pack(const T *p) {
+  Pack<T> r;
+  if constexpr (sizeof(T) == 8) {
+    const double2 q = *reinterpret_cast<const double2 *>(p);
+    r.v[0] = q.x; r.v[1] = q.y;
+  } else {
+    const float4 q = *reinterpret_cast<const float4 *>(p);
+    r.v[0] = q.x; r.v[1] = q.y; r.v[2] = q.z; r.v[3] = q.w;
+  }
+  return r;
+}
+template <typename T> __device__ __forceinline__ void store_pack(T *p, const Pack<T> &r) {
+  if constexpr (sizeof(T) == 8)
+    *reinterpret_cast<double2 *>(p) = make_double2(r.v[0], r.v[1]);
+  else
+    *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+}
+
+// Steps 11-14 on entries lo .. n-1: x += alpha p^ + omega s^ (both halves'
+// updates in one pass), r = s - omega t, ||r||, rho' = (r, rt),
+// beta = (rho'/rho)(alpha/omega). The vectors start on 16-byte boundaries
+// (they are allocations of their own); entries lo up to the first such
+// boundary and the last few go one by one. 16-byte loads, two of each vector
+// in flight a thread: a pass of a few microseconds is bound by how many trips
+// to memory a thread makes, not by the bytes (8-byte and 4-byte loads, three
+// trips: FP64 19.6, FP32 14.6 us for the 500k-cell system's tail; now 18.5 and
+// 12.4).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_update_r(Ctl *ctl, int n, T *__restrict__ x, const T *__restrict__ ph,
+k_update_r(Ctl *ctl, int lo, int n, T *__restrict__ x, const T *__restrict__ ph,
            const T *__restrict__ sh, const T *__restrict__ s, const T *__restrict__ t,
            const T *__restrict__ rt, T *__restrict__ r, double *partials) {
   if (ctl->done) return;
   const T alpha = (T)ctl->alpha, omega = (T)ctl->omega;
   double d1 = 0.0, d2 = 0.0;
   DF f1 = {0.f, 0.f}, f2 = {0.f, 0.f};
-  const int stride = gridDim.x * kThreads;
-  // 4 elements per trip: their loads are in flight together
-  for (int i0 = blockIdx.x * kThreads + threadIdx.x; i0 < n; i0 += 4 * stride) {
-    T xv[4], phv[4], shv[4], sv[4], tv[4], rtv[4];
+  auto one = [&](T &xi, T phi, T shi, T si, T ti, T rti) -> T {
+    xi = fma(omega, shi, fma(alpha, phi, xi));
+    const T ri = fma(-omega, ti, si);
+    if (sizeof(T) == 8) { d1 += (double)ri * ri; d2 += (double)ri * rti; }
+    else { df_add_prod(f1, (float)ri, (float)ri); df_add_prod(f2, (float)ri, (float)rti); }
+    return ri;
+  };
+  constexpr int W = Pack<T>::N, U = 2;
+  const int a0 = min((lo + W - 1) / W * W, n), a1 = max(n / W * W, a0);
+  if (blockIdx.x == 0 && threadIdx.x < (a0 - lo) + (n - a1)) {
+    const int q = threadIdx.x, i = q < a0 - lo ? lo + q : a1 + q - (a0 - lo);
+    T xi = x[i];
+    r[i] = one(xi, ph[i], sh[i], s[i], t[i], rt[i]);
+    x[i] = xi;
+  }
+  const int stride = gridDim.x * kThreads * W;
+  for (int i0 = a0 + (blockIdx.x * kThreads + threadIdx.x) * W; i0 < a1; i0 += U * stride) {
+    Pack<T> xv[U], phv[U], shv[U], sv[U], tv[U], rtv[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int i = i0 + u * stride;
-      if (i < n) {
-        xv[u] = x[i]; phv[u] = ph[i]; shv[u] = sh[i]; sv[u] = s[i]; tv[u] = t[i]; rtv[u] = rt[i];
+      if (i < a1) {
+        xv[u] = load_pack(x + i); phv[u] = load_pack(ph + i); shv[u] = load_pack(sh + i);
+        sv[u] = load_pack(s + i); tv[u] = load_pack(t + i); rtv[u] = load_pack(rt + i);
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int i = i0 + u * stride;
-      if (i < n) {
-        x[i] = fma(omega, shv[u], fma(alpha, phv[u], xv[u]));
-        const T ri = fma(-omega, tv[u], sv[u]);
-        r[i] = ri;
-        if (sizeof(T) == 8) { d1 += (double)ri * ri; d2 += (double)ri * rtv[u]; }
-        else { df_add_prod(f1, (float)ri, (float)ri); df_add_prod(f2, (float)ri, (float)rtv[u]); }
+      if (i < a1) {
+        Pack<T> rv;
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+          rv.v[k] = one(xv[u].v[k], phv[u].v[k], shv[u].v[k], sv[u].v[k], tv[u].v[k], rtv[u].v[k]);
+        store_pack(x + i, xv[u]);
+        store_pack(r + i, rv);
       }
     }
   }
   if (sizeof(T) == 4) { d1 = df_value(f1); d2 = df_value(f2); }
   double vv[2] = {d1, d2}, tot[2];
-  if (grid_sum<2>(vv, partials, &ctl->counter[4], tot) && threadIdx.x == 0)
+  if (grid_sum<2>(vv, partials, &ctl->counter[4], tot) && threadIdx.x < 32)
     finish_r(ctl, tot[0], tot[1],
              ctl->timeout_ns && globaltimer() - ctl->t_start > ctl->timeout_ns);
 }
@@ -1980,7 +2056,7 @@ k_dot_check(Ctl *ctl, int n, const float *__restrict__ x, const float *__restric
 // permuted row spread each store over 32 cache lines, a warp per row waited
 // on a chain of dependent loads, a thread per entry of the permuted pattern
 // wrote scattered blocks: 1.44, 0.51 and 0.47 ms for the 2M-cell system; this
-// with a 64-bit division per entry 0.32, without NEW.)
+// with a 64-bit division per entry 0.32.)
 constexpr int kEntryThreads = 9 * 32;   // one thread per entry of 32 blocks
 __global__ void __launch_bounds__(kEntryThreads)
 k_grad_a(int nnzb, const int *__restrict__ brow, const int *__restrict__ col,

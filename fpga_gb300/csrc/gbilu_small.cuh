@@ -518,7 +518,7 @@ template <typename V, typename T> struct SmallSolve {
           v[2] = 1.0;
         partial(v, 6);
         if (!totals<3>(6)) return false;
-        if (threadIdx.x == 0) finish_r(&k, S.tot[0], S.tot[1], S.tot[2] != 0.0);
+        if (threadIdx.x < 32) finish_r(&k, S.tot[0], S.tot[1], S.tot[2] != 0.0);
         __syncthreads();
         if (k.done) return true;
       }
