@@ -675,11 +675,11 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
 // Block rows up to which a solve runs in one launch, FP64 and FP32 (inner
 // solves): above, the CTA's 12 warps are too few to stream what its shared
 // memory does not hold. Measured per iteration, separate kernels / one launch,
-// us: FP64 4,000 rows 59 / 28, 35,000 69 / 36, 81,000 83 / 67, 108,000 88 / 72,
-// 180,000 112 / 130; with fault connections (three colors) 103,000 111 / 88,
-// 171,000 140 / 142; FP32 108,000 99 / 75, 180,000 116 / 118.
+// us: FP64 4,000 rows 55 / 27, 35,000 68 / 34, 108,000 87 / 63, 162,000 108 /
+// 98, 216,000 115 / 153; with fault connections (three colors) 33,000 91 / 49,
+// 154,000 112 / 95, 205,000 149 / 172; FP32 108,000 99 / 75, 180,000 116 / 118.
 #ifndef GBILU_SMALL_ROWS64
-#define GBILU_SMALL_ROWS64 140000
+#define GBILU_SMALL_ROWS64 170000
 #endif
 #ifndef GBILU_SMALL_ROWS32
 #define GBILU_SMALL_ROWS32 140000
@@ -1802,9 +1802,10 @@ int gbilu_fpga_export(void *handle, const double *b, const double *x0, int *vect
 // device from lambda (still in the device vector) and gx (the forward
 // solution, input numbering), inside the timed region, into gdA (input
 // block order; host or device like the other arrays).
+// from_zero: x0 = 0, and x is only written.
 static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, bool transpose,
                       double tol, int maxit, gbilu_result *res, const double *gx = nullptr,
-                      double *gdA = nullptr) {
+                      double *gdA = nullptr, bool from_zero = false) {
   int rc = check_solve_ready(h);
   if (rc) return rc;
   if (!b || !x) return h->fail(GBILU_BAD_INPUT, "b and x must not be NULL");
@@ -1829,7 +1830,8 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
     const double *db = b;
     double *dx = x;
     if (!device_ptrs) {
-      CK(cudaMemcpyAsync(h->io64b.p, x, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
+      if (!from_zero)
+        CK(cudaMemcpyAsync(h->io64b.p, x, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
       CK(cudaMemcpyAsync(h->io64.p, b, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
       db = h->io64.p;
       dx = h->io64b.p;
@@ -1840,6 +1842,7 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
     A.perm = h->perm.p;
     A.b_in = db;
     A.x_io = dx;
+    A.from_zero = from_zero;
     A.tol = tol;
     A.absolute = h->opt.absolute_tol;
     A.maxit = maxit;
@@ -1888,10 +1891,12 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
     // together, measured), so x0 goes first and alone; b follows on the copy
     // engine, which takes no SMs from the SpMV, and is permuted on the device.
     const bool overlap_b = fp64 && !device_ptrs;
-    if (!device_ptrs && !mapped_x)
+    if (!device_ptrs && !mapped_x && !from_zero)
       CK(cudaMemcpyAsync(h->io64b.p, x, n * sizeof(double), cudaMemcpyHostToDevice, h->st));
     CK(cudaMemsetAsync(h->x0nz.p, 0, sizeof(int), h->st));
-    if (mapped_x)   // host side read in order, device side written permuted
+    if (from_zero)
+      CK(cudaMemsetAsync(h->v64.x.p, 0, n * sizeof(double), h->st));
+    else if (mapped_x)   // host side read in order, device side written permuted
       k_scatter<double><<<g, kThreads, 0, h->st>>>(nb, h->iperm.p, dx, h->v64.x.p, h->x0nz.p);
     else
       k_gather<double, double><<<g, kThreads, 0, h->st>>>(nb, h->perm.p, dx, h->v64.x.p, 1.0,
@@ -1982,6 +1987,13 @@ int gbilu_solve(void *handle, const double *b, double *x, double tol, int maxit,
   return solve_impl(h, b, x, false, false, tol, maxit, res);
 }
 
+int gbilu_solve_from_zero(void *handle, const double *b, double *x, double tol, int maxit,
+                          gbilu_result *res) {
+  Handle *h = static_cast<Handle *>(handle);
+  if (!h) return GBILU_BAD_INPUT;
+  return solve_impl(h, b, x, false, false, tol, maxit, res, nullptr, nullptr, true);
+}
+
 int gbilu_solve_device(void *handle, const double *d_b, double *d_x, double tol, int maxit,
                        gbilu_result *res) {
   Handle *h = static_cast<Handle *>(handle);
@@ -2048,8 +2060,7 @@ int gbilu_adjoint(void *handle, const double *g_in, const double *x, double *lam
     CK(h->dA.alloc((size_t)h->an.nnzb * 9));
   }
   // lambda = A^-T g: the transposed solve, x0 = 0, then dL/dA on the device
-  memset(lambda, 0, 3 * (size_t)h->an.nb * sizeof(double));
-  return solve_impl(h, g_in, lambda, false, true, tol, maxit, res, dA ? x : nullptr, dA);
+  return solve_impl(h, g_in, lambda, false, true, tol, maxit, res, dA ? x : nullptr, dA, true);
 }
 
 int gbilu_adjoint_device(void *handle, const double *d_g, const double *d_x, double *d_lambda,
@@ -2060,9 +2071,8 @@ int gbilu_adjoint_device(void *handle, const double *d_g, const double *d_x, dou
     return h->fail(GBILU_BAD_INPUT, "g, x and lambda must not be NULL");
   int rc = check_solve_ready(h);
   if (rc) return rc;
-  CK(cudaSetDevice(h->opt.device));
-  CK(cudaMemsetAsync(d_lambda, 0, 3 * (size_t)h->an.nb * sizeof(double), h->st));
-  return solve_impl(h, d_g, d_lambda, true, true, tol, maxit, res, d_dA ? d_x : nullptr, d_dA);
+  return solve_impl(h, d_g, d_lambda, true, true, tol, maxit, res, d_dA ? d_x : nullptr, d_dA,
+                    true);
 }
 
 int gbilu_get_stats(void *handle, gbilu_stats *s) {

@@ -59,6 +59,7 @@ template <typename V, typename T> struct SmallArgs {
   const int *perm;                // device row -> input row
   const double *b_in;
   double *x_io;
+  bool from_zero;                 // x0 = 0: x_io is only written
   const double *r64;
   double *x64;
   double scale, unscale;          // 1 / ||r64||, ||r64||
@@ -82,12 +83,13 @@ template <typename V, typename T> struct SmallCta {
 // Component c of one row: a -+ sum over its blocks' row c times x (other SMs
 // wrote it in this launch, before a grid barrier, whose acquire makes L1 loads
 // see it). Columns ascend; those from limit on end the row, as padding does.
-// All gathers of a row of up to eight blocks go out together. (Not inlined:
-// its sites would spill each other.)
+// The gathers of B blocks go out together: FP64 3 (an iteration of 108,000
+// cells 63 us; with 2 63, 4 66, 5 72, 8 71), FP32 8 (74; 3 to 6: 75-79). (Not
+// inlined: its sites would spill each other.)
 template <typename V, typename T, bool NEG>
 __device__ __noinline__ T comp_row(const V *sv, const int *sc, int w, int lane, int c, const T *x,
                                    int limit, T a) {
-  constexpr int B = 8;
+  constexpr int B = sizeof(T) == 8 ? 3 : 8;
   for (int k0 = 0; k0 < w; k0 += B) {
     int cc[B];
     T y[B][3];
@@ -388,14 +390,14 @@ template <typename V, typename T> struct SmallSolve {
       each(0, own, [&](int i, bool act, int row) {
         if (!act) return;
         const int e = 3 * row + c, g = 3 * A.perm[row] + c;
-        const double x = A.x_io[g];
+        const double x = A.from_zero ? 0.0 : A.x_io[g];
         A.x[e] = x;
         A.b[e] = A.b_in[g];
         nz |= x != 0.0;
       });
       if (nz) *A.x_nonzero = 1;
-      if (!barrier()) return false;
-      const bool mul = __ldcg(A.x_nonzero) != 0;
+      if (!A.from_zero && !barrier()) return false;
+      const bool mul = !A.from_zero && __ldcg(A.x_nonzero) != 0;
       each(0, own, [&](int i, bool act, int row) {
         if (!act) return;
         const int e = 3 * row + c, s = slice(i), o = A.offA[s];
@@ -563,7 +565,7 @@ template <typename V, typename T> struct SmallSolve {
       });
     }
     if constexpr (sizeof(T) == 8) {
-      if (moved)
+      if (moved || A.from_zero)
         each(0, own, [&](int i, bool act, int row) {
           if (act) A.x_io[3 * A.perm[row] + c] = A.x[3 * row + c];
         });

@@ -104,6 +104,7 @@ def load():
     L.gbilu_factor.argtypes = [VP, F64P]
     L.gbilu_get_factors.argtypes = [VP, VP, VP]
     L.gbilu_solve.argtypes = [VP, VP, VP, C.c_double, C.c_int, C.POINTER(Result)]
+    L.gbilu_solve_from_zero.argtypes = L.gbilu_solve.argtypes
     L.gbilu_solve_device.argtypes = [VP, VP, VP, C.c_double, C.c_int, C.POINTER(Result)]
     L.gbilu_apply_spmv.argtypes = [VP, F64P, F64P, C.c_int]
     L.gbilu_apply_ilu.argtypes = [VP, F64P, F64P, C.c_int]
@@ -241,10 +242,14 @@ class GbIlu:
     # --- compute
     def solve(self, b, x0=None, tol=1e-2, maxit=200):
         b = _f64(b)
-        x = np.zeros(3 * self.nb) if x0 is None else _f64(x0).copy()
         res = Result()
-        self._check(self.L.gbilu_solve(self.h, b.ctypes.data, x.ctypes.data, tol, maxit,
-                                       C.byref(res)))
+        if x0 is None:
+            x = np.empty(3 * self.nb)
+            call = self.L.gbilu_solve_from_zero
+        else:
+            x = _f64(x0).copy()
+            call = self.L.gbilu_solve
+        self._check(call(self.h, b.ctypes.data, x.ctypes.data, tol, maxit, C.byref(res)))
         return x, res
 
     def solve_device(self, b_ptr, x_ptr, tol=1e-2, maxit=200):

@@ -249,6 +249,12 @@ int gbilu_get_factors(void *handle, double *lu, double *dinv);
 int gbilu_solve(void *handle, const double *b, double *x, double tol,
                 int maxit, gbilu_result *res);
 
+/* As gbilu_solve from x0 = 0 (what a simulator's Newton step starts from):
+ * x[3*nb] is only written, so no start vector crosses the link. The same bits
+ * as gbilu_solve with zeros in x. */
+int gbilu_solve_from_zero(void *handle, const double *b, double *x, double tol,
+                          int maxit, gbilu_result *res);
+
 /* As gbilu_solve with DEVICE pointers (original numbering). */
 int gbilu_solve_device(void *handle, const double *d_b, double *d_x,
                        double tol, int maxit, gbilu_result *res);

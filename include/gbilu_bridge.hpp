@@ -14,7 +14,7 @@
 //       pattern changed (a new well, a changed grid), gbilu_factor always
 //       (new values every Newton step): the coloring, permutation and device
 //       layout survive across solves on one pattern;
-//   solve(b, res) / get_result(x)            -> gbilu_solve from x0 = 0;
+//   solve(b, res) / get_result(x)            -> gbilu_solve_from_zero;
 //   solve_system(...)                        -> both, with the status
 //       classes a backend reports (analysis failed, preconditioner failed,
 //       other failure) and a result record with the fields of Dune's
@@ -108,10 +108,9 @@ class BsrBridge {
       if (ok_) err_ = "solve before update_matrix";
       return SolverStatus::UnknownError;
     }
-    std::fill(x_.begin(), x_.end(), 0.0);
     gbilu_result r;
     const auto t0 = std::chrono::steady_clock::now();
-    const int rc = gbilu_solve(h_, b, x_.data(), tol_, maxit_, &r);
+    const int rc = gbilu_solve_from_zero(h_, b, x_.data(), tol_, maxit_, &r);
     res.elapsed = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (rc != GBILU_OK) {
       err_ = gbilu_last_error(h_);

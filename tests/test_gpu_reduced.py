@@ -89,3 +89,21 @@ def test_stops_leave_the_iterate(case, maxit):
     if r_ref.status == 1:
         assert r.status == 1 and r.half_iters == r_ref.half_iters
     assert np.linalg.norm(x - x_ref) <= 1e-10 * np.linalg.norm(x_ref)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_from_zero_is_the_solve_from_zeros(case, precision):
+    """Without a start vector x is only written: the same bits as from an
+    array of zeros, and zeros where no iteration ran, whatever x held."""
+    s, A = case
+    with GbIlu(device=0, precision=precision) as g:
+        g.analyze(s.rowptr, s.colind).factor(s.vals)
+        x1, r1 = g.solve(s.b, tol=1e-6, maxit=500)
+        x2, r2 = g.solve(s.b, x0=np.zeros(s.n), tol=1e-6, maxit=500)
+        assert r1.half_iters == r2.half_iters and np.array_equal(x1, x2)
+        x, r = g.solve(np.zeros(s.n), tol=1e-6, maxit=500)
+        assert r.status == 2 and not x.any()
+        b = s.b.copy()
+        b[3] = np.inf
+        x, r = g.solve(b, tol=1e-6, maxit=500)
+        assert r.status == 4 and not x.any()
