@@ -49,17 +49,17 @@ struct DevMat {
 // the work vectors of one BiCGSTAB run
 template <typename T> struct Vecs {
   DevBuf<T> x, r, rt, p, ph, v, s, sh, t;
-  DevBuf<T> y;               // first sweep of a preconditioner apply
+  DevBuf<T> y, ysh;          // first sweep of a preconditioner apply (of s)
   DevBuf<T> base;            // reduced iteration (gbilu_reduced.cuh)
   cudaError_t alloc(size_t n) {
-    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y, &base}) {
+    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y, &ysh, &base}) {
       cudaError_t e = b->alloc(n);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
   }
   void release() {
-    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y, &base}) b->release();
+    for (DevBuf<T> *b : {&x, &r, &rt, &p, &ph, &v, &s, &sh, &t, &y, &ysh, &base}) b->release();
   }
 };
 
@@ -336,9 +336,11 @@ int coop_grid(Handle *h) {
   int per_sm = 0, per_sm_red = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilu_coop<V, T, false>,
                                                 coop_threads<T>(), 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_red, k_ilu_coop<V, T, true>,
-                                                coop_threads<T>(), 0);
-  per_sm = std::min(per_sm, per_sm_red);
+  if constexpr (sizeof(T) == 4) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_red, k_ilu_coop<V, T, true>,
+                                                  coop_threads<T>(), 0);
+    per_sm = std::min(per_sm, per_sm_red);
+  }
   long long most = 0;
   for (int c = 0; c < h->an.ncolors; ++c) {
     const long long rows = h->an.color_ptr[c + 1] - h->an.color_ptr[c];
@@ -539,20 +541,24 @@ cudaError_t launch_coop(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *
 }
 
 // hat = M^-1 src (forward) or M^-T src (transpose); the vector set's y holds
-// the first sweep's result. RED: what the reduced iteration leaves of it,
-// with coef = &Ctl::cp (src = p) or &Ctl::cs (src = s); with two colors that
-// is one step, launched by itself.
+// the first sweep's result. RED: what the reduced iteration leaves of it, with
+// coef = &Ctl::cp (src = p) or &Ctl::cs (src = s): in FP32 one launch as well;
+// with two colors, or behind k_tail_flow (head_only), the last step alone.
 template <typename V, typename T, bool RED = false>
 void apply_prec(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *hat,
-                int &launches, const double *coef = nullptr) {
-  const int C = h->an.ncolors;
-  if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 && !(RED && C == 2)) {
-    const cudaError_t e = launch_coop<V, T, RED>(h, s, o, src, hat, 0, coef);
-    if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
-    ++launches;
-    return;
+                int &launches, const double *coef = nullptr, bool head_only = false) {
+  if constexpr (!RED || sizeof(T) == 4) {
+    const int C = h->an.ncolors;
+    if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 && !(RED && C == 2)) {
+      const cudaError_t e = launch_coop<V, T, RED>(h, s, o, src, hat, 0, coef);
+      if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
+      ++launches;
+      return;
+    }
   }
-  for (const Phase &P : h->sweep[RED][sizeof(T) == 4 ? 1 : 0][o.transpose ? 1 : 0].steps) {
+  const std::vector<Phase> &steps = h->sweep[RED][sizeof(T) == 4 ? 1 : 0][o.transpose ? 1 : 0].steps;
+  for (size_t q = head_only ? steps.size() - 1 : 0; q < steps.size(); ++q) {
+    const Phase &P = steps[q];
     k_phase<V, T, RED><<<(unsigned)((P.nrows + kThreads - 1) / kThreads), kThreads, 0, s>>>(
         h->ctl.p, P, P.mat ? o.off2 : RED ? o.off1r : o.off1,
         P.mat ? o.col2 : RED ? o.col1r : o.col1, P.mat ? o.val2 : RED ? o.val1r : o.val1, o.dmat,
@@ -594,7 +600,7 @@ void enqueue_iteration(Handle *h, cudaStream_t s, const Ops<V, T> &o,
   apply_prec(h, s, o, w.s.p, w.sh.p, launches);
   spmv<V, T, SPMV_OMEGA>(h, s, o, w.sh.p, w.t.p, w.s.p, launches);
   k_update_r<T><<<gr, kThreads, 0, s>>>(c, 0, n, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p,
-                                        w.r.p, part);
+                                        w.r.p, part, 0, n, w.y.p, w.ysh.p);
   if (ru64 && sizeof(T) == 4) {
     Vecs<double> &d = h->v64;
     k_ru_accumulate<<<g, kThreads, 0, s>>>(c, n, (float *)w.x.p, d.x.p, 0);
@@ -611,7 +617,8 @@ void enqueue_iteration(Handle *h, cudaStream_t s, const Ops<V, T> &o,
 // residual is not a multiple of the initial one on the head.
 bool reduced_run(const Handle *h, bool ru) { return h->an.ncolors > 1 && !ru; }
 
-template <typename V, typename T> Tail<V, T> make_tail(const Handle *h, const Ops<V, T> &o, T *hat) {
+template <typename V, typename T>
+Tail<V, T> make_tail(const Handle *h, const Ops<V, T> &o, T *hat, T *y = nullptr) {
   const Analysis &an = h->an;
   Tail<V, T> P;
   P.row0 = an.color_ptr[1];
@@ -622,7 +629,7 @@ template <typename V, typename T> Tail<V, T> make_tail(const Handle *h, const Op
   P.d_first = o.transpose;
   P.dmat = o.dmat;
   P.base = o.vec->base.p;
-  P.ybuf = o.vec->y.p;
+  P.ybuf = y ? y : o.vec->y.p;
   P.hat = hat;
   return P;
 }
@@ -632,8 +639,45 @@ int row_grid(const Handle *h, int rows, int ctas_per_sm) {
   return std::max(1, std::min((rows + kThreads - 1) / kThreads, h->sm_count * ctas_per_sm));
 }
 
+// Whether the small steps run beside the vector kernels (k_tail_flow): FP64,
+// three and more colors, few enough for the step list.
+template <typename T> bool flow_run(const Handle *h, bool transpose) {
+  return sizeof(T) == 8 && h->an.ncolors > 2 && h->sweep[1][0][transpose].phases.n > 0;
+}
+
+template <typename V, typename T, int MODE>
+void tail_flow(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned long long cond,
+               int &launches) {
+  const int f = sizeof(T) == 4, t = o.transpose;
+  const PhaseList &pl = h->sweep[1][f][t].phases;
+  Vecs<T> &w = *o.vec;
+  long long slices = 0;
+  for (int q = 0; q + 1 < pl.n; ++q) slices += (pl.p[q].nrows + kSliceRows - 1) / kSliceRows;
+  // one group of three warps for about two slices
+  const long long share = 2ll * h->sm_count;
+  const Flow<V, T> F{o.off1r, o.col1r, o.val1r, o.off2, o.col2, o.val2, w.sh.p, w.ysh.p,
+                     (int)std::max<long long>(1, std::min<long long>(kFlowGroups, (slices + share - 1) / share))};
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.gridDim = dim3(h->sm_count);
+  cfg.blockDim = dim3(kFlowThreads);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const Tail<V, T> P =
+      MODE == 1 ? make_tail(h, o, w.sh.p, w.ysh.p) : make_tail(h, o, w.ph.p, w.y.p);
+  const cudaError_t e = cudaLaunchKernelEx(
+      &cfg, k_tail_flow<V, T, MODE>, h->ctl.p, P, F, pl, (const T *)w.r.p, (const T *)w.v.p,
+      MODE == 1 ? w.s.p : w.p.p, w.rt.p, h->partials.p, cond);
+  if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
+  ++launches;
+}
+
 // One iteration of the reduced form (gbilu_reduced.cuh): the first sweep of
-// p on color 1 was done by the kernel before the loop body.
+// p on color 1 (and its small steps) was done by the kernel before the loop
+// body.
 template <typename V, typename T>
 void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned long long cond,
                      int &launches) {
@@ -642,17 +686,29 @@ void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned lon
   double *part = h->partials.p;
   const Tail<V, T> tp = make_tail(h, o, w.ph.p), ts = make_tail(h, o, w.sh.p);
   const int S0 = tp.slice1, n0 = 3 * tp.row0, nt = 3 * tp.rows;
-  apply_prec<V, T, true>(h, s, o, w.p.p, w.ph.p, launches, &c->cp);
+  const bool flow = flow_run<T>(h, o.transpose);
+  apply_prec<V, T, true>(h, s, o, w.p.p, w.ph.p, launches, &c->cp, flow);
   spmv<V, T, SPMV_ALPHA>(h, s, o, w.ph.p, w.v.p, w.rt.p, launches, nullptr, S0);
-  k_tail_s<V, T><<<row_grid(h, tp.rows, GBILU_REDUCE_CTAS_PER_SM), kThreads, 0, s>>>(
-      c, ts, w.r.p, w.v.p, w.s.p, part);
-  apply_prec<V, T, true>(h, s, o, w.s.p, w.sh.p, launches, &c->cs);
+  if (flow) {
+    tail_flow<V, T, 1>(h, s, o, 0ull, launches);
+  } else {
+    k_tail_s<V, T><<<row_grid(h, tp.rows, GBILU_REDUCE_CTAS_PER_SM), kThreads, 0, s>>>(
+        c, ts, w.r.p, w.v.p, w.s.p, part);
+    ++launches;
+  }
+  apply_prec<V, T, true>(h, s, o, w.s.p, w.sh.p, launches, &c->cs, flow);
   spmv<V, T, SPMV_OMEGA>(h, s, o, w.sh.p, w.t.p, w.s.p, launches, nullptr, S0);
   k_update_r<T><<<update_r_grid<T>(h, nt), kThreads, 0, s>>>(
-      c, n0, n0 + nt, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p, w.r.p, part);
-  k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, s>>>(c, tp, w.r.p, w.v.p, w.p.p,
+      c, n0, n0 + nt, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p, w.r.p, part,
+      flow ? n0 + 3 * tp.split1 : n0, flow ? n0 + 3 * tp.rows1 : n0 + nt, w.y.p, w.ysh.p);
+  ++launches;
+  if (flow) {
+    tail_flow<V, T, 2>(h, s, o, cond, launches);
+  } else {
+    k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, s>>>(c, tp, w.r.p, w.v.p, w.p.p,
                                                                        w.rt.p, cond);
-  launches += 3;
+    ++launches;
+  }
 }
 
 // The reduced form's start, after the initial residual (base holds the
@@ -660,6 +716,7 @@ void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned lon
 template <typename V, typename T>
 void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
   const Tail<V, T> tp = make_tail(h, o, o.vec->ph.p);
+  const bool flow = flow_run<T>(h, o.transpose);
   if (o.transpose) {
     k_base_head<V, T><<<(tp.row0 + kThreads - 1) / kThreads, kThreads, 0, h->st>>>(
         h->ctl.p, tp.row0, o.dmat, o.vec->base.p);
@@ -668,8 +725,13 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
   const int S = h->an.S;
   k_base_tail<V, T><<<std::min((S - tp.slice1 + kWarps - 1) / kWarps, 8 * h->sm_count), kThreads, 0,
                       h->st>>>(h->ctl.p, tp, S, h->srows.p, o.off1, o.col1, o.val1, o.vec->p.p,
-                               o.vec->base.p);
+                               o.vec->base.p, flow ? o.vec->sh.p : nullptr, o.vec->ysh.p);
   ++launches;
+  if (flow) {
+    int l = 0;
+    tail_flow<V, T, 0>(h, h->st, o, 0ull, l);
+    launches += l;
+  }
 }
 
 // Block rows up to which a solve runs in one launch, FP64 and FP32 (inner
@@ -1175,8 +1237,6 @@ int setup_device(Handle *h) {
     for (int t = 0; t < 2; ++t) {
       int rc = build_stage_plan<double, double, false>(h, 0, t, h->coop_grid64);
       if (rc) return rc;
-      rc = build_stage_plan<double, double, true>(h, 0, t, h->coop_grid64);
-      if (rc) return rc;
       if (h->with_32) {
         rc = build_stage_plan<float, float, false>(h, 1, t, h->coop_grid32);
         if (rc) return rc;
@@ -1191,7 +1251,7 @@ int setup_device(Handle *h) {
   } else if (int rc = plan_small<double, double>(h, GBILU_SMALL_ROWS64)) {
     return rc;
   }
-  h->device_bytes += nd * 16 + (h->with_32 ? nd * 8 : 0) + n * 8 * 14 + (h->with_32 ? n * 4 * 11 : 0) +
+  h->device_bytes += nd * 16 + (h->with_32 ? nd * 8 : 0) + n * 8 * 15 + (h->with_32 ? n * 4 * 12 : 0) +
                      (size_t)an.nnzb * 16 + (size_t)an.nb * 16;
   return GBILU_OK;
 }
@@ -1526,8 +1586,17 @@ void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, 
     const Tail<V, T> tp = make_tail(h, o, w.ph.p), ts = make_tail(h, o, w.sh.p);
     const int S0 = tp.slice1, n0 = 3 * tp.row0, nt = 3 * tp.rows;
     Ctl *c = h->ctl.p;
+    const bool flow = flow_run<T>(h, o.transpose);
     if (kind == 3) {
-      apply_prec<V, T, true>(h, h->st, o, w.p.p, w.ph.p, l, &c->cp);
+      apply_prec<V, T, true>(h, h->st, o, w.p.p, w.ph.p, l, &c->cp, flow);
+      return;
+    }
+    if (flow && kind == 6) {
+      tail_flow<V, T, 1>(h, h->st, o, 0ull, l);
+      return;
+    }
+    if (flow && kind == 8) {
+      tail_flow<V, T, 2>(h, h->st, o, 0ull, l);
       return;
     }
     if (kind == 4) {
@@ -1543,7 +1612,8 @@ void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, 
           c, ts, w.r.p, w.v.p, w.s.p, h->partials.p);
     else if (kind == 7)
       k_update_r<T><<<update_r_grid<T>(h, nt), kThreads, 0, h->st>>>(
-          c, n0, n0 + nt, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p, w.r.p, h->partials.p);
+          c, n0, n0 + nt, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p, w.rt.p, w.r.p, h->partials.p, n0,
+          n0 + nt, w.y.p, w.ysh.p);
     else
       k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, h->st>>>(c, tp, w.r.p, w.v.p, w.p.p,
                                                                        w.rt.p, 0ull);
@@ -1561,7 +1631,7 @@ void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, 
     ++l;
   } else if (kind == 7) {
     k_update_r<T><<<gr, kThreads, 0, h->st>>>(h->ctl.p, 0, n, w.x.p, w.ph.p, w.sh.p, w.s.p, w.t.p,
-                                              w.rt.p, w.r.p, h->partials.p);
+                                              w.rt.p, w.r.p, h->partials.p, 0, n, w.y.p, w.ysh.p);
     ++l;
   } else {
     k_update_p<T><<<g, kThreads, 0, h->st>>>(h->ctl.p, n, w.r.p, w.v.p, w.p.p, 0ull);

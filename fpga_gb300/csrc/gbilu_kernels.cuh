@@ -1103,19 +1103,18 @@ __device__ __forceinline__ void staged_row(const Phase &P, int row, int lane, in
 // Component c of one staged row: own_c - sum_k B_k[c,:] y_k with the FMA
 // sequence of that component in staged_row, so a row whose three components
 // are computed by three warps gets the same bits.
-template <typename V, typename T, bool RED>
+template <typename V, typename T>
 __device__ __forceinline__ T staged_comp(const Phase &P, int c, int row, int lane, int w,
                                          const V *sv, const int *sc, const T *src, const T *ybuf,
-                                         const T *hat, Ctl *ctl, const T *__restrict__ base, T coef) {
+                                         const T *hat, Ctl *ctl) {
   constexpr int SB = sizeof(T) == 8 ? 4 : 8;
-  const T *own = P.own_y ? ybuf : RED && P.own_base == 1 ? base : src;
+  const T *own = P.own_y ? ybuf : src;
   const T *nbr = P.nbr_hat ? hat : ybuf;
   T a;
   unsigned int spins = 0;
   do {   // (src is never checked: see staged_row)
     a = ld_relaxed(own + 3 * row + c);
   } while (P.own_y && is_sentinel(a) && poll_again(ctl, spins));
-  if (RED && P.own_base) a = P.own_base == 1 ? a * coef : fma(coef, base[3 * row + c], a);
   for (int k0 = 0; k0 < w; k0 += SB) {
     int cc[SB];
     T y[SB][3];
@@ -1340,7 +1339,7 @@ __device__ __forceinline__ void ring_row(const Phase &P, int row, int lane, int 
 // ring (sp.ring_ns > 0) the last warp becomes the producer of the large
 // steps' slices and the other warps compute, synchronising among
 // themselves on a named barrier.
-// RED: the steps of the reduced iteration (base, coef: see k_tail_s). The
+// RED (FP32): the steps of the reduced iteration (base, coef: see k_tail_s). The
 // sentinels of its staged rows were written by the kernel before, so its
 // first steps start at once.
 template <typename V, typename T, bool RED>
@@ -1498,8 +1497,7 @@ k_ilu_coop(Ctl *ctl, PhaseList ph, StagePlan sp, const int *__restrict__ off1,
             sd = reinterpret_cast<const V *>(stage_smem + E.pos + E.w * 9 * 32 * sizeof(V) +
                                              E.w * 32 * sizeof(int));
             if (valid)
-              a = staged_comp<V, T, RED>(P, c, row, lane, E.w, sv, sc, src, ybuf, hat, ctl, base,
-                                         coef);
+              a = staged_comp<V, T>(P, c, row, lane, E.w, sv, sc, src, ybuf, hat, ctl);
           }
           if (!act) continue;   // the whole group (same e) skips the round
           // the D products need all three components: the group's warps
@@ -1808,17 +1806,23 @@ template <typename T> __device__ __forceinline__ void store_pack(T *p, const Pac
 // in flight a thread: a pass of a few microseconds is bound by how many trips
 // to memory a thread makes, not by the bytes (8-byte and 4-byte loads, three
 // trips: FP64 19.6, FP32 14.6 us for the 500k-cell system's tail; now 18.5 and
-// 12.4).
+// 12.4). Entries below split and from later on are those that the small
+// steps of the next applies write or wait for (k_tail_flow): p^, s^ and their
+// y become sentinels there (split = lo, later = n: none).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_update_r(Ctl *ctl, int lo, int n, T *__restrict__ x, const T *__restrict__ ph,
-           const T *__restrict__ sh, const T *__restrict__ s, const T *__restrict__ t,
-           const T *__restrict__ rt, T *__restrict__ r, double *partials) {
+k_update_r(Ctl *ctl, int lo, int n, T *__restrict__ x, T *ph, T *sh, const T *__restrict__ s,
+           const T *__restrict__ t, const T *__restrict__ rt, T *__restrict__ r, double *partials,
+           int split, int later, T *yp, T *ysh) {
   if (ctl->done) return;
   const T alpha = (T)ctl->alpha, omega = (T)ctl->omega;
   double d1 = 0.0, d2 = 0.0;
   DF f1 = {0.f, 0.f}, f2 = {0.f, 0.f};
-  auto one = [&](T &xi, T phi, T shi, T si, T ti, T rti) -> T {
+  auto one = [&](int i, T &xi, T phi, T shi, T si, T ti, T rti) -> T {
+    if (i < split || i >= later) {
+      const T sent = sentinel_value<T>();
+      ph[i] = sent; sh[i] = sent; yp[i] = sent; ysh[i] = sent;
+    }
     xi = fma(omega, shi, fma(alpha, phi, xi));
     const T ri = fma(-omega, ti, si);
     if (sizeof(T) == 8) { d1 += (double)ri * ri; d2 += (double)ri * rti; }
@@ -1830,7 +1834,7 @@ k_update_r(Ctl *ctl, int lo, int n, T *__restrict__ x, const T *__restrict__ ph,
   if (blockIdx.x == 0 && threadIdx.x < (a0 - lo) + (n - a1)) {
     const int q = threadIdx.x, i = q < a0 - lo ? lo + q : a1 + q - (a0 - lo);
     T xi = x[i];
-    r[i] = one(xi, ph[i], sh[i], s[i], t[i], rt[i]);
+    r[i] = one(i, xi, ph[i], sh[i], s[i], t[i], rt[i]);
     x[i] = xi;
   }
   const int stride = gridDim.x * kThreads * W;
@@ -1851,7 +1855,7 @@ k_update_r(Ctl *ctl, int lo, int n, T *__restrict__ x, const T *__restrict__ ph,
         Pack<T> rv;
 #pragma unroll
         for (int k = 0; k < W; ++k)
-          rv.v[k] = one(xv[u].v[k], phv[u].v[k], shv[u].v[k], sv[u].v[k], tv[u].v[k], rtv[u].v[k]);
+          rv.v[k] = one(i + k, xv[u].v[k], phv[u].v[k], shv[u].v[k], sv[u].v[k], tv[u].v[k], rtv[u].v[k]);
         store_pack(x + i, xv[u]);
         store_pack(r + i, rv);
       }

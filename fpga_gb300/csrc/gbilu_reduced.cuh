@@ -99,7 +99,7 @@ template <typename V, typename T>
 __global__ void __launch_bounds__(kThreads)
 k_base_tail(const Ctl *ctl, Tail<V, T> P, int S, const int2 *__restrict__ srows,
             const int *__restrict__ off, const int *__restrict__ col, const V *__restrict__ val,
-            const T *__restrict__ p, T *base) {
+            const T *__restrict__ p, T *base, T *sh, T *ysh) {
   if (ctl->done) return;
   const int lane = threadIdx.x & 31;
   for (int s = P.slice1 + blockIdx.x * kWarps + (threadIdx.x >> 5); s < S; s += gridDim.x * kWarps) {
@@ -121,6 +121,12 @@ k_base_tail(const Ctl *ctl, Tail<V, T> P, int S, const int2 *__restrict__ srows,
     }
     base[3 * row] = a0; base[3 * row + 1] = a1; base[3 * row + 2] = a2;
     tail_first(P, row - P.row0, (T)1, a0, a1, a2, p[3 * row], p[3 * row + 1], p[3 * row + 2]);
+    // what the small steps of the first s write or wait for (k_tail_flow)
+    const int t = row - P.row0;
+    if (sh && (t < P.split1 || t >= P.rows1)) {
+      const T sent = sentinel_value<T>();
+      for (int e = 0; e < 3; ++e) { sh[3 * row + e] = sent; ysh[3 * row + e] = sent; }
+    }
   }
 }
 
@@ -187,6 +193,218 @@ k_tail_p(Ctl *ctl, Tail<V, T> P, const T *__restrict__ r, const T *__restrict__ 
     if (restart) { rt[i] = r0; rt[i + 1] = r1; rt[i + 2] = r2; }
     p[i] = p0; p[i + 1] = p1; p[i + 2] = p2;
     tail_first(P, t, cp, b0, b1, b2, p0, p1, p2);
+  }
+}
+
+// --------------------------------------------------------------------------
+// the vector kernels with the small steps beside them (FP64, three and more
+// colors)
+// --------------------------------------------------------------------------
+
+// What a tail kernel needs to run the small steps too.
+template <typename V, typename T> struct Flow {
+  const int *off1r, *col1r; const V *val1r;   // first sweep, the tail's columns
+  const int *off2, *col2; const V *val2;      // second sweep
+  T *sh, *ysh;            // s^ and the small steps' y of s (Tail: p's or s's)
+  int groups;             // groups of three warps on the small steps
+};
+constexpr int kFlowThreads = 512;
+constexpr int kFlowWarps = kFlowThreads / 32;
+constexpr int kFlowGroups = 4;     // at most: the other warps form p or s
+
+// Component c of a row: a - its blocks' row c times x, once every value is
+// there (sentinels in x are waited for; *late: the wait ran out).
+template <typename V, typename T>
+__device__ __forceinline__ T flow_row(const V *__restrict__ sv, const int *__restrict__ sc, int w,
+                                      int lane, int c, const T *x, T a, Ctl *ctl) {
+  constexpr int B = 2;   // (4: 2 % slower)
+  for (int k0 = 0; k0 < w; k0 += B) {
+    int cc[B];
+    T y[B][3];
+    V b[B][3];
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      cc[j] = k0 + j < w ? sc[(k0 + j) * 32 + lane] : -1;
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        if (k0 + j < w) b[j][e] = sv[(size_t)(k0 + j) * 288 + sl_idx<V>(0, 3 * c + e, lane)];
+    }
+    unsigned int spins = 0;
+    bool wait;
+    do {
+      const T *miss = nullptr;
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+        if (cc[j] >= 0) {
+          const T *xs = x + 3 * cc[j];
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            y[j][e] = ld_relaxed(xs + e);
+            if (is_sentinel(y[j][e])) miss = xs + e;
+          }
+        }
+      wait = miss != nullptr;
+      // one missing value is watched, then all are loaded again (watching all
+      // of them crowds out the stores that they wait for)
+      while (wait && is_sentinel(ld_relaxed(miss))) wait = poll_again(ctl, spins);
+    } while (wait);
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+      if (cc[j] >= 0)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) a = fma(-(T)b[j][e], y[j][e], a);
+  }
+  return a;
+}
+
+// k_tail_s and k_tail_p (MODE 1, 2; 0: p is there, the small steps alone) for
+// three and more colors: while most warps form s or p and color 1's first
+// sweep, a few run the small colors' steps of the next apply, ordered by
+// their data: their results (hat of color 1's split rows and of the later
+// colors) and y were preset to the sentinel by k_update_r, split rows come
+// first among color 1's, and a consumer loads again until a value is there.
+// A step reads only rows of earlier steps and of warps that wait for nothing,
+// every group takes its slices in step order, and the launch is cooperative:
+// every wait ends. (In the apply's launch, before the head's step and a grid
+// barrier, the small steps of a 500k-cell system with five colors kept the GPU
+// waiting for 17 us an apply in FP64, and FP64's few warps cannot hide them
+// there.) Measured, vector kernel + apply with 475,000 rows: s 16.4 + 52.5 ->
+// 24.6 + 34.4 us, p 12.3 + 52.5 -> 20.7 + 34.4; an iteration 238 -> 219, with
+// 209,000 rows 149 -> 126. In FP32 the small steps cost 6 us, and a cooperative
+// vector kernel with fewer warps takes more than that (11.6 + 24.8 against 20.5
+// + 18.0): there they stay in the apply's launch (k_ilu_coop).
+template <typename V, typename T, int MODE>
+__global__ void __launch_bounds__(kFlowThreads, 1)
+k_tail_flow(Ctl *ctl, Tail<V, T> P, Flow<V, T> F, const __grid_constant__ PhaseList ph,
+            const T *__restrict__ r, const T *__restrict__ v, T *w, T *rt, double *partials,
+            unsigned long long cond) {
+  __shared__ T xch[kFlowGroups][3][32];
+  __shared__ double red[kFlowThreads];
+  __shared__ bool last;
+  if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->body_runs += 1;
+    // hard stop as a second guard: the loop can never run past maxit + 1
+    if (cond)
+      cudaGraphSetConditional((cudaGraphConditionalHandle)cond,
+                              (ctl->done || ctl->body_runs > ctl->maxit + 1) ? 0u : 1u);
+  }
+  if (ctl->done) return;
+  const T alpha = (T)ctl->alpha, beta = (T)ctl->beta, omega = (T)ctl->omega;
+  const T coef = (T)(MODE == 1 ? ctl->cs : ctl->cp);
+  const bool restart = MODE == 2 && ctl->restart;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = gridDim.x, bid = blockIdx.x;
+  const int w0 = 3 * F.groups;
+  double d = 0.0;
+  DF f = {0.f, 0.f};
+  auto updated = [&](int i) -> T {   // the new s or p at entry i
+    if (MODE == 0) return w[i];
+    const T ri = r[i];
+    const T x = MODE == 1 ? fma(-alpha, v[i], ri) : fma(beta, fma(-omega, v[i], w[i]), ri);
+    w[i] = x;
+    if (MODE == 2 && restart) rt[i] = ri;
+    if (MODE == 1) {
+      if (sizeof(T) == 8) d = fma((double)x, (double)x, d);
+      else df_add_prod(f, (float)x, (float)x);
+    }
+    return x;
+  };
+  if (warp < w0) {
+    // slice s of a step belongs to CTA s % G; three warps, one per component
+    const int g = warp / 3, c = warp % 3;
+    T(&xg)[3][32] = xch[g];
+    auto times_d = [&](const V *dm, T a) -> T {
+      xg[c][lane] = a;
+      group_sync(g);
+      const T z = dot3<T>((T)dm[sl_idx<V>(0, 3 * c, lane)], (T)dm[sl_idx<V>(0, 3 * c + 1, lane)],
+                          (T)dm[sl_idx<V>(0, 3 * c + 2, lane)], xg[0][lane], xg[1][lane],
+                          xg[2][lane]);
+      group_sync(g);
+      return z;
+    };
+    T *y = P.ybuf, *hat = P.hat;
+    for (int q = 0; q + 1 < ph.n; ++q) {
+      const Phase &S = ph.p[q];
+      const int *off = S.mat ? F.off2 : F.off1r, *col = S.mat ? F.col2 : F.col1r;
+      const V *val = S.mat ? F.val2 : F.val1r;
+      const int end = S.slice0 + ((S.nrows + 31) >> 5);
+      int s = S.slice0 + ((bid - S.slice0) % G + G) % G;   // the CTA's first slice of the step
+      for (s += g * G; s < end; s += F.groups * G) {
+        const int rr = 32 * (s - S.slice0) + lane, row = S.row0 + rr, e = 3 * row + c;
+        const bool act = rr < S.nrows;
+        const V *dm = P.dmat + (size_t)s * 288;
+        const int o = off[s], wd = off[s + 1] - o;
+        T a = 0;
+        if (act) {
+          if (S.own_y) {
+            unsigned int spins = 0;
+            while (is_sentinel(a = ld_relaxed(y + e)) && poll_again(ctl, spins)) {}
+          } else {   // a row of color 2 and up gets its p or s here
+            a = updated(e);
+            a = fma(coef, P.base[e], a);
+          }
+          a = flow_row<V, T>(val + (size_t)o * 288, col + (size_t)o * 32, wd, lane, c,
+                             S.nbr_hat ? hat : y, a, ctl);
+        }
+        if (S.has_d) a = times_d(dm, a);
+        bool fin = true;
+        if (S.to_y) {
+          fin = row >= S.final0;
+          if (act && !fin) st_relaxed(y + e, a);
+          if (S.final_d) a = times_d(dm, a);
+        }
+        if (act && fin) st_relaxed(hat + e, a);
+      }
+    }
+  } else if (MODE != 0) {
+    // color 1, groups of 32 rows dealt to the CTAs in turn
+    for (int j = (warp - w0) * G + bid; 32 * j < P.rows1; j += (kFlowWarps - w0) * G) {
+      const int t = 32 * j + lane;
+      if (t >= P.rows1) continue;
+      const int i = 3 * (P.row0 + t);
+      const T b0 = P.base[i], b1 = P.base[i + 1], b2 = P.base[i + 2];
+      const T x0 = updated(i), x1 = updated(i + 1), x2 = updated(i + 2);
+      T a0 = fma(coef, b0, x0), a1 = fma(coef, b1, x1), a2 = fma(coef, b2, x2);
+      const bool split = t < P.split1;
+      if (P.d_first || !split)
+        apply_dp<V, T, true>(P.dmat + (size_t)(P.slice1 + j) * 288, lane, a0, a1, a2);
+      T *out = (split ? P.ybuf : P.hat) + i;
+      if (split) {
+        st_relaxed(out, a0); st_relaxed(out + 1, a1); st_relaxed(out + 2, a2);
+      } else {
+        out[0] = a0; out[1] = a1; out[2] = a2;
+      }
+    }
+  }
+  if (MODE != 1) return;
+  // ||s||^2: the CTA's sum, then the CTAs' by the last one, in a fixed order
+  const int t = threadIdx.x;
+  red[t] = sizeof(T) == 4 ? df_value(f) : d;
+  __syncthreads();
+  double x = 0.0;
+  if (t < 128) x = (red[t] + red[t + 128]) + (red[t + 256] + red[t + 384]);
+  __syncthreads();
+  if (t < 128) red[t] = x;
+  __syncthreads();
+  if (t >= 32) return;
+  x = (red[t] + red[t + 32]) + (red[t + 64] + red[t + 96]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  if (t == 0) {
+    partials[bid] = x;
+    unsigned int prev;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
+                 : "=r"(prev) : "l"(&ctl->counter[3]) : "memory");
+    last = prev == gridDim.x - 1;
+  }
+  __syncwarp();
+  if (!last) return;
+  x = 0.0;
+  for (int b = t; b < G; b += 32) x += __ldcg(partials + b);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  if (t == 0) {
+    ctl->counter[3] = 0u;
+    finish_s(ctl, x);
   }
 }
 
