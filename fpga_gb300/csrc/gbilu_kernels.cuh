@@ -482,13 +482,14 @@ template <bool CG, typename T> __device__ __forceinline__ T ldv(const T *p) {
 // Neighbour columns below lo are read from xlo instead of x (the first sweep
 // reads the input vector for color 0, whose L rows are empty). EARLY: the
 // block values are loaded without waiting for the column indices.
-template <typename V, typename T, bool NEG, bool CG, bool EARLY>
+// B32: FP32 blocks in flight together.
+template <typename V, typename T, bool NEG, bool CG, bool EARLY, int B32 = kBatch>
 __device__ __forceinline__ void row_blocks(const int *__restrict__ col, const V *__restrict__ val,
                                            int o, int wdt, int lane, const T *x, const T *xlo,
                                            int lo, T &a0, T &a1, T &a2) {
   // FP64 batches of 2 keep the kernels within 128 registers (the FP64 pipe,
   // not the load latency, bounds them); FP32 batches of kBatch
-  constexpr int B = sizeof(V) == 8 ? kBatch64 : kBatch;
+  constexpr int B = sizeof(V) == 8 ? kBatch64 : B32;
   for (int k0 = 0; k0 < wdt; k0 += B) {
     int c[B];
 #pragma unroll
@@ -755,7 +756,7 @@ __device__ __forceinline__ void scale_own(const Phase &P, const T *__restrict__ 
 #endif
 // One row of a step, one thread: a = own_i - sum_j B_ij nbr_j, then stored.
 // RED: steps of the reduced iteration, own rows from base (Phase::own_base).
-template <typename V, typename T, bool CG, bool RED>
+template <typename V, typename T, bool CG, bool RED, int B32 = kBatch>
 __device__ __forceinline__ void phase_row(const Phase &P, int row, int s, int lane,
                                           const int *__restrict__ off, const int *__restrict__ col,
                                           const V *__restrict__ val, const V *__restrict__ dmat,
@@ -773,7 +774,7 @@ __device__ __forceinline__ void phase_row(const Phase &P, int row, int s, int la
   const int o = off[s], wdt = off[s + 1] - o;
   T a0 = ldv<CG>(own + 3 * row), a1 = ldv<CG>(own + 3 * row + 1), a2 = ldv<CG>(own + 3 * row + 2);
   if (RED && P.own_base) scale_own(P, base, row, coef, a0, a1, a2);
-  row_blocks<V, T, true, CG, true>(col, val, o, wdt, lane, P.nbr_hat ? hat : ybuf, src, P.src_rows, a0,
+  row_blocks<V, T, true, CG, true, B32>(col, val, o, wdt, lane, P.nbr_hat ? hat : ybuf, src, P.src_rows, a0,
                              a1, a2);
   phase_store<V, T, true>(P, row, dmat + (size_t)s * 9 * 32, lane, a0, a1, a2, ybuf, hat);
 }
@@ -782,10 +783,17 @@ __device__ __forceinline__ void phase_row(const Phase &P, int row, int s, int la
 // latency-bound and the single-launch apply stages them in shared memory.
 constexpr int kSmallRows = 16384;
 
-// One step per launch (the per-color mode; the same row arithmetic as the
-// single-launch apply, so both give identical bits).
+// One step per launch: color 0's step of the reduced iteration, and every step
+// of the per-color mode (the same row arithmetic as the single-launch apply, so
+// both give identical bits). Resident CTAs a SM: color 0 of the 500k-cell
+// system took 34.5 us in FP64 with two (88 registers), 32.8 with three, 35.1
+// with four; in FP32 19.8 with two and batches of four blocks, 17.6 with three,
+// 15.6 with four and batches of two, 14.7 with five (the solve no faster).
+template <typename T> __host__ __device__ constexpr int phase_ctas() {
+  return sizeof(T) == 4 ? 4 : 3;
+}
 template <typename V, typename T, bool RED>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, phase_ctas<T>())
 k_phase(const Ctl *ctl, Phase P, const int *__restrict__ off, const int *__restrict__ col,
         const V *__restrict__ val, const V *__restrict__ dmat, const T *src, T *ybuf, T *hat,
         const T *__restrict__ base, const double *coef) {
@@ -793,7 +801,7 @@ k_phase(const Ctl *ctl, Phase P, const int *__restrict__ off, const int *__restr
   const int t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= P.nrows) return;
   const T c = RED ? (T)*coef : (T)0;
-  phase_row<V, T, false, RED>(P, P.row0 + t, P.slice0 + (t >> 5), t & 31, off, col, val, dmat, src,
+  phase_row<V, T, false, RED, 2>(P, P.row0 + t, P.slice0 + (t >> 5), t & 31, off, col, val, dmat, src,
                               ybuf, hat, base, c);
 }
 

@@ -270,9 +270,10 @@ __device__ __forceinline__ T flow_row(const V *__restrict__ sv, const int *__res
 // waiting for 17 us an apply in FP64, and FP64's few warps cannot hide them
 // there.) Measured, vector kernel + apply with 475,000 rows: s 16.4 + 52.5 ->
 // 24.6 + 34.4 us, p 12.3 + 52.5 -> 20.7 + 34.4; an iteration 238 -> 219, with
-// 209,000 rows 149 -> 126. In FP32 the small steps cost 6 us, and a cooperative
-// vector kernel with fewer warps takes more than that (11.6 + 24.8 against 20.5
-// + 18.0): there they stay in the apply's launch (k_ilu_coop).
+// 209,000 rows 149 -> 126. In FP32 the small steps cost less, and a cooperative
+// vector kernel with fewer warps takes as much more: s 11.2 + 24.8 against 20.9
+// + 14.8 us, an iteration 200 against 208. There they stay in the apply's
+// launch (k_ilu_coop).
 template <typename V, typename T, int MODE>
 __global__ void __launch_bounds__(kFlowThreads, 1)
 k_tail_flow(Ctl *ctl, Tail<V, T> P, Flow<V, T> F, const __grid_constant__ PhaseList ph,
