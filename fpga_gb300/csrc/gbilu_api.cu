@@ -569,14 +569,15 @@ void apply_prec(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *
 
 template <typename V, typename T, int MODE>
 void spmv(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *x, T *y, const T *w,
-          int &launches, const int *x_nonzero = nullptr, int S0 = 0) {
+          int &launches, const int *x_nonzero = nullptr, int S0 = 0, Ctl *ctl = nullptr) {
   const int S = h->an.S;
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmv<V, T, MODE>, kThreads, 0);
   const int grid =
       std::max(1, std::min((S - S0 + kWarps - 1) / kWarps, std::max(1, per_sm) * h->sm_count));
   k_spmv<V, T, MODE><<<grid, kThreads, 0, s>>>(
-      h->ctl.p, S0, S, h->srows.p, o.offA, o.colA, o.valA, x, y, w, h->partials.p, x_nonzero);
+      ctl ? ctl : h->ctl.p, S0, S, h->srows.p, o.offA, o.colA, o.valA, x, y, w, h->partials.p,
+      x_nonzero);
   ++launches;
 }
 
@@ -1399,12 +1400,9 @@ int solve_mixed_ru(Handle *h, bool transpose, double tol, int maxit, gbilu_resul
   if (out.status != ST_OK) {
     Ctl *outer = h->ctl.p + 1;
     k_ctl_init<<<1, 32, 0, h->st>>>(outer, 0.0, 1, 0, 0ull);
-    const int S = h->an.S;
-    k_spmv<double, double, SPMV_RESID><<<std::min((S + kWarps - 1) / kWarps, 2 * h->sm_count),
-                                         kThreads, 0, h->st>>>(outer, 0, S, h->srows.p, o64.offA,
-                                                               o64.colA, o64.valA, w.x.p, w.r.p,
-                                                               h->b64.p, h->partials.p);
-    launches += 2;
+    l = 1;
+    spmv<double, double, SPMV_RESID>(h, h->st, o64, w.x.p, w.r.p, h->b64.p, l, nullptr, 0, outer);
+    launches += l;
     CK(cudaMemcpyAsync(h->h_ctl, outer, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     tn = h->h_ctl->norm0;
@@ -1432,23 +1430,17 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
   auto enqueue_residual = [&]() -> int {
     // r = b - A x in FP64 with the FP64 copy of A, ||r|| into h_ctl
     k_ctl_init<<<1, 32, 0, h->st>>>(outer, 0.0, 1, 0, 0ull);
-    const int S = h->an.S;
-    k_spmv<double, double, SPMV_RESID><<<std::min((S + kWarps - 1) / kWarps, 2 * h->sm_count), kThreads, 0, h->st>>>(
-        outer, 0, S, h->srows.p, o64.offA, o64.colA, o64.valA, w.x.p, w.r.p, h->b64.p, h->partials.p);
-    launches += 2;
+    int l = 1;
+    spmv<double, double, SPMV_RESID>(h, h->st, o64, w.x.p, w.r.p, h->b64.p, l, nullptr, 0, outer);
+    launches += l;
     CK(cudaMemcpyAsync(h->h_ctl, outer, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     return GBILU_OK;
   };
-  auto residual = [&](double &nrm) -> int {
-    if (int rc = enqueue_residual()) return rc;
-    CK(cudaStreamSynchronize(h->st));
-    nrm = h->h_ctl->norm0;
-    return GBILU_OK;
-  };
-  double nrm0 = 0, nrm = 0;
-  int rc = residual(nrm0);
+  int rc = enqueue_residual();
   if (rc) return rc;
-  nrm = nrm0;
+  CK(cudaStreamSynchronize(h->st));
+  const double nrm0 = h->h_ctl->norm0;
+  double nrm = nrm0;
   memset(&out, 0, sizeof out);
   out.norm0 = nrm0;
   out.norms[0] = nrm0;
@@ -1468,11 +1460,9 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
   const long long budget = 2LL * maxit + 1;
   while (nrm > bound && outer_steps < h->opt.max_outer && inner_half < budget) {
     const int left = (int)std::min<long long>((budget - inner_half - 1) / 2, h->opt.inner_maxit);
-    Ctl ic;
-    if (h->small_grid[1]) {
-      // the inner solve, its right-hand side and x += ||r|| d in one launch,
-      // the next residual behind it and one look at both (a run that broke
-      // down leaves x, and with it the residual, as they were)
+    // the correction A d = r / ||r|| in FP32 from d = 0, x += ||r|| d unless it
+    // broke down, the next residual behind it, and one look at both
+    if (h->small_grid[1]) {   // all but the residual in one launch
       SmallArgs<float, float> A = small_args(h, make_ops<float, float>(h, transpose));
       A.host_ctl = h->h_inner;
       A.r64 = w.r.p;
@@ -1484,43 +1474,31 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
       A.timeout_ns = tmo;
       CK(launch_small(h, A));
       ++launches;
-      rc = enqueue_residual();
+    } else {
+      k_ctl_init<<<1, 32, 0, h->st>>>(h->ctl.p, h->opt.inner_tol, 0, left, tmo);
+      const int nh = reduced_run(h, false) ? 3 * h->an.color_ptr[1] : 0;
+      k_init_rhs<<<reduce_grid(h, n), kThreads, 0, h->st>>>(h->ctl.p, n, nh, 1.0 / nrm, w.r.p,
+                                                            f.r.p, f.rt.p, f.p.p, f.x.p, f.base.p,
+                                                            h->partials.p);
+      // the inner run starts from x = 0: its right-hand side is rt
+      rc = run_loop<float, float>(h, transpose, left, launches, f.rt.p);
       if (rc) return rc;
-      CK(cudaStreamSynchronize(h->st));
-      CK(last_error(h));
-      ic = *h->h_inner;
-      rc = reset_small(h, ic);
-      if (rc) return rc;
-      inner_half += (ic.half >= 0 ? ic.half + 1 : 0);
-      ++outer_steps;
-      if (ic.status == ST_BREAKDOWN || ic.status == ST_NONFINITE) { out.status = ic.status; break; }
-      nrm = h->h_ctl->norm0;
-      if (!std::isfinite(nrm)) { out.status = ST_NONFINITE; break; }
-      if (ic.status == ST_TIMEOUT) { out.status = ST_TIMEOUT; break; }
-      continue;
+      k_axpy_f2d<<<g, kThreads, 0, h->st>>>(h->ctl.p, n, nrm, f.x.p, w.x.p);
+      launches += 3;
+      CK(cudaMemcpyAsync(h->h_inner, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     }
-    // right-hand side of the correction equation A d = r / ||r|| in FP32
-    // (staged in f.t, which the inner run overwrites only after reading it)
-    k_scale_convert<<<g, kThreads, 0, h->st>>>(n, 1.0 / nrm, w.r.p, f.t.p);
-    k_ctl_init<<<1, 32, 0, h->st>>>(h->ctl.p, h->opt.inner_tol, 0, left, tmo);
-    const int nh = reduced_run(h, false) ? 3 * h->an.color_ptr[1] : 0;
-    k_init_rhs<float><<<reduce_grid(h, n), kThreads, 0, h->st>>>(
-        h->ctl.p, n, nh, f.t.p, f.r.p, f.rt.p, f.p.p, f.x.p, f.base.p, h->partials.p);
-    launches += 3;
-    // the inner run starts from x = 0: its right-hand side is rt
-    rc = run_loop<float, float>(h, transpose, left, launches, f.rt.p);
+    rc = enqueue_residual();
     if (rc) return rc;
-    CK(cudaMemcpyAsync(h->h_ctl, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
-    ic = *h->h_ctl;
-    if (h->opt.use_graph) launches += (long long)ic.body_runs * h->per_iter[transpose ? 1 : 0];
+    CK(last_error(h));
+    const Ctl ic = *h->h_inner;
+    if (h->small_grid[1]) rc = reset_small(h, ic);
+    else if (h->opt.use_graph) launches += (long long)ic.body_runs * h->per_iter[transpose ? 1 : 0];
+    if (rc) return rc;
     inner_half += (ic.half >= 0 ? ic.half + 1 : 0);
     ++outer_steps;
     if (ic.status == ST_BREAKDOWN || ic.status == ST_NONFINITE) { out.status = ic.status; break; }
-    k_axpy_f2d<<<g, kThreads, 0, h->st>>>(n, nrm, f.x.p, w.x.p);
-    launches += 1;
-    rc = residual(nrm);
-    if (rc) return rc;
+    nrm = h->h_ctl->norm0;
     if (!std::isfinite(nrm)) { out.status = ST_NONFINITE; break; }
     if (ic.status == ST_TIMEOUT) { out.status = ST_TIMEOUT; break; }
   }

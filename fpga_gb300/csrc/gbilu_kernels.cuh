@@ -1723,30 +1723,29 @@ k_init_resid(Ctl *ctl, int n, int nh, const T *b, const int *__restrict__ perm, 
 }
 
 // Inner solves of iterative refinement start from d = 0: r = rt = p = rhs,
-// rho = ||rhs||^2 (step 1 without the SpMV of step 0). nh, base: as in
-// k_init_resid.
-template <typename T>
+// rho = ||rhs||^2 (step 1 without the SpMV of step 0), where rhs is the FP64
+// residual times scale, rounded once. nh, base: as in k_init_resid. One pass
+// over the vectors (a conversion of its own before it wrote and read rhs once
+// more); with 1.5 million entries 28 bytes each, bound by memory.
 __global__ void __launch_bounds__(kThreads)
-k_init_rhs(Ctl *ctl, int n, int nh, const T *__restrict__ rhs, T *__restrict__ r,
-           T *__restrict__ rt, T *__restrict__ p, T *__restrict__ x, T *__restrict__ base,
-           double *partials) {
-  double d = 0.0, dh = 0.0;
+k_init_rhs(Ctl *ctl, int n, int nh, double scale, const double *__restrict__ r64,
+           float *__restrict__ r, float *__restrict__ rt, float *__restrict__ p,
+           float *__restrict__ x, float *__restrict__ base, double *partials) {
   DF f = {0.f, 0.f}, fh = {0.f, 0.f};
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    const T v = rhs[i];
-    rt[i] = v; x[i] = 0;
+    const float v = (float)(scale * r64[i]);
+    rt[i] = v; x[i] = 0.f;
     if (i < nh) {
       base[i] = v;
-      if (sizeof(T) == 8) dh += (double)v * v; else df_add_prod(fh, (float)v, (float)v);
+      df_add_prod(fh, v, v);
     } else {
       r[i] = v; p[i] = v;
-      if (sizeof(T) == 8) d += (double)v * v; else df_add_prod(f, (float)v, (float)v);
+      df_add_prod(f, v, v);
     }
   }
-  if (sizeof(T) == 4) { d = df_value(f); dh = df_value(fh); }
-  double v[2] = {d, dh}, tot[2];
+  double v[2] = {df_value(f), df_value(fh)}, tot[2];
   if (grid_sum<2>(v, partials, &ctl->counter[0], tot) && threadIdx.x == 0)
-    finish_init<T>(ctl, tot[0] + tot[1], nh > 0, tot[1]);
+    finish_init<float>(ctl, tot[0] + tot[1], nh > 0, tot[1]);
 }
 
 // Steps 6-8 without the x update (deferred to the second half): s = r - alpha v,
@@ -2024,9 +2023,11 @@ __global__ void k_scale_convert(int n, double scale, const double *__restrict__ 
     out[i] = (float)(scale * in[i]);
 }
 
-// x += scale * d (FP64 x, FP32 correction of one refinement step)
-__global__ void k_axpy_f2d(int n, double scale, const float *__restrict__ d,
+// x += scale * d (FP64 x, FP32 correction of one refinement step) unless the
+// inner solve broke down
+__global__ void k_axpy_f2d(const Ctl *ctl, int n, double scale, const float *__restrict__ d,
                            double *__restrict__ x) {
+  if (ctl->status == ST_BREAKDOWN || ctl->status == ST_NONFINITE) return;
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
     x[i] = fma(scale, (double)d[i], x[i]);
 }
