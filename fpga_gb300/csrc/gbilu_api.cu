@@ -544,12 +544,15 @@ cudaError_t launch_coop(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *
 // the first sweep's result. RED: what the reduced iteration leaves of it, with
 // coef = &Ctl::cp (src = p) or &Ctl::cs (src = s): in FP32 one launch as well;
 // with two colors, or behind k_tail_flow (head_only), the last step alone.
+// An FP64 apply with two colors is a launch a step: a cooperative launch costs
+// more than the two launches that it saves (4,000 rows 24.6 us against 18.5,
+// 59,000 rows 24.6 against 20.9, 500,000 rows 74.2 against 76.0).
 template <typename V, typename T, bool RED = false>
 void apply_prec(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *hat,
                 int &launches, const double *coef = nullptr, bool head_only = false) {
   if constexpr (!RED || sizeof(T) == 4) {
     const int C = h->an.ncolors;
-    if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 && !(RED && C == 2)) {
+    if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 && !(C == 2 && (RED || sizeof(T) == 8))) {
       const cudaError_t e = launch_coop<V, T, RED>(h, s, o, src, hat, 0, coef);
       if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
       ++launches;
