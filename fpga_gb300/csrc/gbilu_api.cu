@@ -649,18 +649,17 @@ template <typename T> bool flow_run(const Handle *h, bool transpose) {
   return sizeof(T) == 8 && h->an.ncolors > 2 && h->sweep[1][0][transpose].phases.n > 0;
 }
 
-template <typename V, typename T, int MODE>
-void tail_flow(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned long long cond,
+template <int MODE>
+void tail_flow(Handle *h, cudaStream_t s, const Ops<double, double> &o, unsigned long long cond,
                int &launches) {
-  const int f = sizeof(T) == 4, t = o.transpose;
-  const PhaseList &pl = h->sweep[1][f][t].phases;
-  Vecs<T> &w = *o.vec;
+  const PhaseList &pl = h->sweep[1][0][o.transpose].phases;
+  Vecs<double> &w = *o.vec;
   long long slices = 0;
   for (int q = 0; q + 1 < pl.n; ++q) slices += (pl.p[q].nrows + kSliceRows - 1) / kSliceRows;
   // one group of three warps for about two slices
   const long long share = 2ll * h->sm_count;
-  const Flow<V, T> F{o.off1r, o.col1r, o.val1r, o.off2, o.col2, o.val2, w.sh.p, w.ysh.p,
-                     (int)std::max<long long>(1, std::min<long long>(kFlowGroups, (slices + share - 1) / share))};
+  const Flow F{o.off1r, o.col1r, o.val1r, o.off2, o.col2, o.val2,
+               (int)std::max<long long>(1, std::min<long long>(kFlowGroups, (slices + share - 1) / share))};
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -670,10 +669,10 @@ void tail_flow(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned long long
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const Tail<V, T> P =
+  const Tail<double, double> P =
       MODE == 1 ? make_tail(h, o, w.sh.p, w.ysh.p) : make_tail(h, o, w.ph.p, w.y.p);
   const cudaError_t e = cudaLaunchKernelEx(
-      &cfg, k_tail_flow<V, T, MODE>, h->ctl.p, P, F, pl, (const T *)w.r.p, (const T *)w.v.p,
+      &cfg, k_tail_flow<MODE>, h->ctl.p, P, F, pl, (const double *)w.r.p, (const double *)w.v.p,
       MODE == 1 ? w.s.p : w.p.p, w.rt.p, h->partials.p, cond);
   if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
   ++launches;
@@ -694,7 +693,7 @@ void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned lon
   apply_prec<V, T, true>(h, s, o, w.p.p, w.ph.p, launches, &c->cp, flow);
   spmv<V, T, SPMV_ALPHA>(h, s, o, w.ph.p, w.v.p, w.rt.p, launches, nullptr, S0);
   if (flow) {
-    tail_flow<V, T, 1>(h, s, o, 0ull, launches);
+    if constexpr (sizeof(T) == 8) tail_flow<1>(h, s, o, 0ull, launches);
   } else {
     k_tail_s<V, T><<<row_grid(h, tp.rows, GBILU_REDUCE_CTAS_PER_SM), kThreads, 0, s>>>(
         c, ts, w.r.p, w.v.p, w.s.p, part);
@@ -707,7 +706,7 @@ void enqueue_reduced(Handle *h, cudaStream_t s, const Ops<V, T> &o, unsigned lon
       flow ? n0 + 3 * tp.split1 : n0, flow ? n0 + 3 * tp.rows1 : n0 + nt, w.y.p, w.ysh.p);
   ++launches;
   if (flow) {
-    tail_flow<V, T, 2>(h, s, o, cond, launches);
+    if constexpr (sizeof(T) == 8) tail_flow<2>(h, s, o, cond, launches);
   } else {
     k_tail_p<V, T><<<row_grid(h, tp.rows, 8), kThreads, 0, s>>>(c, tp, w.r.p, w.v.p, w.p.p,
                                                                        w.rt.p, cond);
@@ -733,7 +732,7 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
   ++launches;
   if (flow) {
     int l = 0;
-    tail_flow<V, T, 0>(h, h->st, o, 0ull, l);
+    if constexpr (sizeof(T) == 8) tail_flow<0>(h, h->st, o, 0ull, l);
     launches += l;
   }
 }
@@ -797,7 +796,6 @@ template <typename V, typename T> SmallArgs<V, T> small_args(Handle *h, const Op
   A.S0 = an.slice_color_ptr[1];
   A.S1 = an.slice_color_ptr[2];
   A.n0 = an.color_ptr[1];
-  A.rows1 = an.color_ptr[2] - A.n0;
   A.split1 = an.split[1];
   A.transpose = o.transpose;
   A.offA = o.offA; A.colA = o.colA; A.valA = o.valA;
@@ -1573,11 +1571,11 @@ void iter_kernel(Handle *h, int kind, const Ops<V, T> &o, int n, int g, int gr, 
       return;
     }
     if (flow && kind == 6) {
-      tail_flow<V, T, 1>(h, h->st, o, 0ull, l);
+      if constexpr (sizeof(T) == 8) tail_flow<1>(h, h->st, o, 0ull, l);
       return;
     }
     if (flow && kind == 8) {
-      tail_flow<V, T, 2>(h, h->st, o, 0ull, l);
+      if constexpr (sizeof(T) == 8) tail_flow<2>(h, h->st, o, 0ull, l);
       return;
     }
     if (kind == 4) {

@@ -202,10 +202,9 @@ k_tail_p(Ctl *ctl, Tail<V, T> P, const T *__restrict__ r, const T *__restrict__ 
 // --------------------------------------------------------------------------
 
 // What a tail kernel needs to run the small steps too.
-template <typename V, typename T> struct Flow {
-  const int *off1r, *col1r; const V *val1r;   // first sweep, the tail's columns
-  const int *off2, *col2; const V *val2;      // second sweep
-  T *sh, *ysh;            // s^ and the small steps' y of s (Tail: p's or s's)
+struct Flow {
+  const int *off1r, *col1r; const double *val1r;   // first sweep, the tail's columns
+  const int *off2, *col2; const double *val2;      // second sweep
   int groups;             // groups of three warps on the small steps
 };
 constexpr int kFlowThreads = 512;
@@ -213,30 +212,30 @@ constexpr int kFlowWarps = kFlowThreads / 32;
 constexpr int kFlowGroups = 4;     // at most: the other warps form p or s
 
 // Component c of a row: a - its blocks' row c times x, once every value is
-// there (sentinels in x are waited for; *late: the wait ran out).
-template <typename V, typename T>
-__device__ __forceinline__ T flow_row(const V *__restrict__ sv, const int *__restrict__ sc, int w,
-                                      int lane, int c, const T *x, T a, Ctl *ctl) {
+// there (sentinels in x are waited for; a wait that runs out stops the solve).
+__device__ __forceinline__ double flow_row(const double *__restrict__ sv,
+                                           const int *__restrict__ sc, int w, int lane, int c,
+                                           const double *x, double a, Ctl *ctl) {
   constexpr int B = 2;   // (4: 2 % slower)
   for (int k0 = 0; k0 < w; k0 += B) {
     int cc[B];
-    T y[B][3];
-    V b[B][3];
+    double y[B][3];
+    double b[B][3];
 #pragma unroll
     for (int j = 0; j < B; ++j) {
       cc[j] = k0 + j < w ? sc[(k0 + j) * 32 + lane] : -1;
 #pragma unroll
       for (int e = 0; e < 3; ++e)
-        if (k0 + j < w) b[j][e] = sv[(size_t)(k0 + j) * 288 + sl_idx<V>(0, 3 * c + e, lane)];
+        if (k0 + j < w) b[j][e] = sv[(size_t)(k0 + j) * 288 + sl_idx<double>(0, 3 * c + e, lane)];
     }
     unsigned int spins = 0;
     bool wait;
     do {
-      const T *miss = nullptr;
+      const double *miss = nullptr;
 #pragma unroll
       for (int j = 0; j < B; ++j)
         if (cc[j] >= 0) {
-          const T *xs = x + 3 * cc[j];
+          const double *xs = x + 3 * cc[j];
 #pragma unroll
           for (int e = 0; e < 3; ++e) {
             y[j][e] = ld_relaxed(xs + e);
@@ -252,7 +251,7 @@ __device__ __forceinline__ T flow_row(const V *__restrict__ sv, const int *__res
     for (int j = 0; j < B; ++j)
       if (cc[j] >= 0)
 #pragma unroll
-        for (int e = 0; e < 3; ++e) a = fma(-(T)b[j][e], y[j][e], a);
+        for (int e = 0; e < 3; ++e) a = fma(-b[j][e], y[j][e], a);
   }
   return a;
 }
@@ -274,11 +273,13 @@ __device__ __forceinline__ T flow_row(const V *__restrict__ sv, const int *__res
 // vector kernel with fewer warps takes as much more: s 11.2 + 24.8 against 20.9
 // + 14.8 us, an iteration 200 against 208. There they stay in the apply's
 // launch (k_ilu_coop).
-template <typename V, typename T, int MODE>
+template <int MODE>
 __global__ void __launch_bounds__(kFlowThreads, 1)
-k_tail_flow(Ctl *ctl, Tail<V, T> P, Flow<V, T> F, const __grid_constant__ PhaseList ph,
-            const T *__restrict__ r, const T *__restrict__ v, T *w, T *rt, double *partials,
-            unsigned long long cond) {
+k_tail_flow(Ctl *ctl, Tail<double, double> P, Flow F, const __grid_constant__ PhaseList ph,
+            const double *__restrict__ r, const double *__restrict__ v, double *w, double *rt,
+            double *partials, unsigned long long cond) {
+  using V = double;
+  using T = double;
   __shared__ T xch[kFlowGroups][3][32];
   __shared__ double red[kFlowThreads];
   __shared__ bool last;
@@ -296,17 +297,13 @@ k_tail_flow(Ctl *ctl, Tail<V, T> P, Flow<V, T> F, const __grid_constant__ PhaseL
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = gridDim.x, bid = blockIdx.x;
   const int w0 = 3 * F.groups;
   double d = 0.0;
-  DF f = {0.f, 0.f};
   auto updated = [&](int i) -> T {   // the new s or p at entry i
     if (MODE == 0) return w[i];
     const T ri = r[i];
     const T x = MODE == 1 ? fma(-alpha, v[i], ri) : fma(beta, fma(-omega, v[i], w[i]), ri);
     w[i] = x;
     if (MODE == 2 && restart) rt[i] = ri;
-    if (MODE == 1) {
-      if (sizeof(T) == 8) d = fma((double)x, (double)x, d);
-      else df_add_prod(f, (float)x, (float)x);
-    }
+    if (MODE == 1) d = fma(x, x, d);
     return x;
   };
   if (warp < w0) {
@@ -343,7 +340,7 @@ k_tail_flow(Ctl *ctl, Tail<V, T> P, Flow<V, T> F, const __grid_constant__ PhaseL
             a = updated(e);
             a = fma(coef, P.base[e], a);
           }
-          a = flow_row<V, T>(val + (size_t)o * 288, col + (size_t)o * 32, wd, lane, c,
+          a = flow_row(val + (size_t)o * 288, col + (size_t)o * 32, wd, lane, c,
                              S.nbr_hat ? hat : y, a, ctl);
         }
         if (S.has_d) a = times_d(dm, a);
@@ -379,7 +376,7 @@ k_tail_flow(Ctl *ctl, Tail<V, T> P, Flow<V, T> F, const __grid_constant__ PhaseL
   if (MODE != 1) return;
   // ||s||^2: the CTA's sum, then the CTAs' by the last one, in a fixed order
   const int t = threadIdx.x;
-  red[t] = sizeof(T) == 4 ? df_value(f) : d;
+  red[t] = d;
   __syncthreads();
   double x = 0.0;
   if (t < 128) x = (red[t] + red[t + 128]) + (red[t + 256] + red[t + 384]);

@@ -16,7 +16,7 @@
 // same launch.
 //
 // Measured against the separate kernels: an iteration of 4,000 cells 59 -> 28
-// us, of 33,000 cells (three colors) 97 -> 53, of 108,000 cells 88 -> 72 (see
+// us, of 33,000 cells (three colors) 97 -> 49, of 108,000 cells 88 -> 63 (see
 // GBILU_SMALL_ROWS64 for where it ends). Ordering the steps between two
 // reductions by their data instead (results preset to a sentinel, consumers
 // polling) gave 28.7 us for 4,000 cells with two colors, but 47 instead of 44
@@ -48,7 +48,7 @@ template <typename V, typename T> struct SmallArgs {
   double *partials;               // 9 sums a CTA
   const int2 *srows;
   int S, S0, S1;                  // slices; the first of the tail, of color 2
-  int n0, rows1, split1;          // head rows; Tail's rows1 and split1
+  int n0, split1;                 // head rows; Tail's split1
   int transpose;
   const int *offA, *colA; const V *valA;
   const int *off1, *col1; const V *val1;
