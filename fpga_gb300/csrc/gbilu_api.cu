@@ -899,7 +899,8 @@ template <> Ops<float, float> make_ops(Handle *h, bool t) {
 // right-hand side in the device numbering (only the head's rows are read,
 // by the reduced form).
 template <typename V, typename T>
-int run_loop(Handle *h, bool transpose, int maxit, long long &launches, const T *b, bool ru = false) {
+int run_loop(Handle *h, bool transpose, int maxit, long long &launches, const T *b, bool ru = false,
+             Refine out = {nullptr, 0.0}) {
   Ops<V, T> o = make_ops<V, T>(h, transpose);
   Ops<double, double> o64 = make_ops<double, double>(h, transpose);
   const Ops<double, double> *ru64 = ru ? &o64 : nullptr;
@@ -928,13 +929,15 @@ int run_loop(Handle *h, bool transpose, int maxit, long long &launches, const T 
       if (h->h_ctl->done) break;
     }
   }
-  k_finish_x<T><<<grid_for(h, n), kThreads, 0, h->st>>>(h->ctl.p, n, o.vec->x.p + n0,
-                                                        o.vec->ph.p + n0);
+  k_finish_x<T><<<grid_for(h, n), kThreads, 0, h->st>>>(
+      h->ctl.p, n, o.vec->x.p + n0, o.vec->ph.p + n0,
+      Refine{out.x64 ? out.x64 + n0 : nullptr, out.scale});
   launches += 1;
   if (red) {
     const int rows = n0 / 3;
     k_finish_head<V, T><<<(rows + kThreads - 1) / kThreads, kThreads, 0, h->st>>>(
-        h->ctl.p, rows, transpose, o.off2, o.col2, o.val2, o.dmat, b, o.vec->rt.p, o.vec->x.p);
+        h->ctl.p, rows, transpose, o.off2, o.col2, o.val2, o.dmat, b, o.vec->rt.p, o.vec->x.p,
+        out);
     launches += 1;
   }
   CK(last_error(h));
@@ -1427,7 +1430,6 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
   Vecs<double> &w = h->v64;
   Vecs<float> &f = h->v32;
   Ctl *outer = h->ctl.p + 1;
-  const int g = grid_for(h, n);
   auto enqueue_residual = [&]() -> int {
     // r = b - A x in FP64 with the FP64 copy of A, ||r|| into h_ctl
     k_ctl_init<<<1, 32, 0, h->st>>>(outer, 0.0, 1, 0, 0ull);
@@ -1482,10 +1484,9 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
                                                             f.r.p, f.rt.p, f.p.p, f.x.p, f.base.p,
                                                             h->partials.p);
       // the inner run starts from x = 0: its right-hand side is rt
-      rc = run_loop<float, float>(h, transpose, left, launches, f.rt.p);
+      rc = run_loop<float, float>(h, transpose, left, launches, f.rt.p, false, Refine{w.x.p, nrm});
       if (rc) return rc;
-      k_axpy_f2d<<<g, kThreads, 0, h->st>>>(h->ctl.p, n, nrm, f.x.p, w.x.p);
-      launches += 3;
+      launches += 2;
       CK(cudaMemcpyAsync(h->h_inner, h->ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));
     }
     rc = enqueue_residual();

@@ -409,12 +409,13 @@ k_tail_flow(Ctl *ctl, Tail<double, double> P, Flow F, const __grid_constant__ Ph
 // The head's x after the loop, from its equations and the residual they are
 // left with: forward x = D^-1 (b - c r0 - sum U x), adjoint
 // x = D^-T (b - c r0) - sum L^T x, c = cs after a stop in a first half, else
-// cr. x keeps its start value when no iteration moved it.
+// cr. x keeps its start value when no iteration moved it (zero in a
+// refinement step, which then adds nothing).
 template <typename V, typename T>
 __global__ void __launch_bounds__(kThreads)
 k_finish_head(const Ctl *ctl, int rows, int d_first, const int *__restrict__ off,
               const int *__restrict__ col, const V *__restrict__ val, const V *__restrict__ dmat,
-              const T *__restrict__ b, const T *__restrict__ r0, T *x) {
+              const T *__restrict__ b, const T *__restrict__ r0, T *x, Refine out) {
   if (ctl->half < 0 || !(ctl->stop_half || ctl->x_moved)) return;
   const int t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= rows) return;
@@ -428,6 +429,12 @@ k_finish_head(const Ctl *ctl, int rows, int d_first, const int *__restrict__ off
   row_blocks<V, T, true, false, true>(col, val, o, off[s + 1] - o, lane, x, x, 0, a0, a1, a2);
   if (!d_first) apply_dp<V, T, true>(d, lane, a0, a1, a2);
   x[3 * t] = a0; x[3 * t + 1] = a1; x[3 * t + 2] = a2;
+  if (out.x64 && ctl->status != ST_BREAKDOWN && ctl->status != ST_NONFINITE) {
+    double *y = out.x64 + 3 * t;
+    y[0] = fma(out.scale, (double)a0, y[0]);
+    y[1] = fma(out.scale, (double)a1, y[1]);
+    y[2] = fma(out.scale, (double)a2, y[2]);
+  }
 }
 
 }  // namespace gbilu

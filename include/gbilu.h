@@ -68,7 +68,9 @@ typedef struct {
   int device;         /* CUDA device ordinal; -1 = host-only handle that
                          can analyze and factor but not solve */
   int use_graph;      /* 1: iteration loop as a CUDA graph with a device-
-                         side while loop; 0: host-driven launches */
+                         side while loop; 0: host-driven launches (no
+                         difference for solves that run in one launch: small
+                         systems of two and more colors) */
   double timeout_ms;  /* 0 = none; else a solve that exceeds this device
                          time stops with GBILU_TIMEOUT */
   double inner_tol;   /* mixed: relative tolerance of each inner solve */
@@ -78,7 +80,9 @@ typedef struct {
   int sweep_mode;     /* 1: the whole ILU0 apply is one cooperative launch
                          (default): grid barriers around the large
                          colors, the small ones ordered by their data;
-                         0: one launch per color */
+                         0: one launch per color (same results). An FP64
+                         apply with two colors, and the loop of a solve in
+                         FP64 or in one launch, do not depend on it */
   int factor_on_device; /* 1: gbilu_factor permutes and ILU0-factors on the
                          GPU (color-parallel, bit-identical to the host
                          factorization); 0: on the host (default) */
