@@ -209,16 +209,16 @@ Csr transpose_csr(int nb, const Csr &m) {
   return t;
 }
 
-// The blocks of m whose column is c0 or later.
+// The blocks of m whose column is c0 or later (columns ascend in a row).
 Csr from_column(int nb, const Csr &m, int c0) {
   Csr r;
   r.rowptr.assign(static_cast<size_t>(nb) + 1, 0);
   for (int i = 0; i < nb; ++i) {
-    for (int k = m.rowptr[i]; k < m.rowptr[i + 1]; ++k)
-      if (m.col[k] >= c0) {
-        r.col.push_back(m.col[k]);
-        r.src.push_back(m.src[k]);
-      }
+    const int e = m.rowptr[i + 1];
+    int b = e;
+    while (b > m.rowptr[i] && m.col[b - 1] >= c0) --b;
+    r.col.insert(r.col.end(), m.col.begin() + b, m.col.begin() + e);
+    r.src.insert(r.src.end(), m.src.begin() + b, m.src.begin() + e);
     r.rowptr[i + 1] = static_cast<int>(r.col.size());
   }
   return r;
@@ -305,19 +305,26 @@ std::string analyze(int nb, const int *rowptr, const int *colind, Analysis &an,
 
   // L / U / A row selections (src = permuted block index)
   Csr a, l, u;
-  a.rowptr.assign(static_cast<size_t>(nb) + 1, 0);
-  l.rowptr = a.rowptr;
-  u.rowptr = a.rowptr;
+  a.rowptr = an.prowptr;
+  a.col = an.pcolind;
+  a.src.resize(an.nnzb);
+  std::iota(a.src.begin(), a.src.end(), 0);
+  l.rowptr.assign(static_cast<size_t>(nb) + 1, 0);
+  u.rowptr = l.rowptr;
   for (int i = 0; i < nb; ++i) {
-    for (int k = an.prowptr[i]; k < an.prowptr[i + 1]; ++k) {
-      const int j = an.pcolind[k];
-      a.col.push_back(j); a.src.push_back(k);
-      if (j < i) { l.col.push_back(j); l.src.push_back(k); }
-      if (j > i) { u.col.push_back(j); u.src.push_back(k); }
-    }
-    a.rowptr[i + 1] = static_cast<int>(a.col.size());
-    l.rowptr[i + 1] = static_cast<int>(l.col.size());
-    u.rowptr[i + 1] = static_cast<int>(u.col.size());
+    l.rowptr[i + 1] = l.rowptr[i] + an.pdiag[i] - an.prowptr[i];
+    u.rowptr[i + 1] = u.rowptr[i] + an.prowptr[i + 1] - an.pdiag[i] - 1;
+  }
+  l.col.resize(l.rowptr[nb]);
+  l.src.resize(l.rowptr[nb]);
+  u.col.resize(u.rowptr[nb]);
+  u.src.resize(u.rowptr[nb]);
+  for (int i = 0; i < nb; ++i) {
+    const auto col = an.pcolind.begin(), src = a.src.begin();
+    std::copy(col + an.prowptr[i], col + an.pdiag[i], l.col.begin() + l.rowptr[i]);
+    std::copy(src + an.prowptr[i], src + an.pdiag[i], l.src.begin() + l.rowptr[i]);
+    std::copy(col + an.pdiag[i] + 1, col + an.prowptr[i + 1], u.col.begin() + u.rowptr[i]);
+    std::copy(src + an.pdiag[i] + 1, src + an.prowptr[i + 1], u.src.begin() + u.rowptr[i]);
   }
   an.nnzb_l = static_cast<int>(l.col.size());
   an.nnzb_u = static_cast<int>(u.col.size());
