@@ -255,19 +255,17 @@ def gpu_bench(args, world, rank, local):
     it_ms = value / max(1, (r0.half_iters + 1) / 2.0)
     solve_gbs = st["alg_bytes_iter"][0] / it_ms / 1e6 if it_ms > 0 else None
     traffic = None
-    tfile = os.path.join(ROOT, "profiles", "ilu64_c2_traffic.txt")
+    tfile = os.path.join(ROOT, "profiles", "spmv_omega64_c2_traffic.txt")
     if os.path.exists(tfile):
         for line in open(tfile):
             if line.startswith("bytes_per_launch:"):
                 traffic = float(line.split(":")[1])
     # the dominant kernel of the FP64 solve by device-time share (ncu launch
-    # list, profiles/): the single-launch ILU0 apply
-    dom = kern["ilu64"]
-    # its FP64 floor: 9 FMA per block of L, U and D^-1 at the FP64 rate
-    # measured on GB300 (1.68 FMA lanes per clock per SM, 2.07 GHz)
-    fp64_fma_per_s = 1.68 * torch.cuda.get_device_properties(local).multi_processor_count * 2.07e9
-    fp64_floor_us = 9 * (st["nnzb_lower"] + st["nnzb_upper"] + st["nb"]) / fp64_fma_per_s * 1e6
-    roofline = {"bound": "hbm", "kernel": "k_ilu_coop<double> (ILU0 L+U sweeps, FP64)",
+    # list, profiles/): the SpMV of the rows outside color 0 with its dots
+    ms, by, la = g.bench_kernel("spmv_omega64", reps=20)
+    dom = {"ms": ms, "alg_bytes": by, "gbs": by / ms / 1e6}
+    fp64_floor_us = iteration_fmas(g64, st, s.rowptr)["spmv_omega"] / fp64_fma_rate(local) * 1e6
+    roofline = {"bound": "hbm", "kernel": "k_spmv<double> with the omega dots (rows outside color 0)",
                 "achieved": dom["gbs"], "peak": peak, "unit": "GB/s",
                 "frac": dom["gbs"] / peak, "traffic": traffic,
                 "peak_kind": peak_kind, "alg_bytes_per_launch": dom["alg_bytes"],
@@ -313,30 +311,39 @@ FP64_FMA_LANES_PER_CLK_SM = 1.68   # measured on GB300 (independent DFMA chains)
 SM_CLOCK_HZ = 2.07e9
 
 
-def iteration_budget(g, g64, st, rowptr, b_dev, x_dev, local):
-    """Where one BiCGSTAB iteration's time goes: every kernel of the
-    iteration timed alone (back to back, CUDA events), beside its HBM floor
-    (algorithmic bytes at the measured copy peak) and, for FP64, its FP64
-    floor (DFMA count at the measured FP64 rate); and the measured time per
-    iteration of whole solves (the slope between maxit 4 and 12, tol 0)."""
-    import numpy as np
+def fp64_fma_rate(local):
+    """FP64 multiply-adds a second of one GPU."""
     import torch
-    peak, _ = peaks()
     sms = torch.cuda.get_device_properties(local).multi_processor_count
-    fma_rate = FP64_FMA_LANES_PER_CLK_SM * sms * SM_CLOCK_HZ
-    # DFMA per launch (FP64) over the rows that the iteration runs on: color 0
-    # (n0 rows, a0 blocks of A) takes part in the apply's last step alone; the
-    # other n rows in the SpMV (9 per block and the dots) and the vector
-    # kernels (update_s and update_p also apply D^-1 to color 1)
+    return FP64_FMA_LANES_PER_CLK_SM * sms * SM_CLOCK_HZ
+
+
+def iteration_fmas(g64, st, rowptr):
+    """DFMA per launch (FP64) over the rows that the iteration runs on: color
+    0 (n0 rows, a0 blocks of A) takes part in the apply's last step alone; the
+    other n rows in the SpMV (9 per block and the dots) and the vector kernels
+    (update_s and update_p also apply D^-1 to color 1)."""
+    import numpy as np
     _, color, _, cp = g64.ordering()
     n0, n1 = int(cp[1]), int(cp[2] - cp[1])
     deg = np.diff(rowptr)
     a0 = int(deg[color == 0].sum())
     nb, nnzb, n = st["nb"], st["nnzb"], 3 * (st["nb"] - n0)
     inner = st["nnzb_lower"] + st["nnzb_upper"] - 2 * (a0 - n0)
-    fmas = {"apply": 9 * (a0 - n0 + inner + nb - n1), "spmv_alpha": 9 * (nnzb - a0) + n,
+    return {"apply": 9 * (a0 - n0 + inner + nb - n1), "spmv_alpha": 9 * (nnzb - a0) + n,
             "spmv_omega": 9 * (nnzb - a0) + 2 * n, "update_s": 3 * n + 9 * n1,
             "update_r": 5 * n, "update_p": 3 * n + 9 * n1}
+
+
+def iteration_budget(g, g64, st, rowptr, b_dev, x_dev, local):
+    """Where one BiCGSTAB iteration's time goes: every kernel of the
+    iteration timed alone (back to back, CUDA events), beside its HBM floor
+    (algorithmic bytes at the measured copy peak) and, for FP64, its FP64
+    floor (DFMA count at the measured FP64 rate); and the measured time per
+    iteration of whole solves (the slope between maxit 4 and 12, tol 0)."""
+    peak, _ = peaks()
+    fma_rate = fp64_fma_rate(local)
+    fmas = iteration_fmas(g64, st, rowptr)
     out = {}
     for prec, suf in (("fp64", "64"), ("fp32", "32")):
         rows = {}
@@ -680,7 +687,8 @@ def main():
                     help="host-driven launches instead of the graph loop (profiler runs: "
                          "kernels inside a conditional graph node are not listed by ncu)")
     ap.add_argument("--kernel-only", default=None,
-                    choices=["spmv64", "ilu64", "spmv32", "ilu32"],
+                    choices=["spmv64", "ilu64", "spmv32", "ilu32", "spmv_omega64", "spmv_omega32",
+                             "apply64", "apply32"],
                     help="time one kernel family alone (3 warm-up + --steps launches)")
     ap.add_argument("--mixed-only", action="store_true",
                     help="only mixed solves of the 500k-cell system to 1e-8 (profiler runs of "
