@@ -562,7 +562,7 @@ void apply_prec(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *
   const std::vector<Phase> &steps = h->sweep[RED][sizeof(T) == 4 ? 1 : 0][o.transpose ? 1 : 0].steps;
   for (size_t q = head_only ? steps.size() - 1 : 0; q < steps.size(); ++q) {
     const Phase &P = steps[q];
-    k_phase<V, T, RED><<<(unsigned)((P.nrows + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+    k_phase<V, T, RED><<<(unsigned)((P.nrows + kPhaseThreads - 1) / kPhaseThreads), kPhaseThreads, 0, s>>>(
         h->ctl.p, P, P.mat ? o.off2 : RED ? o.off1r : o.off1,
         P.mat ? o.col2 : RED ? o.col1r : o.col1, P.mat ? o.val2 : RED ? o.val1r : o.val1, o.dmat,
         src, o.vec->y.p, hat, o.vec->base.p, coef);

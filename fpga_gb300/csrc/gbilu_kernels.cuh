@@ -785,20 +785,24 @@ constexpr int kSmallRows = 16384;
 
 // One step per launch: color 0's step of the reduced iteration, and every step
 // of the per-color mode (the same row arithmetic as the single-launch apply, so
-// both give identical bits). Resident CTAs a SM: color 0 of the 500k-cell
-// system took 34.5 us in FP64 with two (88 registers), 32.8 with three, 35.1
-// with four; in FP32 19.8 with two and batches of four blocks, 17.6 with three,
-// 15.6 with four and batches of two, 14.7 with five (the solve no faster).
+// both give identical bits). Resident CTAs of 256 threads a SM: color 0 of the
+// 500k-cell system took 34.5 us in FP64 with two (88 registers), 32.8 with
+// three, 35.1 with four; in FP32 19.8 with two and batches of four blocks, 17.6
+// with three, 15.6 with four and batches of two, 14.7 with five (the solve no
+// faster).
+// CTAs of 128 threads, so that the last ones to run hold less work: 2M cells
+// FP64 110.0 -> 108.2 us, the 500k-cell system the same.
+constexpr int kPhaseThreads = 128;
 template <typename T> __host__ __device__ constexpr int phase_ctas() {
   return sizeof(T) == 4 ? 4 : 3;
 }
 template <typename V, typename T, bool RED>
-__global__ void __launch_bounds__(kThreads, phase_ctas<T>())
+__global__ void __launch_bounds__(kPhaseThreads, phase_ctas<T>() * kThreads / kPhaseThreads)
 k_phase(const Ctl *ctl, Phase P, const int *__restrict__ off, const int *__restrict__ col,
         const V *__restrict__ val, const V *__restrict__ dmat, const T *src, T *ybuf, T *hat,
         const T *__restrict__ base, const double *coef) {
   if (ctl->done) return;
-  const int t = blockIdx.x * kThreads + threadIdx.x;
+  const int t = blockIdx.x * kPhaseThreads + threadIdx.x;
   if (t >= P.nrows) return;
   const T c = RED ? (T)*coef : (T)0;
   phase_row<V, T, false, RED, 2>(P, P.row0 + t, P.slice0 + (t >> 5), t & 31, off, col, val, dmat, src,
