@@ -148,7 +148,9 @@ typedef struct {
   long long slots_l;
   long long slots_u;
   long long device_bytes;   /* device memory held by the handle */
-  int launches_per_iter;    /* kernels one BiCGSTAB iteration launches */
+  int launches_per_iter;    /* kernels one BiCGSTAB iteration launches (0
+                               before the first solve, and for solves that
+                               run in one launch) */
   long long last_launches;  /* kernels launched by the last solve */
   double factor_ms;         /* host ILU0 + upload time of the last factor */
   double analyze_ms;
