@@ -436,6 +436,20 @@ int bilu0(const Analysis &an, double *v, double *dinv) {
   return -1;
 }
 
+double head_gain(const Analysis &an, const double *lu, const double *dinv) {
+  double most = 0.0;
+  for (int i = 0; i < an.color_ptr[1]; ++i) {
+    const double *a = lu + static_cast<size_t>(an.pdiag[i]) * 9, *d = dinv + static_cast<size_t>(i) * 9;
+    for (int r = 0; r < 3; ++r)
+      for (int c = 0; c < 3; ++c) {
+        const double g = std::fabs(d[3 * r + c] * a[3 * c + r]);
+        if (!(g <= most)) most = g;
+        if (std::isnan(g)) return g;
+      }
+  }
+  return most;
+}
+
 template <typename V>
 void fill_sliced(const SlicedMatrix &m, const double *src, V *out) {
   const size_t slots = static_cast<size_t>(m.slots());

@@ -100,6 +100,12 @@ std::string color_parity_device(int nb, const int *rowptr, const int *colind, in
 // inverses of U's diagonal blocks. Returns -1 or the first singular row.
 int bilu0(const Analysis &an, double *pvals, double *dinv);
 
+// The largest entry of the relative gain arrays |A_ii| o |A_ii^-T| (entry by
+// entry) of color 0's diagonal blocks (lu, dinv as bilu0 leaves them): how far
+// each 3x3 block is from well conditioned under the best scaling of its rows
+// and columns. Not finite when an entry is not. reduced_run says what it is for.
+double head_gain(const Analysis &an, const double *lu, const double *dinv);
+
 // Gathers input-order values into the permuted order.
 void permute_values(const Analysis &an, const double *vals, double *pvals);
 

@@ -2171,7 +2171,8 @@ __global__ void k_block_positions(long long n, const int *__restrict__ vsrc,
 // k < i in row i, L_ik = A_ik U_kk^-1, then A_ij -= L_ik U_kj for the j > k
 // present in both rows (a merge of the two sorted column lists);
 // D_i^-1 = inv(A_ii) by cofactors. A singular (or not finite) pivot records
-// the smallest failing row in *bad. Finished blocks also go straight to the
+// the smallest failing row in bad[0]; bad[1] gets minus the high word of color
+// 0's head_gain (both start from 0x7f7f7f7f). Finished blocks also go straight to the
 // sliced L, U, their transposes and D^-1, D^-T (FactorOut): the FP64 unit
 // bounds the kernel, and a pass of its own for each array took 0.2 ms more.
 //
@@ -2316,6 +2317,7 @@ k_bilu0_rows(int row_a, int rows_a, int row_b, int rows_b, int color_row0, int c
     a[3 * q + 1] = __shfl_sync(0xffffffffu, g1, from);
     a[3 * q + 2] = __shfl_sync(0xffffffffu, g2, from);
   }
+  const unsigned int active = __ballot_sync(0xffffffffu, act);
   if (!act) return;
   const double c00 = dsub(dmul(a[4], a[8]), dmul(a[5], a[7]));
   const double c01 = dsub(dmul(a[5], a[6]), dmul(a[3], a[8]));
@@ -2333,6 +2335,15 @@ k_bilu0_rows(int row_a, int rows_a, int row_b, int rows_b, int color_row0, int c
   }
   double *o = dinv + (size_t)i * 9 + 3 * r;
   o[0] = o0; o[1] = o1; o[2] = o2;
+  if (color_row0 == 0) {   // head_gain: row r of the inverse, column r of the block
+    auto high = [&](double x) { return __double2hiint(x) & 0x7fffffff; };
+    const int g = max(max(high(dmul(o0, r == 0 ? a[0] : r == 1 ? a[1] : a[2])),
+                          high(dmul(o1, r == 0 ? a[3] : r == 1 ? a[4] : a[5]))),
+                      high(dmul(o2, r == 0 ? a[6] : r == 1 ? a[7] : a[8])));
+    const int most = __reduce_max_sync(active, g);
+    // one address for all warps: few of them still raise it
+    if (lane == 0 && -most < *(volatile int *)(bad + 1)) atomicMin(bad + 1, -most);
+  }
   const int d = F.drow[i] - color_row0, dl = d & 31;
   const size_t ds = (size_t)(color_slice0 + (d >> 5));
   const double oo[3] = {o0, o1, o2};
