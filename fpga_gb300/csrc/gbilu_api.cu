@@ -1918,6 +1918,11 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
       db = h->io64.p;
       dx = h->io64b.p;
     }
+    // dL/dA reads gx after this launch wrote lambda: where the caller's two
+    // arrays overlap, lambda stays in the staging buffer until then
+    const bool overlap = device_ptrs && gx && gdA && (uintptr_t)x < (uintptr_t)(gx + n) &&
+                         (uintptr_t)gx < (uintptr_t)(x + n);
+    if (overlap) dx = h->io64b.p;
     SmallArgs<double, double> A = small_args(h, make_ops<double, double>(h, transpose));
     A.host_ctl = h->h_ctl;
     A.b = h->b64.p;
@@ -1940,6 +1945,8 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
       k_grad_a<<<entry_grid(h, h->an.nnzb), kEntryThreads, 0, h->st>>>(
           h->an.nnzb, h->ibrow.p, h->icol.p, dx, xin, device_ptrs ? gdA : h->dA.p);
       ++launches;
+      if (overlap)
+        CK(cudaMemcpyAsync(x, dx, n * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
     }
     CK(cudaEventRecord(h->e1, h->st));
     if (!device_ptrs)
