@@ -159,9 +159,11 @@ struct Handle {
   cudaError_t launch_err = cudaSuccess;    // first failed cooperative launch
   int coop_grid64 = 1, coop_grid32 = 1;    // CTAs of the cooperative apply
   // solves in one launch (gbilu_small.cuh), [fp32]: CTAs (0: not used),
-  // dynamic shared memory; their barrier counters and x0 flag
+  // dynamic shared memory; their barrier counters, x0 flag and failed wait
   int small_grid[2] = {0, 0}, small_smem[2] = {0, 0};
   DevBuf<unsigned long long> small_bar;
+  int *h_fail = nullptr;                   // pinned: a failed wait of one (0: none)
+  bool small_probe = false;                // the next one's waits run out (gbilu_wait_probe)
   Ctl *h_inner = nullptr;                  // pinned: an inner solve's outcome
   size_t device_bytes = 0;
 
@@ -806,8 +808,11 @@ template <typename V, typename T> SmallArgs<V, T> small_args(Handle *h, const Op
   const int f = sizeof(T) == 4;
   Vecs<T> &w = *o.vec;
   SmallArgs<V, T> A = {};
-  A.ctl = h->ctl.p;
+  A.fail = reinterpret_cast<int *>(h->small_bar.p + 3);
+  A.host_fail = h->h_fail;
   A.bar = h->small_bar.p + f;
+  A.arrivals = (unsigned int)h->small_grid[f];
+  A.spins = kBarrierSpins;
   A.x_nonzero = reinterpret_cast<int *>(h->small_bar.p + 2);
   A.partials = h->partials.p;
   A.srows = h->srows.p;
@@ -829,8 +834,14 @@ template <typename V, typename T> SmallArgs<V, T> small_args(Handle *h, const Op
 }
 
 template <typename V, typename T>
-cudaError_t launch_small(Handle *h, const SmallArgs<V, T> &A) {
+cudaError_t launch_small(Handle *h, SmallArgs<V, T> A) {
   const int f = sizeof(T) == 4;
+  *h->h_fail = 0;
+  if (h->small_probe) {   // a barrier that one CTA never reaches
+    h->small_probe = false;
+    A.arrivals += 1;
+    A.spins = 1024;
+  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -844,12 +855,14 @@ cudaError_t launch_small(Handle *h, const SmallArgs<V, T> &A) {
   return cudaLaunchKernelEx(&cfg, k_solve_small<V, T>, A, h->sweep[1][f][A.transpose].phases);
 }
 
-// After a failed wait the barrier counters no longer hold a multiple of
-// their grid.
-int reset_small(Handle *h, const Ctl &c) {
-  if (!c.bar_fail) return GBILU_OK;
-  CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
-  CK(cudaMemset(h->ctl.p, 0, sizeof(Ctl)));
+// The outcome of a one-launch solve that has ended, where a wait of it failed:
+// its status, and the counters (no longer a multiple of their grid) and the
+// mark cleared, in stream order before the next launch.
+int check_small(Handle *h, Ctl &c) {
+  if (!*h->h_fail) return GBILU_OK;
+  c.status = ST_TIMEOUT;
+  c.bar_fail = *h->h_fail;
+  CK(cudaMemsetAsync(h->small_bar.p, 0, 4 * sizeof(unsigned long long), h->st));
   return GBILU_OK;
 }
 
@@ -1135,6 +1148,7 @@ int setup_device(Handle *h) {
     CK(cudaEventCreate(&h->e1));
     CK(cudaMallocHost(&h->h_ctl, sizeof(Ctl)));
     CK(cudaMallocHost(&h->h_inner, sizeof(Ctl)));
+    CK(cudaMallocHost(&h->h_fail, sizeof(int)));
     CK(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->opt.device));
   }
   release_device(h);
@@ -1195,8 +1209,8 @@ int setup_device(Handle *h) {
   CK(cudaMemset(h->x0nz.p, 0xff, sizeof(int)));   // "nonzero" until a gather clears it
   CK(h->ctl.alloc(2));
   CK(cudaMemset(h->ctl.p, 0, 2 * sizeof(Ctl)));
-  CK(h->small_bar.alloc(3));
-  CK(cudaMemset(h->small_bar.p, 0, 3 * sizeof(unsigned long long)));
+  CK(h->small_bar.alloc(4));
+  CK(cudaMemset(h->small_bar.p, 0, 4 * sizeof(unsigned long long)));
   if (h->opt.factor_on_device) {
     CK(h->pdiag.alloc(an.nb));
     CK(cudaMemcpy(h->pdiag.p, an.pdiag.data(), an.nb * sizeof(int), cudaMemcpyHostToDevice));
@@ -1522,8 +1536,8 @@ int solve_mixed(Handle *h, bool transpose, double tol, int maxit, gbilu_result *
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
     CK(last_error(h));
-    const Ctl ic = *h->h_inner;
-    if (small) rc = reset_small(h, ic);
+    Ctl ic = *h->h_inner;
+    if (small) rc = check_small(h, ic);
     else if (h->opt.use_graph) launches += (long long)ic.body_runs * h->per_iter[transpose ? 1 : 0];
     if (rc) return rc;
     inner_half += (ic.half >= 0 ? ic.half + 1 : 0);
@@ -1708,6 +1722,7 @@ int gbilu_destroy(void *handle) {
     cudaEventDestroy(h->e1);
     cudaFreeHost(h->h_ctl);
     cudaFreeHost(h->h_inner);
+    cudaFreeHost(h->h_fail);
   }
   delete h;
   return GBILU_OK;
@@ -2049,8 +2064,22 @@ static int solve_impl(Handle *h, const double *b, double *x, bool device_ptrs, b
     c = *h->h_ctl;
     if (h->opt.use_graph) launches += (long long)c.body_runs * h->per_iter[transpose ? 1 : 0];
     if (small) {
-      rc = reset_small(h, c);
+      rc = check_small(h, c);
       if (rc) return rc;
+      // after a failed wait x has not been written: zero where it was to be
+      // (as by a run that ends before its first iteration), and dL/dA with it
+      if (c.bar_fail && from_zero) {
+        const size_t xb = n * sizeof(double);
+        const size_t ab = gx && gdA ? (size_t)h->an.nnzb * 9 * sizeof(double) : 0;
+        if (device_ptrs) {
+          CK(cudaMemsetAsync(x, 0, xb, h->st));
+          if (ab) CK(cudaMemsetAsync(gdA, 0, ab, h->st));
+          CK(cudaStreamSynchronize(h->st));
+        } else {
+          memset(x, 0, xb);
+          if (ab) memset(gdA, 0, ab);
+        }
+      }
     }
   }
   const int outer = r->outer_iters, inner = r->inner_half_iters;
@@ -2231,9 +2260,18 @@ int gbilu_dot_check(void *handle, int n, const float *x, const float *y, double 
 
 int gbilu_wait_probe(void *handle, int mode, int *bar_fail, int *status, double *ms) {
   Handle *h = static_cast<Handle *>(handle);
-  if (!h || (mode != 0 && mode != 1)) return GBILU_BAD_INPUT;
+  if (!h || mode < 0 || mode > 2) return GBILU_BAD_INPUT;
   if (!h->analyzed) return h->fail(GBILU_NOT_READY, "gbilu_analyze has not been called");
   if (h->opt.device < 0) return h->fail(GBILU_NO_DEVICE, "host-only handle cannot run the probe");
+  if (mode == 2) {
+    if (!h->small_grid[0] && !h->small_grid[1])
+      return h->fail(GBILU_BAD_INPUT, "solves of this handle do not run in one launch");
+    h->small_probe = true;
+    if (bar_fail) *bar_fail = 0;
+    if (status) *status = GBILU_OK;
+    if (ms) *ms = 0.0;
+    return GBILU_OK;
+  }
   CK(cudaSetDevice(h->opt.device));
   Ctl *c = h->ctl.p + 1;   // the spare control block: the solve state stays as it is
   k_ctl_init<<<1, 32, 0, h->st>>>(c, 0.0, 0, 0, 0ull);

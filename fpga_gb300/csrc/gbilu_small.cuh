@@ -41,9 +41,12 @@ constexpr int kSmallOwn = 64;                          // slices of a CTA
 // FP32 (T = float), an inner solve of the mixed form: A d = scale * r64 from
 // d = 0, then x64 += unscale * d (device numbering).
 template <typename V, typename T> struct SmallArgs {
-  Ctl *ctl;                       // where a failed wait is marked
   Ctl *host_ctl;                  // the final state (mapped host memory)
-  unsigned long long *bar;        // barrier counter: a multiple of the grid
+  int *fail, *host_fail;          // the kind of a failed wait (see give_up): for the
+                                  // other CTAs, and for the host (mapped); 0 before
+  unsigned long long *bar;        // barrier counter: a multiple of arrivals
+  unsigned int arrivals;          // CTAs that a barrier waits for: the grid
+  unsigned int spins;             // polls after which a wait gives up
   int *x_nonzero;                 // 0 between launches
   double *partials;               // 9 sums a CTA
   const int2 *srows;
@@ -180,6 +183,15 @@ template <typename V, typename T> struct SmallSolve {
     return A.dmat + (size_t)slice(i) * 9 * 32;
   }
 
+  // A wait ran out (1: of a barrier, 2: of the copies): the first kind is kept.
+  // The host learns of it from the CTA that gave up itself: CTA 0 may have
+  // passed the last barrier by then.
+  __device__ void give_up(int kind) {
+    const int first = atomicCAS(A.fail, 0, kind);
+    *(volatile int *)A.host_fail = first ? first : kind;
+    __threadfence_system();
+  }
+
   // Grid barrier; the counter only grows, 64 bits wide, and every launch adds
   // a multiple of its grid. Bounded; a wait that ran out, here or before
   // (late), fails the run in every CTA.
@@ -187,22 +199,18 @@ template <typename V, typename T> struct SmallSolve {
     const int any_late = __syncthreads_or(late);
     if (threadIdx.x == 0) {
       S.ok = !any_late;
-      if (any_late && !*(volatile int *)&A.ctl->bar_fail) mark_stage_timeout(A.ctl);
+      if (any_late) give_up(2);
       unsigned long long ticket, now;
       asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
                    : "=l"(ticket) : "l"(A.bar), "l"(1ull) : "memory");
-      const unsigned long long target = (ticket / G + 1) * G;
+      const unsigned long long target = (ticket / A.arrivals + 1) * A.arrivals;
       unsigned int spins = 0;
       while (true) {
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(A.bar) : "memory");
         if (now >= target) break;
-        if (++spins > kBarrierSpins ||
-            ((spins & 1023) == 0 && *(volatile int *)&A.ctl->bar_fail)) {
+        if (++spins > A.spins || ((spins & 1023) == 0 && *(volatile int *)A.fail)) {
           S.ok = 0;
-          atomicCAS(&A.ctl->bar_fail, 0, 1);
-          A.ctl->status = ST_TIMEOUT;
-          __threadfence();
-          atomicExch(&A.ctl->done, 1);
+          give_up(1);
           break;
         }
         if (spins > 256) __nanosleep(32);
@@ -595,15 +603,7 @@ k_solve_small(const __grid_constant__ SmallArgs<V, T> A, const __grid_constant__
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) *A.x_nonzero = 0;
     __syncthreads();
-    // the outcome to the host; a failed wait has left its kind in ctl
-    if (run.failed) {
-      if (threadIdx.x == 0) {
-        S.c.status = ST_TIMEOUT;
-        S.c.done = 1;
-        S.c.bar_fail = *(volatile int *)&A.ctl->bar_fail;
-      }
-      __syncthreads();
-    }
+    // the outcome to the host, which sees by host_fail when a wait failed
     const unsigned int *src = reinterpret_cast<const unsigned int *>(&S.c);
     for (int i = threadIdx.x; i < (int)(sizeof(Ctl) / 4); i += kSmallThreads)
       reinterpret_cast<unsigned int *>(A.host_ctl)[i] = src[i];

@@ -220,7 +220,8 @@ class GbIlu:
 
     def wait_probe(self, mode):
         """Runs a device wait that never completes (0: grid barrier, 1: data
-        wait) and returns what its bounded timeout reported."""
+        wait) and returns what its bounded timeout reported; 2: makes the next
+        one-launch solve run into such a wait."""
         bf, st, ms = C.c_int(), C.c_int(), C.c_double()
         self._check(self.L.gbilu_wait_probe(self.h, int(mode), C.byref(bf), C.byref(st),
                                             C.byref(ms)))

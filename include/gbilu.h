@@ -201,7 +201,11 @@ int gbilu_get_ordering(void *handle, int *ncolors, int *color, int *perm,
  * runs out after its poll limit (about a second or two), and the probe
  * reports what the solve kernels would report: *bar_fail (1: barrier, 3:
  * data wait), *status (GBILU_TIMEOUT) and the device time in *ms. The
- * handle's solve state is untouched and stays usable. Counterpart of the
+ * handle's solve state is untouched and stays usable. mode 2 runs nothing: it
+ * makes the handle's next one-launch solve wait for a CTA that never comes,
+ * so that solve gives up after a thousand polls, returns GBILU_TIMEOUT (x: the
+ * start vector, or zeros where it is only written) and leaves the handle
+ * usable; GBILU_BAD_INPUT when solves do not run in one launch. Counterpart of the
  * reference's kernel watchdog (abort_cycles, reported as kernel_aborted by
  * bicgstab_utils.cpp:93-129). */
 int gbilu_wait_probe(void *handle, int mode, int *bar_fail, int *status, double *ms);
