@@ -665,9 +665,11 @@ int row_grid(const Handle *h, int rows, int ctas_per_sm) {
 }
 
 // Whether the small steps run beside the vector kernels (k_tail_flow): FP64,
-// three and more colors, few enough for the step list.
+// three and more colors, few enough for the step list, and cooperative
+// launches not ruled out by the options.
 template <typename T> bool flow_run(const Handle *h, bool transpose) {
-  return sizeof(T) == 8 && h->an.ncolors > 2 && h->sweep[1][0][transpose].phases.n > 0;
+  return sizeof(T) == 8 && h->an.ncolors > 2 && h->sweep[1][0][transpose].phases.n > 0 &&
+         (h->opt.sweep_mode == 1 || h->opt.one_launch);
 }
 
 template <int MODE>
@@ -777,7 +779,7 @@ template <typename V, typename T> int plan_small(Handle *h, int rows) {
   const Analysis &an = h->an;
   const int f = sizeof(T) == 4;
   h->small_grid[f] = 0;
-  if (an.ncolors < 2 || an.nb > rows || h->sweep[1][f][0].phases.n == 0 ||
+  if (!h->opt.one_launch || an.ncolors < 2 || an.nb > rows || h->sweep[1][f][0].phases.n == 0 ||
       h->sweep[1][f][1].phases.n == 0)
     return GBILU_OK;
   const int grid = std::min(h->sm_count, an.S);
@@ -1688,6 +1690,7 @@ int gbilu_default_options(gbilu_options *o) {
   o->coloring = 0;
   o->stream_large_steps = 0;
   o->color_on_device = 0;
+  o->one_launch = 1;
   return GBILU_OK;
 }
 

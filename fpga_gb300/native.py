@@ -29,7 +29,7 @@ class Options(C.Structure):
                 ("factor_on_device", C.c_int), ("mixed_scheme", C.c_int),
                 ("ru_delta", C.c_double), ("stage_small_steps", C.c_int),
                 ("coloring", C.c_int), ("stream_large_steps", C.c_int),
-                ("color_on_device", C.c_int)]
+                ("color_on_device", C.c_int), ("one_launch", C.c_int)]
 
 
 class Result(C.Structure):
@@ -143,7 +143,7 @@ class GbIlu:
                  timeout_ms=0.0, inner_tol=1e-1, inner_maxit=500, max_outer=30,
                  verbose=0, sweep_mode=1, factor_on_device=False, mixed_scheme=0,
                  ru_delta=0.1, stage_small_steps=True, coloring="parity",
-                 stream_large_steps=False, color_on_device=False):
+                 stream_large_steps=False, color_on_device=False, one_launch=True):
         self.L = load()
         o = Options()
         self.L.gbilu_default_options(C.byref(o))
@@ -164,6 +164,7 @@ class GbIlu:
         o.coloring = {"parity": 0, "natural": 1}[coloring]
         o.stream_large_steps = int(stream_large_steps)
         o.color_on_device = int(color_on_device)
+        o.one_launch = int(one_launch)
         self.h = VP()
         rc = self.L.gbilu_create(C.byref(o), C.byref(self.h))
         if rc:

@@ -80,9 +80,9 @@ typedef struct {
   int sweep_mode;     /* 1: the whole ILU0 apply is one cooperative launch
                          (default): grid barriers around the large
                          colors, the small ones ordered by their data;
-                         0: one launch per color (same results). An FP64
-                         apply with two colors, and the loop of a solve in
-                         FP64 or in one launch, do not depend on it */
+                         0: one launch per color (same results). The loop of
+                         a solve in FP64 or in one launch does not depend on
+                         it (see one_launch) */
   int factor_on_device; /* 1: gbilu_factor permutes and ILU0-factors on the
                          GPU (color-parallel, bit-identical to the host
                          factorization); 0: on the host (default) */
@@ -114,6 +114,15 @@ typedef struct {
   int color_on_device; /* 1: gbilu_analyze computes the parity-order coloring
                          (coloring = 0) on the GPU, the same colors bit for
                          bit; 0 (default): on the host */
+  int one_launch;     /* 1 (default): a solve (mixed: an inner solve) of a small
+                         system of two and more colors is one cooperative
+                         launch, which holds every SM until it ends; 0: always
+                         the separate kernels of larger systems, which leave
+                         room for other work between them and obey use_graph,
+                         sweep_mode, stage_small_steps and
+                         stream_large_steps; with sweep_mode 0 none of them is
+                         a cooperative launch. Results agree to rounding (the
+                         dot products are summed in another order) */
 } gbilu_options;
 
 typedef struct {
