@@ -665,11 +665,27 @@ int row_grid(const Handle *h, int rows, int ctas_per_sm) {
 }
 
 // Whether the small steps run beside the vector kernels (k_tail_flow): FP64,
-// three and more colors, few enough for the step list, and cooperative
-// launches not ruled out by the options.
+// three and more colors, few enough for the step list, cooperative launches
+// not ruled out by the options, and steps that are small: a few warps of each
+// CTA run them with polled loads, a launch of their own costs each about 5 us
+// twice an iteration. us an iteration beside / in launches, by rows a step
+// (colors, steps):
+//   forward 7,800 (10, 16) 522 / 702; 12,900 (6, 8) 201 / 246; 18,800 (6, 8)
+//     294 / 305; 23,200 (9, 14) 563 / 586; 28,200 (10, 16) 964 / 945; 38,000
+//     (6, 8) 409 / 362
+//   adjoint, whose first sweep multiplies by D in every step: 7,800 663 / 706;
+//     11,300 (10, 16) 702 / 747; 12,900 238 / 241; 14,400 (8, 12) 521 / 463;
+//     18,800 343 / 293; 28,200 1154 / 943; 38,000 467 / 360
+// (27-point, nine-point-layer, 30 % fault and random patterns).
+constexpr int kFlowRows[2] = {24000, 13000};   // rows a step on average [transpose]
 template <typename T> bool flow_run(const Handle *h, bool transpose) {
-  return sizeof(T) == 8 && h->an.ncolors > 2 && h->sweep[1][0][transpose].phases.n > 0 &&
-         (h->opt.sweep_mode == 1 || h->opt.one_launch);
+  const std::vector<Phase> &st = h->sweep[1][0][transpose].steps;
+  if (sizeof(T) != 8 || h->an.ncolors < 3 || h->sweep[1][0][transpose].phases.n == 0 ||
+      (h->opt.sweep_mode == 0 && !h->opt.one_launch))
+    return false;
+  long long rows = 0;
+  for (size_t q = 0; q + 1 < st.size(); ++q) rows += st[q].nrows;
+  return rows <= (long long)kFlowRows[transpose] * (long long)(st.size() - 1);
 }
 
 template <int MODE>

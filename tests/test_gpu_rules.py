@@ -1,0 +1,76 @@
+"""Patterns other than 7-point grids at the sizes where the solve takes another
+path: large colors beside the vector kernels or in launches of their own.
+
+Bounds: a solve's recursive residual is below tol * ||b||, the true one within
+1e-3 of that (rounding is a few 1e-16 of |A||x| an iteration); operators to
+1e-12 of the oracle's, as everywhere.
+"""
+import numpy as np
+import pytest
+
+from fpga_gb300 import GbIlu
+from fpga_gb300.synth import BlockSystem
+
+pytestmark = pytest.mark.gpu
+
+
+def stencil(grid, keep, seed=0):
+    """A grid coupled over the offsets (dz, dy, dx) in -1..1 that keep() takes,
+    blocks and diagonals as in fpga_gb300.synth."""
+    nx, ny, nz = grid
+    nb = nx * ny * nz
+    idx = np.arange(nb).reshape(nz, ny, nx)
+    cut = lambda d, n: (slice(max(0, -d), n - max(0, d)), slice(max(0, d), n - max(0, -d)))
+    ei, ej = [], []
+    for d in np.ndindex(3, 3, 3):
+        dz, dy, dx = (int(v) - 1 for v in d)
+        if (dz, dy, dx) > (0, 0, 0) and keep(dz, dy, dx):
+            z, y, x = cut(dz, nz), cut(dy, ny), cut(dx, nx)
+            ei.append(idx[z[0], y[0], x[0]].ravel())
+            ej.append(idx[z[1], y[1], x[1]].ravel())
+    ei, ej = np.concatenate(ei), np.concatenate(ej)
+    rng = np.random.default_rng(seed)
+    t = np.exp(rng.standard_normal(ei.size))[:, None, None]
+    bij, bji = (-t * (0.1 * rng.standard_normal((ei.size, 3, 3)) + np.eye(3)) for _ in range(2))
+    diag = np.tile(0.5 * np.eye(3), (nb, 1, 1))
+    for at, blk in ((ei, bij), (ej, bji)):
+        for e in np.ndindex(3, 3):
+            diag[:, e[0], e[1]] -= np.bincount(at, weights=blk[:, e[0], e[1]], minlength=nb)
+    rows = np.concatenate([ei, ej, np.arange(nb)])
+    cols = np.concatenate([ej, ei, np.arange(nb)])
+    order = np.lexsort((cols, rows))
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=nb))]).astype(np.int32)
+    return BlockSystem(nb=nb, rowptr=rowptr, colind=cols[order].astype(np.int32),
+                       vals=np.ascontiguousarray(np.concatenate([bij, bji, diag])[order]),
+                       b=rng.standard_normal(3 * nb), cell_of_row=np.arange(nb), grid=grid)
+
+
+def layers(grid):   # nine points in a layer, two across: six colors, four of them large
+    return stencil(grid, lambda z, y, x: z == 0 or (y == 0 and x == 0))
+
+
+def check(s, g):
+    """Forward and adjoint solve; the kernels an iteration of each launched."""
+    A = s.to_scipy()
+    n = np.linalg.norm(s.b)
+    per_iter = []
+    x, r = g.solve(s.b, tol=1e-6, maxit=500)
+    per_iter.append(g.stats()["last_launches"] / (r.half_iters / 2 + 1))
+    assert r.status == 0 and np.linalg.norm(s.b - A @ x) <= 1e-6 * n * (1 + 1e-3)
+    lam, _, r = g.adjoint(s.b, s.b, tol=1e-6, maxit=500, want_dA=False)
+    per_iter.append(g.stats()["last_launches"] / (r.half_iters / 2 + 1))
+    assert r.status == 0 and np.linalg.norm(s.b - A.T @ lam) <= 1e-6 * n * (1 + 1e-3)
+    return per_iter
+
+
+# 12,300 and 13,300 rows a small step (the adjoint's limit between them), 23,400
+# and 24,300 (the forward one's)
+@pytest.mark.parametrize("nz,beside", [(27, (True, True)), (29, (True, False)),
+                                       (51, (True, False)), (53, (False, False))])
+def test_large_colors(built_lib, nz, beside):
+    s = layers((60, 60, nz))
+    with GbIlu(device=0, factor_on_device=True, one_launch=False) as g:
+        g.analyze(s.rowptr, s.colind).factor(s.vals)
+        per_iter = check(s, g)
+    # 7 kernels an iteration against 23, a few for the start and the end
+    assert tuple(p < 15 for p in per_iter) == beside, per_iter
