@@ -776,26 +776,35 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
   }
 }
 
-// Block rows up to which a solve runs in one launch, FP64 and FP32 (inner
-// solves): above, the CTA's 12 warps are too few to stream what its shared
-// memory does not hold. Measured per iteration, separate kernels / one launch,
-// us: FP64 4,000 rows 55 / 27, 35,000 68 / 34, 108,000 87 / 63, 162,000 108 /
-// 98, 216,000 115 / 153; with fault connections (three colors) 33,000 91 / 49,
-// 154,000 112 / 95, 205,000 149 / 172; FP32 108,000 99 / 75, 180,000 116 / 118.
-#ifndef GBILU_SMALL_ROWS64
-#define GBILU_SMALL_ROWS64 170000
-#endif
-#ifndef GBILU_SMALL_ROWS32
-#define GBILU_SMALL_ROWS32 140000
-#endif
+// Blocks up to which a solve (FP64) or an inner solve (FP32) runs in one launch:
+// above, a CTA's 12 warps are too few to stream what its shared memory does
+// not hold. Later the more steps an apply has: a barrier costs less than a
+// launch. us an iteration by the separate kernels / in one launch, by colors
+// and 1000 blocks (grids of 7, 9 + 2, 19 and 27 points, faults, random):
+//   FP64: 2 colors 742: 86 / 67, 1099: 106 / 98; 3: 1054: 119 / 120; 5: 882: 149 /
+//     139, 1069: 159 / 179 (adjoint 179 / 154); 6: 648: 162 / 133, 1082: 201 / 246
+//     (238 / 238); 8: 540: 264 / 194, 900: 311 / 325 (397 / 329), 1109: 234 / 270
+//     (277 / 259); 10: 1124: 429 / 424, 2146: 522 / 502, 3110: 562 / 579; 10 (banded)
+//     1664: 1139 / 834; 15 (random) 1860: 1073 / 1075 (1487 / 1114)
+//   FP32: 2 colors 742: 94 / 77, 961: 101 / 96; 3: 676: 93 / 84, 860: 98 / 102; 5: 521:
+//     113 / 111, 695: 115 / 122; 6: 648: 180 / 151, 736: 140 / 168, 1082: 165 / 209; 8: 540:
+//     266 / 241, 900: 285 / 336, 2208: 217 / 482; 10: 681: 350 / 285, 1124: 347 / 322,
+//     1559: 362 / 487; 14: 903: 983 / 1008; 15: 930: 760 / 822
+// 170,000 and 140,000 rows are what 7-point grids of those blocks have; with
+// fewer blocks a row the vectors decide.
+bool one_launch_size(int rows, long long blocks, int colors, bool fp32) {
+  if (fp32)
+    return rows <= 140000 && blocks <= (colors == 2 ? 970000 : colors <= 8 ? 700000 : 1150000);
+  return rows <= 170000 && blocks <= (colors <= 8 ? 1170000 : 2300000);
+}
 
 // Plans the one-launch solve: its CTAs and the shared memory that the
 // largest share of slices wants (as much as there is when it is more).
-template <typename V, typename T> int plan_small(Handle *h, int rows) {
+template <typename V, typename T> int plan_small(Handle *h) {
   const Analysis &an = h->an;
   const int f = sizeof(T) == 4;
   h->small_grid[f] = 0;
-  if (!h->opt.one_launch || an.ncolors < 2 || an.nb > rows || h->sweep[1][f][0].phases.n == 0 ||
+  if (!h->opt.one_launch || an.ncolors < 2 || !one_launch_size(an.nb, an.nnzb, an.ncolors, f) || h->sweep[1][f][0].phases.n == 0 ||
       h->sweep[1][f][1].phases.n == 0)
     return GBILU_OK;
   const int grid = std::min(h->sm_count, an.S);
@@ -1306,8 +1315,8 @@ int setup_device(Handle *h) {
   }
   if (h->with_32) {
     if (h->opt.mixed_scheme == 0)
-      if (int rc = plan_small<float, float>(h, GBILU_SMALL_ROWS32)) return rc;
-  } else if (int rc = plan_small<double, double>(h, GBILU_SMALL_ROWS64)) {
+      if (int rc = plan_small<float, float>(h)) return rc;
+  } else if (int rc = plan_small<double, double>(h)) {
     return rc;
   }
   h->device_bytes += nd * 16 + (h->with_32 ? nd * 8 : 0) + n * 8 * 15 + (h->with_32 ? n * 4 * 12 : 0) +

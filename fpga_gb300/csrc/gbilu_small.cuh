@@ -17,7 +17,7 @@
 //
 // Measured against the separate kernels: an iteration of 4,000 cells 59 -> 28
 // us, of 33,000 cells (three colors) 97 -> 49, of 108,000 cells 88 -> 63 (see
-// GBILU_SMALL_ROWS64 for where it ends). Ordering the steps between two
+// one_launch_size for where it ends). Ordering the steps between two
 // reductions by their data instead (results preset to a sentinel, consumers
 // polling) gave 28.7 us for 4,000 cells with two colors, but 47 instead of 44
 // with three and 75 instead of 53 for 33,000 cells: polled loads bypass L1.

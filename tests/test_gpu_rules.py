@@ -1,5 +1,6 @@
 """Patterns other than 7-point grids at the sizes where the solve takes another
-path: large colors beside the vector kernels or in launches of their own.
+path: large colors beside the vector kernels or in launches of their own, a
+solve in one launch or by the separate kernels.
 
 Bounds: a solve's recursive residual is below tol * ||b||, the true one within
 1e-3 of that (rounding is a few 1e-16 of |A||x| an iteration); operators to
@@ -74,3 +75,22 @@ def test_large_colors(built_lib, nz, beside):
         per_iter = check(s, g)
     # 7 kernels an iteration against 23, a few for the start and the end
     assert tuple(p < 15 for p in per_iter) == beside, per_iter
+
+
+def points27(grid):   # eight large colors and two small ones
+    return stencil(grid, lambda z, y, x: True)
+
+
+# blocks below and above the limit of the colors and the precision
+@pytest.mark.parametrize("precision,make,grid,one", [
+    ("fp64", layers, (60, 60, 30), True), ("fp64", layers, (60, 60, 31), False),
+    ("mixed", layers, (60, 60, 18), True), ("mixed", layers, (60, 60, 19), False),
+    ("mixed", points27, (36, 36, 34), True), ("mixed", points27, (36, 36, 35), False),
+    ("fp64", points27, (46, 46, 42), True), ("fp64", points27, (46, 46, 43), False)],
+    ids=lambda v: v if isinstance(v, str) else getattr(v, "__name__", str(v)))
+def test_one_launch_or_not(built_lib, precision, make, grid, one):
+    s = make(grid)
+    with GbIlu(device=0, factor_on_device=True, precision=precision) as g:
+        g.analyze(s.rowptr, s.colind).factor(s.vals)
+        check(s, g)
+        assert (g.stats()["launches_per_iter"] == 0) == one
