@@ -546,19 +546,35 @@ cudaError_t launch_coop(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *
                             o.vec->y.p, hat, (const T *)o.vec->base.p, coef);
 }
 
+// Whether an FP64 apply with two colors is a launch a step. A cooperative launch
+// costs more than the launch or two that it saves, but its warps take the
+// slices of a step in rounds without a gap between them; it loses again where
+// a second round is hardly filled. us in one launch / by steps, by slices of
+// the larger color for each of the grid's 2432 warps: 0.03: 24.7 / 16.4, 0.4:
+// 26.7 / 22.6, 0.7: 28.7 / 26.7 (a whole gbilu_apply_ilu call 99 / 102), 0.93:
+// 28.9 / 30.7, 1.1: 40.6 / 34.9, 1.3: 43.0 / 42.1, 1.44: 43.1 / 42.6 (call 146 /
+// 148), 1.56: 43.3 / 46.5, 1.8: 45.2 / 49.4, 2.6: 61.1 / 62.3, 3.9: 80.9 / 84.3,
+// 6.4: 130.6 / 129.2, 12.9: 243.9 / 244.1.
+bool steps_faster(const Handle *h) {
+  const std::vector<int> &c = h->an.slice_color_ptr;
+  const double rounds = (double)std::max(c[1], c[2] - c[1]) /
+                        (h->sm_count * (coop_threads<double>() / 32));
+  return rounds <= 0.6 || (rounds > 1.0 && rounds <= 1.25);
+}
+
 // hat = M^-1 src (forward) or M^-T src (transpose); the vector set's y holds
 // the first sweep's result. RED: what the reduced iteration leaves of it, with
 // coef = &Ctl::cp (src = p) or &Ctl::cs (src = s): in FP32 one launch as well;
 // with two colors, or behind k_tail_flow (head_only), the last step alone.
-// An FP64 apply with two colors is a launch a step: a cooperative launch costs
-// more than the two launches that it saves (4,000 rows 24.6 us against 18.5,
-// 59,000 rows 24.6 against 20.9, 500,000 rows 74.2 against 76.0).
+// An FP64 apply with two colors is a launch a step where that is the faster
+// form (steps_faster).
 template <typename V, typename T, bool RED = false>
 void apply_prec(Handle *h, cudaStream_t s, const Ops<V, T> &o, const T *src, T *hat,
                 int &launches, const double *coef = nullptr, bool head_only = false) {
   if constexpr (!RED || sizeof(T) == 4) {
     const int C = h->an.ncolors;
-    if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 && !(C == 2 && (RED || sizeof(T) == 8))) {
+    if (h->opt.sweep_mode == 1 && C <= kMaxPhases / 2 &&
+        !(C == 2 && (RED || (sizeof(T) == 8 && steps_faster(h))))) {
       const cudaError_t e = launch_coop<V, T, RED>(h, s, o, src, hat, 0, coef);
       if (e != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = e;
       ++launches;

@@ -1,6 +1,7 @@
 """Patterns other than 7-point grids at the sizes where the solve takes another
 path: large colors beside the vector kernels or in launches of their own, a
-solve in one launch or by the separate kernels.
+solve in one launch or by the separate kernels; and 7-point grids where the
+apply of two colors does.
 
 Bounds: a solve's recursive residual is below tol * ||b||, the true one within
 1e-3 of that (rounding is a few 1e-16 of |A||x| an iteration); operators to
@@ -10,7 +11,8 @@ import numpy as np
 import pytest
 
 from fpga_gb300 import GbIlu
-from fpga_gb300.synth import BlockSystem
+from fpga_gb300.synth import BlockSystem, generate
+from oracle_lib import Prepared
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +96,24 @@ def test_one_launch_or_not(built_lib, precision, make, grid, one):
         g.analyze(s.rowptr, s.colind).factor(s.vals)
         check(s, g)
         assert (g.stats()["launches_per_iter"] == 0) == one
+
+
+# slices of a color for each of 152 x 16 warps: 0.597, 0.617, 0.98, 1.02, 1.23, 1.27
+@pytest.mark.parametrize("nx,kernels", [(31, 2), (32, 1), (51, 1), (53, 2), (64, 2), (66, 1)])
+def test_apply_of_two_colors(built_lib, nx, kernels):
+    s = generate(nx, 60, 50, sigma=1.0, seed=4)
+    P = Prepared(s)
+    p = np.random.default_rng(5).standard_normal(s.n)
+    out = []
+    for sweep_mode in (1, 0):
+        with GbIlu(device=0, factor_on_device=True, sweep_mode=sweep_mode) as g:
+            g.analyze(s.rowptr, s.colind).factor(s.vals)
+            for transpose in (False, True):
+                z = g.ilu_apply(p, transpose)
+                # beside the start's and the two permutations of the vectors
+                assert g.stats()["last_launches"] - 3 == (2 if sweep_mode == 0 else kernels) + \
+                    (1 if transpose and (sweep_mode == 0 or kernels == 2) else 0)
+                z_ref = P.ilu_apply(p, transpose)
+                assert np.linalg.norm(z - z_ref) <= 1e-12 * np.linalg.norm(z_ref)
+                out.append(z)
+    assert np.array_equal(out[0], out[2]) and np.array_equal(out[1], out[3])
