@@ -265,7 +265,7 @@ def gpu_bench(args, world, rank, local):
     ms, by, la = g.bench_kernel("spmv_omega64", reps=20)
     dom = {"ms": ms, "alg_bytes": by, "gbs": by / ms / 1e6}
     fp64_floor_us = iteration_fmas(g64, st, s.rowptr)["spmv_omega"] / fp64_fma_rate(local) * 1e6
-    roofline = {"bound": "hbm", "kernel": "k_spmv<double> with the omega dots (rows outside color 0)",
+    roofline = {"bound": "fp64", "kernel": "k_spmv<double> with the omega dots (rows outside color 0)",
                 "achieved": dom["gbs"], "peak": peak, "unit": "GB/s",
                 "frac": dom["gbs"] / peak, "traffic": traffic,
                 "peak_kind": peak_kind, "alg_bytes_per_launch": dom["alg_bytes"],
@@ -322,7 +322,8 @@ def iteration_fmas(g64, st, rowptr):
     """DFMA per launch (FP64) over the rows that the iteration runs on: color
     0 (n0 rows, a0 blocks of A) takes part in the apply's last step alone; the
     other n rows in the SpMV (9 per block and the dots) and the vector kernels
-    (update_s and update_p also apply D^-1 to color 1)."""
+    (update_s and update_p also apply D^-1 to color 1, and beside them run the
+    small steps of three and more colors)."""
     import numpy as np
     _, color, _, cp = g64.ordering()
     n0, n1 = int(cp[1]), int(cp[2] - cp[1])
@@ -330,9 +331,10 @@ def iteration_fmas(g64, st, rowptr):
     a0 = int(deg[color == 0].sum())
     nb, nnzb, n = st["nb"], st["nnzb"], 3 * (st["nb"] - n0)
     inner = st["nnzb_lower"] + st["nnzb_upper"] - 2 * (a0 - n0)
-    return {"apply": 9 * (a0 - n0 + inner + nb - n1), "spmv_alpha": 9 * (nnzb - a0) + n,
-            "spmv_omega": 9 * (nnzb - a0) + 2 * n, "update_s": 3 * n + 9 * n1,
-            "update_r": 5 * n, "update_p": 3 * n + 9 * n1}
+    small = 9 * (inner + nb - n0 - n1)
+    return {"apply": 9 * a0, "spmv_alpha": 9 * (nnzb - a0) + n,
+            "spmv_omega": 9 * (nnzb - a0) + 2 * n, "update_s": 3 * n + 9 * n1 + small,
+            "update_r": 5 * n, "update_p": 3 * n + 9 * n1 + small}
 
 
 def iteration_budget(g, g64, st, rowptr, b_dev, x_dev, local):

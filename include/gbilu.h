@@ -311,7 +311,9 @@ int gbilu_get_stats(void *handle, gbilu_stats *stats);
  * kernels of one iteration over the rows that it runs on, 4-8 in FP64 and
  * 9-13 in FP32: SpMV with the alpha dot, SpMV with the omega dots, update_s,
  * update_r, update_p, and 14 (FP64), 15 (FP32) its part of the ILU apply
- * (FP32 ids need GBILU_MIXED). Returns the average device ms per application, its
+ * (FP32 ids need GBILU_MIXED). Where the small colors' steps run beside
+ * update_s and update_p (FP64, three and more colors), their time and bytes
+ * count there, not in the apply. Returns the average device ms per application, its
  * algorithmic bytes and the kernel launches per application. The
  * counterpart of the reference's kernel timing around clEnqueueTask
  * (fpga_functions_bicgstab.cpp:1305-1325), per kernel instead of per run. */

@@ -117,3 +117,26 @@ def test_apply_of_two_colors(built_lib, nx, kernels):
                 assert np.linalg.norm(z - z_ref) <= 1e-12 * np.linalg.norm(z_ref)
                 out.append(z)
     assert np.array_equal(out[0], out[2]) and np.array_equal(out[1], out[3])
+
+
+def test_kernel_timings_follow_the_small_steps(built_lib):
+    """gbilu_bench_kernel counts the small colors' steps where they run: beside
+    update_s and update_p, or (no cooperative launches) in the apply. The
+    iteration's bytes are the same either way."""
+    s = generate(30, 24, 12, sigma=1.5, inactive_frac=0.05, fault_frac=0.01, seed=7)
+    got = []
+    for options in (dict(), dict(one_launch=False, sweep_mode=0)):
+        with GbIlu(device=0, factor_on_device=True, **options) as g:
+            g.analyze(s.rowptr, s.colind).factor(s.vals)
+            r = {k: g.bench_kernel(k + "64", reps=5) for k in ("apply", "update_s", "update_r", "update_p")}
+            assert all(ms > 0 for ms, _, _ in r.values())
+            got.append(({k: by for k, (_, by, _) in r.items()}, {k: la for k, (_, _, la) in r.items()},
+                        g.stats()["alg_bytes_iter"][0]))
+            # the handle solves as before
+            x, res = g.solve(s.b, tol=1e-6, maxit=500)
+            assert res.status == 0
+    (beside, la, total), (inside, la0, total0) = got
+    small = inside["apply"] - beside["apply"]
+    assert small > 0 and total == total0 and beside["update_r"] == inside["update_r"]
+    assert beside["update_s"] - inside["update_s"] == small == beside["update_p"] - inside["update_p"]
+    assert set(la.values()) == {1} and la0["apply"] > 1
