@@ -810,7 +810,8 @@ void reduced_start(Handle *h, const Ops<V, T> &o, long long &launches) {
 // fewer blocks a row the vectors decide.
 bool one_launch_size(int rows, long long blocks, int colors, bool fp32) {
   if (fp32)
-    return rows <= 140000 && blocks <= (colors == 2 ? 970000 : colors <= 8 ? 700000 : 1150000);
+    return rows <= 140000 &&
+           blocks <= (colors == 2 ? 970000 : colors > 8 && colors <= 12 ? 1150000 : 700000);
   return rows <= 170000 && blocks <= (colors <= 8 ? 1170000 : 2300000);
 }
 
