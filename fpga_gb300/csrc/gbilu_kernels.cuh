@@ -2045,7 +2045,7 @@ __global__ void k_scatter(int nb, const int *__restrict__ perm, const T *__restr
   if (nz && __syncthreads_or(any) && threadIdx.x == 0) *nz = 1;
 }
 
-// out = (float)(scale * in): the FP32 right-hand side of a refinement step
+// out = (float)(scale * in): FP32 inputs of the kernel timings
 __global__ void k_scale_convert(int n, double scale, const double *__restrict__ in,
                                 float *__restrict__ out) {
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
@@ -2172,9 +2172,7 @@ __global__ void k_block_positions(long long n, const int *__restrict__ vsrc,
 // present in both rows (a merge of the two sorted column lists);
 // D_i^-1 = inv(A_ii) by cofactors. A singular (or not finite) pivot records
 // the smallest failing row in bad[0]; bad[1] gets minus the high word of color
-// 0's head_gain (both start from 0x7f7f7f7f). Finished blocks also go straight to the
-// sliced L, U, their transposes and D^-1, D^-T (FactorOut): the FP64 unit
-// bounds the kernel, and a pass of its own for each array took 0.2 ms more.
+// 0's head_gain (both start from 0x7f7f7f7f).
 //
 // Three threads a row, one per row of its blocks: row r of L_ik and of every
 // update needs row r of A_ik alone, so they meet only in the inverse. On a

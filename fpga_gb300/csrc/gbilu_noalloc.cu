@@ -15,9 +15,10 @@
 // Its only scratch is the file-scope device array below: one partial sum per
 // CTA plus an arrival counter for the grid-wide reduction. Every GPU that
 // loads the library holds this array (about 32 KiB) until the process exits.
-// A call takes at most 4096 partials, and at most 4096 * 256 = 1,048,576
-// block rows; larger systems are rejected with GBILU_BAD_INPUT. Calls share
-// the array: two calls that overlap on the GPU (different streams, or
+// A call writes one partial per CTA (4096 fit). It takes at most 1,048,576
+// block rows, the documented limit of the entry point (an earlier kernel needed
+// a partial per 256 rows); larger systems are rejected with GBILU_BAD_INPUT.
+// Calls share the array: two calls that overlap on the GPU (different streams, or
 // different host threads on one device) race on it and give wrong sums, so
 // serialise them on one stream.
 //
@@ -45,7 +46,7 @@ constexpr int kNoAllocThreads = 3 * kTileRows;
 constexpr int kTileBlocks = 256;          // blocks of a tile that fit its buffer
 constexpr int kCtasPerSm = 10;            // resident tiles of 19.7 KB each
 constexpr int kNoAllocMaxCtas = 4096;     // scratch holds this many partials
-constexpr int kNoAllocMaxRows = 4096 * 256;
+constexpr int kNoAllocMaxRows = 1048576;
 constexpr int kMaxDevices = 64;
 
 struct NoAllocScratch {
@@ -222,8 +223,7 @@ extern "C" int gbilu_bsr_spmv_dot_noalloc(int nb, const int *d_rowptr, const int
   }
   if (nb > kNoAllocMaxRows) {
     fprintf(stderr,
-            "ERROR: gbilu_bsr_spmv_dot_noalloc: nb = %d exceeds the maximum of %d block rows "
-            "of the fixed scratch array\n",
+            "ERROR: gbilu_bsr_spmv_dot_noalloc: nb = %d exceeds the maximum of %d block rows\n",
             nb, kNoAllocMaxRows);
     return GBILU_BAD_INPUT;
   }

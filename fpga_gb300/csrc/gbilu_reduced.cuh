@@ -23,14 +23,15 @@
 //   SpMV of the tail:   v = A p^, (v, rt);
 //
 // i.e. half of the blocks of A, the head's half of U and two diagonals
-// instead of A, L, U and D: 0.55 instead of 1.30 GB an iteration on the
-// 500k-cell system in FP64. x is advanced on the tail alone; at the end the
+// instead of A, L, U and D: 0.71 instead of 1.30 GB an iteration on the
+// 500k-cell system in FP64, the vectors included. x is advanced on the tail alone; at the end the
 // head's equations give its x from the residual they are left with,
 // x_0 = A_00^-1 (b_0 - cr r0 - sum A_0j x_j). In exact arithmetic the
 // iterates, norms and stop tests are those of the full iteration; rounding
 // adds what the head's blocks make of theirs, so that a factorization with
-// ill-conditioned ones keeps the full iteration (reduced_run). (With U^T, L^T and A^T for the adjoint: base0 = D^-T r0,
-// g = U_i0^T base0, head: p^ = cp base0 - sum L^T p^.)
+// ill-conditioned ones keeps the full iteration (reduced_run). (With U^T, L^T
+// and A^T for the adjoint: base0 = D^-T r0, g = U_i0^T base0, head:
+// p^ = cp base0 - sum L^T p^.)
 //
 // base holds, in one vector, r0 (adjoint: D^-T r0) on the head and -g on the
 // tail, so a head row's own value is coef * base and a tail row's is

@@ -15,9 +15,10 @@
 // SpMV in vain. b and x are read and written in the caller's numbering by the
 // same launch.
 //
-// Measured against the separate kernels: an iteration of 4,000 cells 59 -> 28
-// us, of 33,000 cells (three colors) 97 -> 49, of 108,000 cells 88 -> 63 (see
-// one_launch_size for where it ends). Ordering the steps between two
+// Measured against the separate kernels (solves to 1e-8, start and end
+// included): an iteration of 33,000 rows (three colors) 78 -> 49 us, of 59,000
+// 73 -> 49, of 108,000 86 -> 67; one_launch_size has more and where it ends.
+// It holds every SM until it ends (gbilu_options.one_launch). Ordering the steps between two
 // reductions by their data instead (results preset to a sentinel, consumers
 // polling) gave 28.7 us for 4,000 cells with two colors, but 47 instead of 44
 // with three and 75 instead of 53 for 33,000 cells: polled loads bypass L1.

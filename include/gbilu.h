@@ -263,8 +263,10 @@ int gbilu_get_factors(void *handle, double *lu, double *dinv);
  * (2*maxit at the cap), and res->inner_half_iters the total itself.
  * When both arrays are page-locked (cudaHostAlloc / cudaHostRegister), x0
  * and x move over the CPU-GPU link in place and b by the copy engine while
- * A x0 is computed; other host memory goes through staging copies. Both
- * give the same bits. */
+ * A x0 is computed; other host memory, and every array of a solve in one
+ * launch (gbilu_options.one_launch), goes through staging copies. Both give
+ * the same bits. With ill-conditioned 3x3 diagonal blocks the iteration runs
+ * over all rows instead of leaving out color 0's, by the separate kernels. */
 int gbilu_solve(void *handle, const double *b, double *x, double tol,
                 int maxit, gbilu_result *res);
 
@@ -298,7 +300,8 @@ int gbilu_adjoint(void *handle, const double *g, const double *x,
                   gbilu_result *res);
 
 /* As gbilu_adjoint with DEVICE pointers (original numbering): d_g[3*nb],
- * d_x[3*nb] in, d_lambda[3*nb] out (x0 = 0), d_dA[nnzb*9] out or NULL. */
+ * d_x[3*nb] in, d_lambda[3*nb] out (x0 = 0), d_dA[nnzb*9] out or NULL.
+ * d_lambda may be d_g or d_x: dL/dA is formed with the x that was passed. */
 int gbilu_adjoint_device(void *handle, const double *d_g, const double *d_x,
                          double *d_lambda, double *d_dA, double tol, int maxit,
                          gbilu_result *res);
@@ -410,8 +413,8 @@ int gbilu_status_lines(const gbilu_result *res, unsigned long long *buf, int lin
  * memory or create a handle (a host framework that hands out a fixed
  * device arena, a callback in which cudaMalloc's implicit synchronisation
  * is not allowed): it calls no cudaMalloc/cudaFree; its reduction scratch
- * is a fixed ~32 KiB device array inside the library, which limits nb to
- * 1,048,576 block rows (larger nb -> GBILU_BAD_INPUT). y must not alias x
+ * is a fixed ~32 KiB device array inside the library. At most 1,048,576
+ * block rows (larger nb -> GBILU_BAD_INPUT). y must not alias x
  * or w (w may alias x). The first call on a device looks the array's
  * address up in the device's primary context (the CUDA runtime's) and
  * keeps it for the life of the process: make that first call before any
